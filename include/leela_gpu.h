@@ -254,13 +254,16 @@ LG_API int lg_policy_device_static(lg_ctx *ctx, const uint8_t *planes, int B, fl
  * for the first layer (0: 256-row, 1: 128-row tiles; unused by choices 3
  * and 4), and -- for buckets of at most 8 positions -- choice 4: every layer
  * of the net in one small-batch launch (FP32 nets: 0 = the generic per-layer
- * FP32 kernels, 4 = the small-batch kernel), and keeps the fastest.  With a
+ * FP32 kernels, 3 = the trunk in one launch on the tensor cores, each FP32
+ * value as the sum of three BF16 parts, 4 = the small-batch kernel), and
+ * keeps the fastest.  With a
  * cache path, a table saved for the same device, SM count and net shapes is
  * loaded instead (unless force), and a new table is saved there (written to
  * a temporary file and renamed).  Without tuning (measured defaults): a
  * context with a 16-bit net uses choice 4 up to 2 positions and choice 3
  * above; an FP32-only context uses choice 4 up to 8 positions and its
- * per-layer kernels above.  No reference
+ * per-layer kernels above, where nets whose layers have 32 to 256 channels
+ * run the split trunk from 3 positions on.  No reference
  * counterpart (the OpenCL backend reads a fixed cfg_rowtiles,
  * OpenCL.cpp:634-646).  lg_tuning reports the choice for batch B; it returns
  * 1 once tuned, 0 if not, < 0 on error. */

@@ -1,4 +1,6 @@
-// fp32_path.cu -- the plain FP32 evaluation path (the drop-in path).
+// fp32_path.cu -- the plain FP32 evaluation path (the drop-in path) on the
+// FFMA pipes: narrow nets, the allocation-free call, the student's training
+// and hand-set per-layer choices (other FP32 trunks run in split_conv.cu).
 //
 // Same arithmetic as the reference's BLAS build (Network.cpp:345-423:
 // im2col + sgemm + bias + activation, FP32 throughout, expf-based ELU), laid
@@ -320,6 +322,8 @@ __global__ void splitk_reduce_f32(const float *__restrict__ partial, int nsplit,
 __global__ void head_conv_f32(const float *__restrict__ in, const float *__restrict__ wh,
                               float bias, int B, int C, int k, int do_act, int act,
                               float *__restrict__ logits) {
+    ptx::grid_dep_launch();
+    ptx::grid_dep_wait();
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
     int lane = threadIdx.x % 32;
     if (warp >= B * kPoints) return;
@@ -415,10 +419,18 @@ size_t conv_f32_partial_floats(int B, int C, int O, int k) {
 }
 
 void launch_head_conv_f32(const float *in, const float *wh, float bias, int B, int C, int k,
-                          int do_act, int act, float *logits, cudaStream_t s) {
+                          int do_act, int act, float *logits, cudaStream_t s, bool pdl) {
     int warps = B * kPoints;
-    int blocks = (warps * 32 + 255) / 256;
-    head_conv_f32<<<blocks, 256, 0, s>>>(in, wh, bias, B, C, k, do_act, act, logits);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((warps * 32 + 255) / 256);
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, head_conv_f32, in, wh, bias, B, C, k, do_act, act, logits);
 }
 
 }  // namespace lg

@@ -41,6 +41,7 @@ namespace {
 using namespace lg;
 
 constexpr int kMaxConv = 40;
+constexpr int kSplitMaxBatch = 1024;  // positions a launch of the split FP32 trunk (its buffers: 0.6 GB at width 128)
 
 // ------------------------------------------------------------ shapes
 
@@ -98,6 +99,11 @@ struct Net {
     float head_b = 0.0f;
     float *w1s = nullptr, *b1 = nullptr, *w2 = nullptr;
     float b2 = 0.0f;
+    // the FP32 trunk on the tensor cores (split_conv.cu), for the nets it covers
+    bool split_ok = false;
+    std::vector<SplitLayer> split;
+    __nv_bfloat16 *split_w = nullptr;
+    int split_pitch = 0;
     // small-batch path (latency.cu): per conv layer and the head, weights
     // [8][cg][k*k][cout] with each split padded to `slice` floats
     bool lat_ok = false;
@@ -122,6 +128,11 @@ struct lg_ctx {
     // FP32 buffers
     float *act[2] = {nullptr, nullptr};
     float *partial = nullptr;
+    // FP32 layers on the tensor cores: activations as BF16 parts, expanded
+    // planes, counters; launches of at most split_batch positions
+    __nv_bfloat16 *sp_act[2] = {nullptr, nullptr}, *sp_l5 = nullptr;
+    int *sp_flags = nullptr;
+    int split_batch = 0;
     // small-batch path: partial sums, counters (zero between launches),
     // value-head partials
     float *lat_part = nullptr;
@@ -177,6 +188,8 @@ struct lg_ctx {
     // kLatMaxB, nets it supports; the default there); [bucket][1] first
     // layer, 0 = 256-row, 1 = 128-row.
     int tc_variant[17][2] = {};
+    // buckets whose choice was set by hand, tuned or loaded
+    bool chosen[17] = {};
     bool tuned = false;
     std::atomic<long long> launches{0};
     std::atomic<long long> batches{0};
@@ -315,6 +328,44 @@ int build_lat(lg_ctx *c, Net &n, const std::vector<std::vector<float>> &Wraw) {
     return LG_OK;
 }
 
+// FP32 nets that run on the tensor cores (split_conv.cu): a 5x5 first layer
+// and 3x3 layers of 32 to 256 channels, padded to groups of 64, with finite
+// weights (an infinite weight has no parts).  Narrower nets keep the FFMA
+// kernels: less than half of a padded group would be theirs.
+int build_split(lg_ctx *c, Net &n, const std::vector<std::vector<float>> &Wraw,
+                const std::vector<std::vector<float>> &Braw) {
+    const int ntrunk = (int)n.shapes.size() - 1;
+    bool ok = ntrunk >= 2 && ntrunk <= kSpMaxLayers;
+    for (int l = 0; l < ntrunk && ok; ++l) {
+        ok = n.shapes[l].cout >= 32 && n.shapes[l].cout <= 256;
+        for (float v : Wraw[l]) ok = ok && std::isfinite(v);
+    }
+    if (!ok) return LG_OK;
+    size_t elems = 0;
+    for (int l = 0; l < ntrunk; ++l) elems += split_weight_elems(n.shapes[l].k, n.shapes[l].cin, n.shapes[l].cout);
+    if (int rc = dev_alloc(c, &n.split_w, elems)) return rc;
+    size_t at = 0;
+    for (int l = 0; l < ntrunk; ++l) {
+        const Shape sh = n.shapes[l];
+        SplitLayer S{};
+        S.halves = split_pad(l == 0 ? 5 * sh.cin : sh.cin) / 64;
+        S.groups = split_pad(sh.cout) / 64;
+        S.cout = sh.cout;
+        n.split_pitch = std::max(n.split_pitch, S.groups * 64);
+        launch_split_weights(n.wt[l], sh.k, sh.cin, sh.cout, n.split_w + at, c->stream);
+        at += split_weight_elems(sh.k, sh.cin, sh.cout);
+        std::vector<float> b(Braw[l]);
+        b.resize((size_t)S.groups * 64, 0.0f);
+        float *db;
+        if (int rc = upload(c, &db, b)) return rc;
+        S.bias = db;
+        n.split.push_back(S);
+    }
+    LG_CUDA_TRY(cudaGetLastError());
+    n.split_ok = true;
+    return LG_OK;
+}
+
 // The small-batch kernel's layout for tensor-core nets of width 128 (1x1
 // head): the first layer and the head in FP32 on the weights as the
 // precision rounds them (FP8: the E4M3 codes, the per-channel scale being
@@ -430,7 +481,7 @@ int build_net(lg_ctx *c, Net &n, const lg_net_desc *d) {
             for (int t = 0; t < kk; ++t) wh[(size_t)t * hs.cin + ci] = Wraw.back()[(size_t)ci * kk + t];
         if ((rc = upload(c, &n.head_w, wh))) return rc;
         n.head_b = Braw.back()[0];
-        if ((rc = build_lat(c, n, Wraw))) return rc;
+        if ((rc = build_lat(c, n, Wraw)) || (rc = build_split(c, n, Wraw, Braw))) return rc;
     } else {
         // ---- tensor-core layouts: [tap][half][N][64] 16-bit operands (BF16,
         // or FP16 for LG_FP16), K-major rows.
@@ -584,13 +635,26 @@ int bucket_of(int B) {
     return bl;
 }
 
+// Where nobody chose, FP32 nets that the split trunk covers leave the
+// small-batch kernel for it from 3 positions on: that kernel's time grows
+// with the batch (benchmark nets, policy + value pair: 179, 313, 447, 715,
+// 1118 us at 1, 2, 3, 5, 8 positions), the split trunk's items run side by
+// side (430 to 443 us over the same sizes).  A hand-set choice 0 stays the
+// FFMA kernels per layer (at 256 positions 14.3 ms a pair against 3.0).
+constexpr int kLatSplitB = 2;
 bool use_lat(lg_ctx *c, const Net &n, int B) {
-    return n.lat_ok && B <= kLatMaxB && c->lat_part && c->tc_variant[bucket_of(B)][0] == 4;
+    const int bl = bucket_of(B);
+    return n.lat_ok && B <= kLatMaxB && c->lat_part && c->tc_variant[bl][0] == 4 &&
+           (c->chosen[bl] || !n.split_ok || B <= kLatSplitB);
+}
+bool use_split(lg_ctx *c, const Net &n, int B) {
+    const int bl = bucket_of(B);
+    return n.split_ok && (!c->chosen[bl] || c->tc_variant[bl][0] == 3);
 }
 
 // Kernel choices without tuning (measured on GB300, policy + value pairs,
 // device-resident inputs): FP32 nets run the small-batch kernel up to 8
-// positions (B = 8: 1.12 against 1.13 ms on the per-layer kernels); 16-bit
+// positions (but see use_lat) and the split trunk above; 16-bit
 // nets run it up to 2 (B = 2: 220 against 254 us on the persistent trunk;
 // B = 3: 314 against 256 us) and the persistent trunk with the first layer
 // inside from 3 positions on (B = 256: 0.43 against 0.76 ms a pair on the
@@ -601,6 +665,7 @@ void default_tuning(lg_ctx *c) {
     for (int b = 0; b < 17; ++b) {
         c->tc_variant[b][0] = lowp ? ((1 << b) <= 2 ? 4 : 3) : ((1 << b) <= kLatMaxB ? 4 : 0);
         c->tc_variant[b][1] = 0;
+        c->chosen[b] = false;
     }
 }
 
@@ -652,36 +717,69 @@ int forward_fp32(lg_ctx *c, Net &n, const uint8_t *planes, int B, float T, float
     if (use_lat(c, n, B)) return forward_lat(c, n, planes, B, T, probs, logits_out, value, s, nlaunch, prof);
     const lg_net_desc &d = n.d;
     int L = 0;
-    {
-        ProfScope ps(c, prof, LG_PROF_OTHER, s);
-        launch_pack_planes_f32(planes, B, d.c_in, c->act[0], s);
-    }
-    ++L;
     int cur = 0;
-    int ntrunk = (int)n.shapes.size() - 1;
-    for (int l = 0; l < ntrunk; ++l) {
-        auto sh = n.shapes[l];
-        ProfScope ps(c, prof, LG_PROF_FP32_CONV, s);
-        launch_conv_f32(c->act[cur], n.wt[l], n.bias[l], c->act[cur ^ 1], B, sh.cin, sh.cout, sh.k,
-                        d.act, c->partial, s);
-        L += conv_f32_partial_floats(B, sh.cin, sh.cout, sh.k) ? 2 : 1;
-        cur ^= 1;
+    const int ntrunk = (int)n.shapes.size() - 1;
+    const bool split = use_split(c, n, B);
+    if (split) {
+        // the trunk on the tensor cores, split_batch positions a launch; its
+        // output in act[0]
+        const size_t per_in = (size_t)d.c_in * kPoints, per_out = (size_t)kPoints * n.shapes[ntrunk - 1].cout;
+        for (int b0 = 0; b0 < B; b0 += c->split_batch) {
+            const int nb = std::min(c->split_batch, B - b0);
+            {
+                ProfScope ps(c, prof, LG_PROF_OTHER, s);
+                launch_pack_planes_l5(planes + b0 * per_in, nb, d.c_in, n.split[0].halves, false, c->sp_l5, s);
+            }
+            SplitTrunk T{};
+            std::copy(n.split.begin(), n.split.end(), T.L);
+            T.nl = ntrunk;
+            T.B = nb;
+            T.act = d.act;
+            T.l5 = c->sp_l5;
+            T.buf[0] = c->sp_act[0];
+            T.buf[1] = c->sp_act[1];
+            T.cap_rows = c->split_batch * kL3Board;
+            T.pitch = n.split_pitch;
+            T.w = n.split_w;
+            T.out32 = c->act[0] + b0 * per_out;
+            T.flags = c->sp_flags;
+            T.err = c->d_err;
+            {
+                ProfScope ps(c, prof, LG_PROF_FP32_CONV, s);
+                if (int rc = launch_split_trunk(T, s, c->sm_count)) return rc;
+            }
+            L += 2;
+        }
+    } else {
+        {
+            ProfScope ps(c, prof, LG_PROF_OTHER, s);
+            launch_pack_planes_f32(planes, B, d.c_in, c->act[0], s);
+        }
+        ++L;
+        for (int l = 0; l < ntrunk; ++l) {
+            auto sh = n.shapes[l];
+            ProfScope ps(c, prof, LG_PROF_FP32_CONV, s);
+            launch_conv_f32(c->act[cur], n.wt[l], n.bias[l], c->act[cur ^ 1], B, sh.cin, sh.cout, sh.k,
+                            d.act, c->partial, s);
+            L += conv_f32_partial_floats(B, sh.cin, sh.cout, sh.k) ? 2 : 1;
+            cur ^= 1;
+        }
     }
     auto hs = n.shapes.back();
     float *lg = logits_out ? logits_out : c->d_logits;
     {
         ProfScope ps(c, prof, LG_PROF_OTHER, s);
-        launch_head_conv_f32(c->act[cur], n.head_w, n.head_b, B, hs.cin, hs.k, d.act_head, d.act, lg, s);
+        launch_head_conv_f32(c->act[cur], n.head_w, n.head_b, B, hs.cin, hs.k, d.act_head, d.act, lg, s, split);
     }
     ++L;
     {
         ProfScope ps(c, prof, LG_PROF_TAIL, s);
         HeadIn h{lg, 1, 0, 0.0f, 0, d.act, nullptr};
         if (!d.value_head)
-            launch_softmax(h, B, T, probs, s);
+            launch_softmax(h, B, T, probs, s, nullptr, split);
         else
             launch_value_fc(h, B, n.w1s, n.b1, n.w2, n.b2, d.fc_hidden, d.act, d.value_map, value,
-                            c->d_fcpart, c->d_fccnt, s);
+                            c->d_fcpart, c->d_fccnt, s, split);
     }
     ++L;
     *nlaunch = L;
@@ -1506,7 +1604,7 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
         return fail(LG_ERR_CUDA);
     const lg_net_desc *descs[2] = {policy, value};
     size_t max_act = 0, max_partial = 0, max_tc_l3 = 0, max_tc_l5 = 0;
-    int max_c_in = 0, max_fc = 0;
+    int max_c_in = 0, max_fc = 0, sp_pitch = 0, sp_halves = 0;
     for (int i = 0; i < 2; ++i) {
         if (!descs[i]) continue;
         if ((rc = build_net(c, c->nets[i], descs[i]))) return fail(rc);
@@ -1514,6 +1612,11 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
         max_c_in = std::max(max_c_in, n.d.c_in);
         if (n.d.value_head) max_fc = std::max(max_fc, n.d.fc_hidden);
         if (n.d.precision == LG_FP32) {
+            if (n.split_ok) {
+                if ((rc = split_init_device())) return fail(rc);
+                sp_pitch = std::max(sp_pitch, n.split_pitch);
+                sp_halves = std::max(sp_halves, n.split[0].halves);
+            }
             for (auto &s : n.shapes) {
                 max_act = std::max(max_act, (size_t)std::max(s.cin, s.cout));
                 for (int b = 1; b <= max_batch; b = (b < 64 ? b + 1 : b * 2))
@@ -1533,6 +1636,15 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
             (rc = dev_alloc(c, &c->act[1], mb * kPoints * max_act)) ||
             (rc = dev_alloc(c, &c->partial, max_partial)))
             return fail(rc);
+    }
+    if (sp_pitch) {
+        c->split_batch = std::min(max_batch, kSplitMaxBatch);
+        const size_t sb = (size_t)c->split_batch, nf = split_flag_ints(c->split_batch);
+        if ((rc = dev_alloc(c, &c->sp_act[0], 3 * sb * kL3Board * sp_pitch)) ||
+            (rc = dev_alloc(c, &c->sp_act[1], 3 * sb * kL3Board * sp_pitch)) ||
+            (rc = dev_alloc(c, &c->sp_l5, sb * kL5Board * sp_halves * 64)) || (rc = dev_alloc(c, &c->sp_flags, nf)))
+            return fail(rc);
+        if (cudaMemset(c->sp_flags, 0, nf * sizeof(int)) != cudaSuccess) return fail(LG_ERR_CUDA);
     }
     if (max_tc_l3) {
         if ((rc = dev_alloc(c, &c->l3[0], mb * kL3Board * max_tc_l3)) ||
@@ -1982,7 +2094,8 @@ extern "C" int lg_policy_device_static(lg_ctx *c, const uint8_t *planes, int B, 
 // tensor-core nets' forward with each kernel choice for the 3x3 layers and
 // for the first layer (256-row transposed kernel or 128-row kernel), keep
 // the fastest, and cache the table as JSON keyed by device name, SM count
-// and net widths.  FP32 nets have nothing to tune.
+// and net widths.  FP32 nets: the per-layer kernels, the split trunk and the
+// small-batch kernel.
 // ============================================================================
 
 namespace {
@@ -2022,6 +2135,7 @@ bool load_tuning(lg_ctx *c, const char *path) {
         table[b][1] = d;
     }
     std::memcpy(c->tc_variant, table, sizeof table);
+    std::fill(std::begin(c->chosen), std::end(c->chosen), true);
     return true;
 }
 
@@ -2064,12 +2178,13 @@ extern "C" int lg_autotune(lg_ctx *c, const char *cache_path, int force) {
         return LG_ERR_ARG;
     }
     std::lock_guard<std::mutex> g(c->mu);
-    bool any_tc = false, any_lat = false;
+    bool any_tc = false, any_lat = false, any_split = false;
     for (int i = 0; i < 2; ++i) {
         any_tc |= c->nets[i].present && c->nets[i].d.precision != LG_FP32;
+        any_split |= c->nets[i].present && c->nets[i].split_ok;
         any_lat |= c->nets[i].present && c->nets[i].lat_ok;
     }
-    if (!any_tc && !any_lat) return LG_OK;
+    if (!any_tc && !any_lat && !any_split) return LG_OK;
     if (cache_path && !force && load_tuning(c, cache_path)) {
         for (auto &gr : c->graphs) cudaGraphExecDestroy(gr.second.first);
         c->graphs.clear();
@@ -2093,9 +2208,11 @@ extern "C" int lg_autotune(lg_ctx *c, const char *cache_path, int force) {
         const int B = 1 << b;
         double best = 1e30;
         int best_v = 0;
+        c->chosen[b] = true;
         for (int v = 0; v < 8 && rc == LG_OK; ++v) {
             if (v == 7 && (B > kLatMaxB || !any_lat)) continue;
-            if (!any_tc && v != 0 && v != 7) continue;  // FP32 nets: per-layer or small-batch
+            // FP32 nets: per-layer kernels, split trunk or small-batch kernel
+            if (!any_tc && v != 0 && v != 7 && !(v == 6 && any_split)) continue;
             choice(v, c->tc_variant[b][0], c->tc_variant[b][1]);
             const int reps = B >= 64 ? 5 : 20;
             float t = 0.0f;
@@ -2159,6 +2276,7 @@ extern "C" int lg_set_tuning(lg_ctx *c, int B, int variant_3x3, int variant_firs
     while ((1 << bl) < B && bl < 16) ++bl;
     c->tc_variant[bl][0] = variant_3x3;
     c->tc_variant[bl][1] = variant_first;
+    c->chosen[bl] = true;
     for (auto &gr : c->graphs) cudaGraphExecDestroy(gr.second.first);
     c->graphs.clear();
     return LG_OK;

@@ -29,7 +29,39 @@ void launch_pack_planes_f32(const uint8_t *planes, int B, int C, float *out, cud
 void launch_conv_f32(const float *in, const float *wt, const float *bias, float *out, int B,
                      int C, int O, int k, int act, float *partial, cudaStream_t s);
 void launch_head_conv_f32(const float *in, const float *wh, float bias, int B, int C, int k,
-                          int do_act, int act, float *logits, cudaStream_t s);
+                          int do_act, int act, float *logits, cudaStream_t s, bool pdl = false);
+
+// FP32 conv layers on the tensor cores, each value as three BF16 parts
+// (split_conv.cu): the 5x5 first layer (planes already expanded to BF16 L5
+// rows) and the 3x3 layers of a net in one persistent launch.
+constexpr int kSpMaxLayers = 40;
+struct SplitLayer {
+    int halves;         // 64-channel halves of the input (first layer: of the L5 rows)
+    int groups;         // 64-channel groups of the output
+    int cout;           // output channels
+    const float *bias;  // [groups * 64], zero past cout
+};
+struct SplitTrunk {
+    SplitLayer L[kSpMaxLayers];
+    int nl, B, act;
+    const void *l5;          // [B * 399][L[0].halves * 64] BF16
+    __nv_bfloat16 *buf[2];   // [3][cap_rows][pitch] parts, L3 rows
+    int cap_rows, pitch;
+    const void *w;           // per layer [tap][half][group][part][64][64] BF16
+    float *out32;            // the last layer's output, [B * 361][cout]
+    int *flags;              // split_flag_ints(B) ints, zero between launches
+    int *err;
+};
+size_t split_flag_ints(int B);
+int split_pad(int channels);  // channels rounded up to whole groups
+// A layer's weights in that layout, made on the device from the FP32 path's
+// wt [k*k][cin][cout] (k = 5 for the first layer, else 3): elements, launch.
+size_t split_weight_elems(int k, int cin, int cout);
+void launch_split_weights(const float *wt, int k, int cin, int cout, __nv_bfloat16 *out, cudaStream_t s);
+int split_init_device();
+// A programmatic dependent of the previous kernel in the stream.
+int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count);
+
 // Input of the finish kernels: the head output of point (b, p) is
 //   act_head?(sum_k parts[k * part_stride + b * 361 + p] + head_b).
 // When logits_out is set the finish kernel also writes that value there.
@@ -290,5 +322,9 @@ void launch_avg8(const float *v, int B, float *out, cudaStream_t s);
 // Tensor-map encoding through the driver entry point (no -lcuda needed).
 int encode_map_2d_bf16(CUtensorMap *map, const void *base, uint64_t inner, uint64_t rows,
                        uint32_t box_inner, uint32_t box_rows, bool swizzle128 = true);
+// The same over `planes` arrays of rows, `plane_rows` rows apart; boxes of one
+// plane, 128-byte swizzle.  Rows outside [0, rows) of a plane read as zero.
+int encode_map_3d_bf16(CUtensorMap *map, const void *base, uint64_t inner, uint64_t rows, uint64_t planes,
+                       uint64_t plane_rows, uint32_t box_inner, uint32_t box_rows);
 
 }  // namespace lg

@@ -1532,8 +1532,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
 
 // (FP16 activations and weights move through the same maps: tiled copies do
 // not convert, the element type only fixes the 2-byte element size.)
-int encode_map_2d_bf16(CUtensorMap *map, const void *base, uint64_t inner, uint64_t rows,
-                       uint32_t box_inner, uint32_t box_rows, bool swizzle128) {
+static int encode_map(CUtensorMap *map, const void *base, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
+                      const cuuint32_t *box, bool swizzle128) {
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
         cudaDriverEntryPointQueryResult q;
@@ -1546,11 +1546,8 @@ int encode_map_2d_bf16(CUtensorMap *map, const void *base, uint64_t inner, uint6
         }
         fn = (EncodeTiledFn)f;
     }
-    cuuint64_t dims[2] = {inner, rows};
-    cuuint64_t strides[1] = {inner * 2};
-    cuuint32_t box[2] = {box_inner, box_rows};
-    cuuint32_t es[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides,
+    cuuint32_t es[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void *>(base), dims, strides,
                     box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1559,6 +1556,20 @@ int encode_map_2d_bf16(CUtensorMap *map, const void *base, uint64_t inner, uint6
         return LG_ERR_CUDA;
     }
     return LG_OK;
+}
+
+int encode_map_2d_bf16(CUtensorMap *map, const void *base, uint64_t inner, uint64_t rows,
+                       uint32_t box_inner, uint32_t box_rows, bool swizzle128) {
+    const cuuint64_t dims[2] = {inner, rows}, strides[1] = {inner * 2};
+    const cuuint32_t box[2] = {box_inner, box_rows};
+    return encode_map(map, base, 2, dims, strides, box, swizzle128);
+}
+
+int encode_map_3d_bf16(CUtensorMap *map, const void *base, uint64_t inner, uint64_t rows, uint64_t planes,
+                       uint64_t plane_rows, uint32_t box_inner, uint32_t box_rows) {
+    const cuuint64_t dims[3] = {inner, rows, planes}, strides[2] = {inner * 2, plane_rows * inner * 2};
+    const cuuint32_t box[3] = {box_inner, box_rows, 1};
+    return encode_map(map, base, 3, dims, strides, box, true);
 }
 
 }  // namespace lg
