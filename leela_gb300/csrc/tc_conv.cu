@@ -650,20 +650,20 @@ __global__ void __launch_bounds__(kTcThreadsT, 1)
 
 // ===========================================================================
 // Kernel "trunk": every 3x3 128->128 layer of a net in one persistent
-// launch, scheduled as work items (layer l, chunk j) of 256 rows (224 for
-// the fused 5x5 first layer's items).  The
-// producer of each CTA claims items from a global counter in (layer, chunk)
+// launch, scheduled as work items (layer l, chunk j) of TP = 256 rows (224
+// for the fused 5x5 first layer's items), 128 or 64 for small batches
+// (trunk_tp).  The producer of each CTA claims items from a global counter in (layer, chunk)
 // order and runs kernel T's pipeline over each (its windows, weight stages,
 // MMAs, epilogue), ping-ponging between two L3 buffers (layer l reads A when
-// l is even, B when odd).  Item (l, j) reads rows [256j - 24, 256j + 280) of
-// layer l-1's output, written by items (l-1, j-1 .. j+1), and overwrites rows
+// l is even, B when odd).  Item (l, j) reads rows [TP j - 24, TP (j + 1) + 24)
+// of layer l-1's output, written by items (l-1, j-1 .. j+1), and overwrites rows
 // that only those items read for layer l-1: so it starts once flags[j-1 ..
 // j+1] >= l.  flags[j] = number of layers whose chunk-j rows are stored
 // (published with release after the item's TMA stores completed; the
 // producer polls with acquire, bounded).  Items are claimed in order, so an
 // item's dependencies were claimed earlier by CTAs that are running: there
 // is no layer-wide barrier, faster SMs take more items, and every item but a
-// layer's last runs at N = 256.  The last layer can carry the fused 1x1 head.
+// layer's last runs at N = TP.  The last layer can carry the fused 1x1 head.
 // ===========================================================================
 
 struct TrunkParams {
@@ -707,34 +707,40 @@ struct TrunkCtl {
 };
 
 // Shared memory of kernel "trunk": three half-window slots, four staging
-// tiles, five weight stages, the control block.  A 3x3 item covers 256 rows
-// (window 256 + 2 x 24); a first-layer item covers 224 rows so that its
-// window (5 taps of pitch 19: 224 + 2 x 40) fits the same slot: the fifth
-// weight stage lives in the bytes a taller slot would take.  The buffers
-// start at the first 1024-byte boundary of the dynamic region (the 128-byte
-// swizzle's alignment); PAD is the slack left for that.
+// tiles, weight stages in what is left, the control block.  A 3x3 item covers
+// TP rows (window TP + 2 x 24); a first-layer item covers TP5 rows (5 taps of
+// pitch 19: TP5 + 2 x 40): 224 beside TP = 256, so that its window fits the
+// same slot and a fifth weight stage the bytes a taller slot would take.  The
+// buffers start at the first 1024-byte boundary of the dynamic region (the
+// 128-byte swizzle's alignment); PAD is the slack left for that.
+template <int TP_>
 struct TrunkCfg {
     using C0 = TcTCfg<2, 0>;
     using C1 = TcTCfg<2, 1>;
-    static constexpr int TP = 256;
-    static constexpr int TP5 = 224;
+    static constexpr int TP = TP_;
+    static constexpr int TP5 = TP == 256 ? 224 : TP;
+    static constexpr int WIN_ROWS = TP + 2 * C0::WPRE;
+    static constexpr int SUB = WIN_ROWS / 2;  // TMA box rows of a half-window
+    static constexpr int WIN_HALF = WIN_ROWS * 128;
     static constexpr int WIN5_ROWS = TP5 + 2 * C1::WPRE;
-    static constexpr int SUB5 = WIN5_ROWS / 2;  // TMA box rows of a first-layer half-window
+    static constexpr int SUB5 = WIN5_ROWS / 2;
     static constexpr int WIN5_HALF = WIN5_ROWS * 128;
+    static constexpr int RG = TP >= 128 ? TP / 4 : 32;  // rows of an epilogue row group
+    static constexpr int NH = RG / 32;                  // 32-row steps of a group
     static constexpr int NWIN = 3;
-    static constexpr int WIN_SLOT = WIN5_HALF > C0::WIN_HALF ? WIN5_HALF : C0::WIN_HALF;
-    static constexpr int S = 5;
+    static constexpr int WIN_SLOT = WIN5_HALF > WIN_HALF ? WIN5_HALF : WIN_HALF;
     static constexpr int WST_BYTES = C0::WST_BYTES;
     static constexpr int STG_BYTES = C0::STG_BYTES;
     static constexpr int STG_TOTAL = 4 * STG_BYTES;
+    static constexpr int SMEM = 227 * 1024;
+    static constexpr int S = (SMEM - 512 - NWIN * WIN_SLOT - STG_TOTAL) / WST_BYTES;
     using Ctl = TrunkCtl<NWIN, S>;
     static constexpr int CTL_OFF = NWIN * WIN_SLOT + STG_TOTAL + S * WST_BYTES;
-    static constexpr int SMEM = 227 * 1024;
     static constexpr int PAD = SMEM - CTL_OFF - (int)sizeof(Ctl);
-    static_assert(C0::TP == TP && TP5 % 16 == 0 && TP5 <= TP, "item rows");
-    static_assert(WIN_SLOT % 1024 == 0 && (C0::SUBROWS * 128) % 1024 == 0 && (SUB5 * 128) % 1024 == 0,
+    static_assert(TP5 % 16 == 0 && TP5 <= TP && TP % 64 == 0, "item rows");
+    static_assert(WIN_SLOT % 1024 == 0 && (SUB * 128) % 1024 == 0 && (SUB5 * 128) % 1024 == 0,
                   "window boxes keep the 1024-byte swizzle alignment");
-    static_assert(CTL_OFF % 8 == 0 && PAD >= 0, "shared memory budget");
+    static_assert(S >= 5 && CTL_OFF % 8 == 0 && PAD >= 0, "shared memory budget");
 };
 
 // The MMAs of one 64-channel half of an item: NTAPS weight stages (one per
@@ -763,22 +769,29 @@ __device__ __forceinline__ bool issue_taps(uint32_t d_tmem, uint64_t a_desc0, ui
     return true;
 }
 
-__device__ __forceinline__ bool poll_flag(const int *f, int want, uint32_t limit) {
-    uint32_t n = 0;
-    while (ld_acquire_gpu(f) < want && ++n < limit) __nanosleep(64);
-    return n < limit;
+// A converged warp waits until the n counters at f all reach `want`, a lane
+// each (polled one after another they cost up to 2 us of an item's start).
+__device__ __forceinline__ bool poll_flags(const int *f, int n, int want, uint32_t limit) {
+    const int lane = threadIdx.x % 32;
+    bool ok = true;
+    for (int i = lane; i < n; i += 32) {
+        uint32_t k = 0;
+        while (ld_acquire_gpu(f + i) < want && ++k < limit) __nanosleep(32);
+        ok = ok && k < limit;
+    }
+    return __all_sync(0xffffffffu, ok);
 }
 
-template <bool HEAD, bool F16>
+template <int TP, bool HEAD, bool F16>
 __global__ void __maxnreg__(96)
     tc_trunk_kernel(const __grid_constant__ CUtensorMap in_a, const __grid_constant__ CUtensorMap in_b,
                     const __grid_constant__ CUtensorMap out_a, const __grid_constant__ CUtensorMap out_b,
                     const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap in5,
                     const __grid_constant__ CUtensorMap w0_map, const __grid_constant__ CUtensorMap out_a_sw,
                     const __grid_constant__ CUtensorMap out_b_sw, const TrunkParams p) {
-    using C = TrunkCfg;
-    using C0 = TrunkCfg::C0;
-    using C1 = TrunkCfg::C1;
+    using C = TrunkCfg<TP>;
+    using C0 = typename C::C0;
+    using C1 = typename C::C1;
     constexpr int HALVES = 2, NO = 128;
     extern __shared__ uint8_t smem_raw[];
     // The buffers need a 1024-byte aligned base; with no static shared
@@ -793,7 +806,7 @@ __global__ void __maxnreg__(96)
     uint8_t *win = smem;
     uint8_t *stg = smem + C::NWIN * C::WIN_SLOT;
     uint8_t *wst = stg + C::STG_TOTAL;
-    TrunkCfg::Ctl &ctl = *reinterpret_cast<TrunkCfg::Ctl *>(smem + C::CTL_OFF);
+    typename C::Ctl &ctl = *reinterpret_cast<typename C::Ctl *>(smem + C::CTL_OFF);
     uint64_t *const win_full = ctl.win_full, *const win_empty = ctl.win_empty;
     uint64_t *const w_full = ctl.w_full, *const w_empty = ctl.w_empty;
     // item_done: a ring of 4 (an epilogue warp can be up to two items ahead
@@ -891,9 +904,11 @@ __global__ void __maxnreg__(96)
 
     if (warp == kEpiWarpsT + 2) {
         // ------------------------------------------------ item claims + windows
-        if (lane == 0) {
-            uint32_t wn = 0;
-            for (int q = 0;; ++q) {
+        // Lane 0 claims and loads, the whole warp polls the dependencies.
+        uint32_t wn = 0;
+        for (int q = 0;; ++q) {
+            int it = -1;
+            if (lane == 0) {
                 const int slot = q % kItemRing;
                 const uint32_t qk = (uint32_t)(q / kItemRing);
                 // Claim only once the item ring and the next window slot are
@@ -901,7 +916,6 @@ __global__ void __maxnreg__(96)
                 bool ok = mbar_wait(&item_empty[slot], (qk & 1) ^ 1, WAIT_LIM);
                 const int ws0 = wn % C::NWIN;
                 ok = ok && mbar_wait(&win_empty[ws0], ((wn / C::NWIN) & 1) ^ 1, WAIT_LIM);
-                int it = -1;
                 if (ok && !abort_flag) {
                     it = atomicAdd(p.flags + n3L, 1);
                     if (it >= nitems) it = -1;
@@ -910,54 +924,59 @@ __global__ void __maxnreg__(96)
                 }
                 item_id[slot] = it;
                 mbar_arrive(&item_full[slot]);  // releases item_id[slot]
-                if (it < 0) break;
-                int l, j;
-                decode(it, l, j);
-                const bool fl = first && l == 0;
-                const int k = l - first;  // 3x3 layer index
-                if (!fl && k == 0 && first) {
+            }
+            it = __shfl_sync(0xffffffffu, it, 0);
+            if (it < 0) break;
+            int l, j;
+            decode(it, l, j);
+            const bool fl = first && l == 0;
+            const int k = l - first;  // 3x3 layer index
+            if (!fl && (k > 0 || first)) {
+                const int *f;
+                int nf, want;
+                if (k == 0) {
                     // the first layer's chunks whose L5 rows feed L3 rows
-                    // [256j - 24, 256j + 280): an L5 row is the L3 row minus
-                    // (board + y), board + y <= rows / 400 + 19
+                    // [TP j - 24, TP (j + 1) + 24): an L5 row is the L3 row
+                    // minus (board + y), board + y <= rows / 400 + 19
                     const int lo3 = max(0, j * C::TP - C0::WPRE);
                     const int hi3 = min(rows, j * C::TP + C::TP + C0::WPRE);
-                    const int lo5 = max(0, lo3 - (hi3 - 1) / kL3Board - kBoard);
-                    const int hi5 = min(rows5 - 1, hi3 - 1);
-                    for (int jj = lo5 / C::TP5; jj <= hi5 / C::TP5; ++jj)
-                        if (!poll_flag(flags0 + jj, 1, p.poll_limit)) {
-                            fail(71);
-                            goto done_windows;
-                        }
-                    fence_proxy_async_global();
-                } else if (!fl && k > 0) {
+                    const int lo5 = max(0, lo3 - (hi3 - 1) / kL3Board - kBoard) / C::TP5;
+                    f = flags0 + lo5;
+                    nf = min(rows5 - 1, hi3 - 1) / C::TP5 - lo5 + 1;
+                    want = 1;
+                } else {
                     // layer k-1 of chunks j-1 .. j+1 is stored
-                    const int lo = max(0, j - 1), hi = min(n3 - 1, j + 1);
+                    const int lo = max(0, j - 1);
+                    f = p.flags + lo;
+                    nf = min(n3 - 1, j + 1) - lo + 1;
                     // (test hook: the stalled item waits for a layer count
                     // no item ever publishes)
-                    const int want = it == p.stall_item ? (1 << 30) : k;
-                    for (int jj = lo; jj <= hi; ++jj)
-                        if (!poll_flag(p.flags + jj, want, p.poll_limit)) {
-                            fail(71);
-                            goto done_windows;
-                        }
-                    fence_proxy_async_global();
+                    want = it == p.stall_item ? (1 << 30) : k;
                 }
+                if (!poll_flags(f, nf, want, p.poll_limit)) {
+                    if (lane == 0) fail(71);
+                    break;
+                }
+                fence_proxy_async_global();
+                __syncwarp();
+            }
+            if (lane == 0) {
                 const CUtensorMap *im = fl ? &in5 : ((k & 1) ? &in_b : &in_a);
-                const int sub = fl ? C::SUB5 : C0::SUBROWS;
-                const uint32_t bytes = fl ? C::WIN5_HALF : C0::WIN_HALF;
+                const int sub = fl ? C::SUB5 : C::SUB;
+                const uint32_t bytes = fl ? C::WIN5_HALF : C::WIN_HALF;
                 const int row0 = fl ? j * C::TP5 - C1::WPRE : j * C::TP - C0::WPRE;
-                for (int h = 0; h < HALVES; ++h, ++wn) {
-                    const int ws = wn % C::NWIN;
-                    const uint32_t wk = wn / C::NWIN;
+                for (int h = 0; h < HALVES; ++h) {
+                    const int ws = (wn + h) % C::NWIN;
+                    const uint32_t wk = (wn + h) / C::NWIN;
                     // (the first half's slot was waited for before the claim)
-                    if (h > 0 && !mbar_wait(&win_empty[ws], (wk & 1) ^ 1, WAIT_LIM)) { fail(73); goto done_windows; }
+                    if (h > 0 && !mbar_wait(&win_empty[ws], (wk & 1) ^ 1, WAIT_LIM)) { fail(73); break; }
                     mbar_arrive_expect_tx(&win_full[ws], bytes);
                     for (int sb = 0; sb < 2; ++sb)
                         tma_load_2d(win + ws * C::WIN_SLOT + sb * sub * 128, im, &win_full[ws], h * 64,
                                     row0 + sb * sub);
                 }
             }
-        done_windows:;
+            wn += HALVES;
         }
     } else if (warp == 0) {
         // ------------------------------------------------ weight stages
@@ -1014,7 +1033,7 @@ __global__ void __maxnreg__(96)
                 const uint32_t ak = (uint32_t)(q >> 1);
                 if (!mbar_wait(&acc_empty[acc], (ak & 1) ^ 1, WAIT_LIM)) { fail(76); break; }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem + (uint32_t)(acc * C::TP);
+                const uint32_t d_tmem = tmem + (uint32_t)(acc * 256);
                 bool ok = true;
 #pragma unroll
                 for (int h = 0; h < HALVES && ok; ++h, ++wn) {
@@ -1064,13 +1083,13 @@ __global__ void __maxnreg__(96)
             const CUtensorMap *om = (k & 1) ? &out_a : &out_b;
             const int rows_l = fl ? rows5 : rows;
             const int nrows = min(fl ? C::TP5 : C::TP, rows_l - cs);
-            const int nhalf = max(0, min(2, (nrows - rq * 64 + 31) / 32));
+            const int nhalf = max(0, min(C::NH, (nrows - rq * C::RG + 31) / 32));
             const int acc = q & 1;
             const uint32_t ak = (uint32_t)(q >> 1);
             if (!mbar_wait(&acc_full[acc], ak & 1, WAIT_LIM)) { fail(80); break; }
             tc_fence_after();
-            const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * C::TP + rq * 64);
-            const int q_base = cs + rq * 64;
+            const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256 + rq * C::RG);
+            const int q_base = cs + rq * C::RG;
             bool bad = false;
             // 3x3 ReLU items take the fragment path: TMEM read as the MMA
             // accumulator fragments (16x256b: thread t holds channels
@@ -1093,12 +1112,12 @@ __global__ void __maxnreg__(96)
                 const uint32_t st_addr =
                     stg_half + (lane & 7) * 128 + (((((quarter & 1) * 4) + (lane >> 3)) ^ (lane & 7)) * 16);
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
+                for (int c = 0; c < C::NH; ++c) {
                     uint32_t r0[16], r1[16];
                     tmem_ld16x256_x4(t_base + 32 * c, r0);
                     tmem_ld16x256_x4(t_base + (16u << 16) + 32 * c, r1);
                     tmem_ld_wait();
-                    if (c == 1) {
+                    if (c == C::NH - 1) {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&acc_empty[acc]);
@@ -1155,7 +1174,7 @@ __global__ void __maxnreg__(96)
                 }
             }
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int c = 0; c < C::NH; ++c) {
                 if (!fl && !head_layer && p.act == LG_ACT_RELU) break;
                 // One 32-row half at a time (32 registers); the accumulator is
                 // released after the second half's load, which the MMA issuer
@@ -1163,7 +1182,7 @@ __global__ void __maxnreg__(96)
                 uint32_t v[32];
                 tmem_ld32(t_base + 32 * c, v);
                 tmem_ld_wait();
-                if (c == 1) {
+                if (c == C::NH - 1) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&acc_empty[acc]);
@@ -1271,8 +1290,9 @@ __global__ void __maxnreg__(96)
                     if (!mbar_wait(&item_done[done_n & 3], (done_n >> 2) & 1, WAIT_LIM)) {
                         fail(83);
                     } else {
+                        // (the release covers the stores of the warps that
+                        // arrived: no fence of its own)
                         fence_proxy_async_global();
-                        __threadfence();
                         if (fl)
                             st_release_gpu(flags0 + j, 1);
                         else
@@ -1340,9 +1360,11 @@ int tc_init_device() {
     LG_A(64, 1, 0, false) LG_A(64, 1, 0, true) LG_A(64, 2, 1, false) LG_A(64, 3, 1, false)
     LG_A(128, 3, 1, false) LG_A(128, 2, 0, false) LG_A(128, 2, 0, true) LG_A(128, 2, 1, false)
     LG_T(2, 0, false) LG_T(2, 0, true) LG_T(2, 1, false)
-#define LG_TR(HD_, F_) \
-    if (!rc) rc = set_attr<decltype(&tc_trunk_kernel<HD_, F_>), TrunkCfg::SMEM>(tc_trunk_kernel<HD_, F_>);
-    LG_TR(false, false) LG_TR(true, false) LG_TR(false, true) LG_TR(true, true)
+#define LG_TR(TP_, HD_, F_) \
+    if (!rc) rc = set_attr<decltype(&tc_trunk_kernel<TP_, HD_, F_>), TrunkCfg<TP_>::SMEM>(tc_trunk_kernel<TP_, HD_, F_>);
+    LG_TR(256, false, false) LG_TR(256, true, false) LG_TR(256, false, true) LG_TR(256, true, true)
+    LG_TR(128, false, false) LG_TR(128, true, false) LG_TR(128, false, true) LG_TR(128, true, true)
+    LG_TR(64, false, false) LG_TR(64, true, false) LG_TR(64, false, true) LG_TR(64, true, true)
 #undef LG_TR
 #undef LG_A
 #undef LG_T
@@ -1354,14 +1376,28 @@ int tc_init_device() {
 // (variant 1) and the 64-wide nets (kernel A sums all channels per row).
 int tc_head_parts(int n, int variant) { return (n == 128 && variant != 1) ? 4 : 1; }
 
+// Rows per item.  A layer is one item a CTA or less for small batches, so its
+// time is one item's: the hand-off from the layer before (flags, window load,
+// stores: ~5 us, the same for every size) and 72 MMAs of N = rows.  64-row
+// items while every SM has at most one (24 positions), 128-row items while
+// 256-row ones would leave SMs without any (97); then the largest, whose MMAs
+// run at the full rate and read each weight stage for the most rows.  Policy +
+// value pair, us, with 64 / 128 / 256 rows: 8 positions 217 / 220 / 253, 24
+// positions 233 / 235 / 269, 48 positions 277 / 252 / 283, 96 positions
+// 486 / 294 / 300, 128 positions 633 / 356 / 316.  Every output is the same
+// accumulation whatever the item's size: the results are bit for bit equal.
+static int trunk_tp(int rows) { return rows <= 64 * 152 ? 64 : (rows <= 256 * 152 ? 128 : 256); }
+static int trunk_tp5(int tp) { return tp == 256 ? TrunkCfg<256>::TP5 : tp; }
+
 size_t trunk_flag_ints(int rows, int rows5) {
-    // chunk flags, item counter, first-layer chunk flags, exit counter
-    return (size_t)(rows + TrunkCfg::TP - 1) / TrunkCfg::TP + 1 + (size_t)(rows5 + TrunkCfg::TP5 - 1) / TrunkCfg::TP5 +
-           1;
+    // chunk flags, item counter, first-layer chunk flags, exit counter; for
+    // any item size
+    return (size_t)(rows + 63) / 64 + 1 + (size_t)(rows5 + 63) / 64 + 1;
 }
 
 int trunk_layer_item(int rows, int rows5, int k) {
-    return (rows5 + TrunkCfg::TP5 - 1) / TrunkCfg::TP5 + k * ((rows + TrunkCfg::TP - 1) / TrunkCfg::TP);
+    const int tp = trunk_tp(rows), tp5 = trunk_tp5(tp);
+    return (rows5 + tp5 - 1) / tp5 + k * ((rows + tp - 1) / tp);
 }
 
 template <int N, int HALVES, int KIND, bool HEAD>
@@ -1393,18 +1429,20 @@ static int launch_t(const TcLayer &L, TcParams p, cudaStream_t s, int sm_count) 
     return LG_OK;
 }
 
-int launch_tc_trunk(const TcTrunk &T, float *parts, size_t part_stride, int *flags, int *err,
-                    cudaStream_t s, int sm_count) {
-    using C0 = TrunkCfg::C0;
-    using C1 = TrunkCfg::C1;
+template <int TP>
+static int launch_trunk_tp(const TcTrunk &T, float *parts, size_t part_stride, int *flags, int *err, cudaStream_t s,
+                           int sm_count) {
+    using Cfg = TrunkCfg<TP>;
+    using C0 = typename Cfg::C0;
+    using C1 = typename Cfg::C1;
     const bool fused = T.buf5 != nullptr;
     if (T.nl < 1 || T.rows <= 0 || (T.head_w && !parts) || (fused && (T.rows5 <= 0 || !T.w0 || !T.bias0))) {
         lg_set_error("launch_tc_trunk: bad arguments");
         return LG_ERR_ARG;
     }
     CUtensorMap in_a, in_b, out_a, out_b, w_map, in5, w0_map, out_a_sw, out_b_sw;
-    int rc = encode_map_2d_bf16(&in_a, T.buf_a, 128, (uint64_t)T.rows, 64, C0::SUBROWS);
-    if (!rc) rc = encode_map_2d_bf16(&in_b, T.buf_b, 128, (uint64_t)T.rows, 64, C0::SUBROWS);
+    int rc = encode_map_2d_bf16(&in_a, T.buf_a, 128, (uint64_t)T.rows, 64, Cfg::SUB);
+    if (!rc) rc = encode_map_2d_bf16(&in_b, T.buf_b, 128, (uint64_t)T.rows, 64, Cfg::SUB);
     if (!rc) rc = encode_map_2d_bf16(&out_a, T.buf_a, 128, (uint64_t)T.rows, 128, 32, false);
     if (!rc) rc = encode_map_2d_bf16(&out_b, T.buf_b, 128, (uint64_t)T.rows, 128, 32, false);
     // the fragment-path epilogue's stores: 64-channel boxes from 128-byte
@@ -1413,7 +1451,7 @@ int launch_tc_trunk(const TcTrunk &T, float *parts, size_t part_stride, int *fla
     if (!rc) rc = encode_map_2d_bf16(&out_b_sw, T.buf_b, 128, (uint64_t)T.rows, 64, 32, true);
     if (!rc) rc = encode_map_2d_bf16(&w_map, T.w, 64, (uint64_t)T.nl * C0::NTAPS * 2 * 128, 64, 128);
     if (fused) {
-        if (!rc) rc = encode_map_2d_bf16(&in5, T.buf5, 128, (uint64_t)T.rows5, 64, TrunkCfg::SUB5);
+        if (!rc) rc = encode_map_2d_bf16(&in5, T.buf5, 128, (uint64_t)T.rows5, 64, Cfg::SUB5);
         if (!rc) rc = encode_map_2d_bf16(&w0_map, T.w0, 64, (uint64_t)C1::NTAPS * 2 * 128, 64, 128);
     } else {
         in5 = in_a;  // unused
@@ -1440,13 +1478,13 @@ int launch_tc_trunk(const TcTrunk &T, float *parts, size_t part_stride, int *fla
     p.wait_limit = T.wait_limit ? T.wait_limit : kWaitLimit;
     p.poll_limit = T.poll_limit ? T.poll_limit : kFlagPolls;
     p.stall_item = T.stall_item;
-    const int n3 = (T.rows + TrunkCfg::TP - 1) / TrunkCfg::TP;
-    const int n5 = fused ? (T.rows5 + TrunkCfg::TP5 - 1) / TrunkCfg::TP5 : 0;
+    const int n3 = (T.rows + Cfg::TP - 1) / Cfg::TP;
+    const int n5 = fused ? (T.rows5 + Cfg::TP5 - 1) / Cfg::TP5 : 0;
     const int grid = std::min(n5 + T.nl * n3, sm_count);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kTrunkThreads);
-    cfg.dynamicSmemBytes = TrunkCfg::SMEM;
+    cfg.dynamicSmemBytes = Cfg::SMEM;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     if (T.pdl) {
@@ -1463,20 +1501,29 @@ int launch_tc_trunk(const TcTrunk &T, float *parts, size_t part_stride, int *fla
     cfg.numAttrs = 1;
     cudaError_t e;
     if (T.f16)
-        e = T.head_w ? cudaLaunchKernelEx(&cfg, tc_trunk_kernel<true, true>, in_a, in_b, out_a, out_b, w_map, in5,
+        e = T.head_w ? cudaLaunchKernelEx(&cfg, tc_trunk_kernel<TP, true, true>, in_a, in_b, out_a, out_b, w_map, in5,
                                           w0_map, out_a_sw, out_b_sw, p)
-                     : cudaLaunchKernelEx(&cfg, tc_trunk_kernel<false, true>, in_a, in_b, out_a, out_b, w_map, in5,
+                     : cudaLaunchKernelEx(&cfg, tc_trunk_kernel<TP, false, true>, in_a, in_b, out_a, out_b, w_map, in5,
                                           w0_map, out_a_sw, out_b_sw, p);
     else
-        e = T.head_w ? cudaLaunchKernelEx(&cfg, tc_trunk_kernel<true, false>, in_a, in_b, out_a, out_b, w_map, in5,
+        e = T.head_w ? cudaLaunchKernelEx(&cfg, tc_trunk_kernel<TP, true, false>, in_a, in_b, out_a, out_b, w_map, in5,
                                           w0_map, out_a_sw, out_b_sw, p)
-                     : cudaLaunchKernelEx(&cfg, tc_trunk_kernel<false, false>, in_a, in_b, out_a, out_b, w_map, in5,
+                     : cudaLaunchKernelEx(&cfg, tc_trunk_kernel<TP, false, false>, in_a, in_b, out_a, out_b, w_map, in5,
                                           w0_map, out_a_sw, out_b_sw, p);
     if (e != cudaSuccess) {
         lg_set_error("trunk launch: %s", cudaGetErrorString(e));
         return LG_ERR_CUDA;
     }
     return LG_OK;
+}
+
+int launch_tc_trunk(const TcTrunk &T, float *parts, size_t part_stride, int *flags, int *err,
+                    cudaStream_t s, int sm_count) {
+    switch (trunk_tp(T.rows)) {
+    case 64: return launch_trunk_tp<64>(T, parts, part_stride, flags, err, s, sm_count);
+    case 128: return launch_trunk_tp<128>(T, parts, part_stride, flags, err, s, sm_count);
+    default: return launch_trunk_tp<256>(T, parts, part_stride, flags, err, s, sm_count);
+    }
 }
 
 size_t tc_conv_smem_bytes(int n, int ntaps, int cin_halves) {
