@@ -639,7 +639,7 @@ int bucket_of(int B) {
 // small-batch kernel for it from 3 positions on: that kernel's time grows
 // with the batch (benchmark nets, policy + value pair: 179, 313, 447, 715,
 // 1118 us at 1, 2, 3, 5, 8 positions), the split trunk's items run side by
-// side (430 to 443 us over the same sizes).  A hand-set choice 0 stays the
+// side (317 to 328 us over the same sizes).  A hand-set choice 0 stays the
 // FFMA kernels per layer (at 256 positions 14.3 ms a pair against 3.0).
 constexpr int kLatSplitB = 2;
 bool use_lat(lg_ctx *c, const Net &n, int B) {

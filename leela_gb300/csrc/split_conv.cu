@@ -24,7 +24,8 @@
 // (FFMA kernels 6.9e-7 to 1.64e-6, growing with the batch as their K splits
 // go; 64-deep chains gain nothing over a whole net and cost 10%).
 //
-// GEMM shape: M = 128 flat rows (the L3 / L5 layouts of lg_common.cuh: a tap
+// GEMM shape (NO = 64 output channels an item; 32 for small batches, with
+// half the N): M = 128 flat rows (the L3 / L5 layouts of lg_common.cuh: a tap
 // is a row shift, the window of rows is loaded once and read at 9 or 5
 // offsets), N = the weight parts of 64 output channels side by side:
 //   xh x [wh wm wl] -> columns 0..191, xm x [wh wm] -> columns 64..191,
@@ -34,11 +35,11 @@
 // for each of the six products alone: 92% of the MMA rate.
 //
 // One persistent launch runs all layers of a net: items (layer, 128-row tile,
-// 64-channel group) claimed in order from a counter; an item starts once the
+// NO-channel group) claimed in order from a counter; an item starts once the
 // tiles that its window covers are complete in the layer before (counters,
 // bounded polls).  A layer has at least two items a tile, so no SM waits at
 // a layer's end for more than its own dependencies.  Per CTA (one per SM):
-//   warp 0     weight stages (a tap x 64 channels x 3 parts: 24 KB, ring of 3)
+//   warp 0     weight stages (a tap x 64 channels x 3 parts: 24 KB, ring of 3, or 6 of 12 KB)
 //   warp 1     MMA issuer, TMEM owner
 //   warp 2     item claims, dependency polls, windows (2 slots: one 64-channel
 //              half of 3 parts x 176 rows each)
@@ -71,39 +72,47 @@ constexpr int kSpEpiWarps = 8;                    // per epilogue group
 constexpr int kSpGroups = 2;                      // epilogue groups, taking items in turn
 constexpr int kSpThreads = 128 + kSpGroups * kSpEpiWarps * 32;
 constexpr int kSpTile = 128;                      // rows per item
-constexpr int kSpNO = 64;                         // output channels per item
 constexpr int kSpPre3 = 24, kSpPre5 = 40;         // window rows before the tile
 constexpr int kSpWin3 = kSpTile + 2 * kSpPre3;    // 176
 constexpr int kSpWin5 = kSpTile + 2 * kSpPre5;    // 208
 constexpr int kSpPart = kSpWin3 * 128;            // bytes of one part's window
 constexpr int kSpSlot = 3 * kSpPart;
 constexpr int kSpSlots = 2;
-constexpr int kSpStage = 3 * kSpNO * 128;
-constexpr int kSpStages = 3;
 constexpr int kSpChain = 2;                       // taps (of 64 channels) per accumulator chain
 constexpr int kSpRing = 4;                        // item descriptors in flight
 constexpr uint32_t kSpWait = 1u << 21;
 constexpr uint32_t kSpPolls = 1u << 22;
 static_assert(kSpWin5 * 128 <= kSpSlot, "a first-layer window fits a slot");
-static_assert(kSpPart % 1024 == 0 && kSpSlot % 1024 == 0 && kSpStage % 1024 == 0, "swizzle alignment");
+static_assert(kSpPart % 1024 == 0 && kSpSlot % 1024 == 0, "swizzle alignment");
 
+// NO = output channels per item.  Weight stages: NO rows of each part.
+constexpr int kSpMaxStages = 6;
 struct SpCtl {
-    uint64_t win_full[kSpSlots], win_empty[kSpSlots], w_full[kSpStages], w_empty[kSpStages];
+    uint64_t win_full[kSpSlots], win_empty[kSpSlots], w_full[kSpMaxStages], w_empty[kSpMaxStages];
     uint64_t acc_full[kSpGroups][2], acc_empty[2], item_full[kSpRing], item_empty[kSpRing], mma_done;
     int item_id[kSpRing];
     uint32_t tmem_base;
     int abort_flag, last_out;
 };
 constexpr int kSpTileBytes = 32 * 32;             // an epilogue warp's staging tile
-constexpr int kSpStgOff = kSpSlots * kSpSlot + kSpStages * kSpStage;
-constexpr int kSpCtlOff = kSpStgOff + kSpGroups * kSpEpiWarps * kSpTileBytes;
-constexpr int kSpSmem = kSpCtlOff + (int)sizeof(SpCtl) + 1024;
-static_assert(kSpSmem <= 227 * 1024, "shared memory budget");
+template <int NO_>
+struct SpCfg {
+    static constexpr int NO = NO_;
+    static constexpr int STAGE = 3 * NO * 128;
+    static constexpr int STAGES = kSpMaxStages * 32 / NO;
+    static constexpr int CH = NO / 2;             // channels of an epilogue warp
+    static constexpr int ACC = NO == 64 ? 256 : 128;  // columns between accumulators
+    static constexpr int STG_OFF = kSpSlots * kSpSlot + STAGES * STAGE;
+    static constexpr int CTL_OFF = STG_OFF + kSpGroups * kSpEpiWarps * kSpTileBytes;
+    static constexpr int SMEM = CTL_OFF + (int)sizeof(SpCtl) + 1024;
+    static_assert(STAGE % 1024 == 0 && STAGES <= kSpMaxStages && SMEM <= 227 * 1024, "shared memory budget");
+};
 
 struct SpLayerDev {
     int first;        // 5x5 first layer (L5 rows, planes: one part), else 3x3 (L3 rows)
     int halves;       // 64-channel halves of the input
-    int groups;       // 64-channel groups of the output
+    int groups;       // NO-channel groups of the output
+    int wgroups;      // 64-channel groups in the weight layout
     int wrow;         // first row of the layer's weights in the weight map
     int item0;        // first item
     int need;         // tile counter value at which the layer before is complete
@@ -124,10 +133,15 @@ struct SpParams {
     int *err;
 };
 
-__device__ __forceinline__ bool sp_poll(const int *f, int want) {
-    uint32_t n = 0;
-    while (ld_acquire_gpu(f) < want && ++n < kSpPolls) __nanosleep(32);
-    return n < kSpPolls;
+// A converged warp waits until the n counters at f reach `want`, a lane each.
+__device__ __forceinline__ bool sp_poll(const int *f, int n, int want) {
+    bool ok = true;
+    for (int i = threadIdx.x % 32; i < n; i += 32) {
+        uint32_t k = 0;
+        while (ld_acquire_gpu(f + i) < want && ++k < kSpPolls) __nanosleep(32);
+        ok = ok && k < kSpPolls;
+    }
+    return __all_sync(0xffffffffu, ok);
 }
 
 // x as three BF16 parts, h = rn(x), m = rn(x - h), l = x - h - m (exact).
@@ -206,37 +220,38 @@ __device__ __forceinline__ void store_zero_parts(__nv_bfloat16 *dst, size_t part
 #pragma unroll
     for (int p = 0; p < 3; ++p)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) reinterpret_cast<uint4 *>(dst + p * part_stride)[i] = z;
+        for (int i = 0; i < 2; ++i) reinterpret_cast<uint4 *>(dst + p * part_stride)[i] = z;
 }
 
 // The MMAs of one 64-channel half of an item, chains of kSpChain taps: the
 // window in the slot of descriptor x, weight stages g, g + 1, ... of the
 // ring.  Called by a converged warp.  False if a wait ran out.
-template <bool FIRST>
+template <int NO, bool FIRST>
 __device__ __forceinline__ bool issue_half(SpCtl &ctl, uint32_t tmem, uint64_t x, uint64_t w_desc, int group,
                                            uint32_t &g, uint32_t &chain) {
     constexpr int NT = FIRST ? 5 : 9;
-    constexpr uint32_t id192 = idesc_bf16(128, 192), id128 = idesc_bf16(128, 128), id64 = idesc_bf16(128, 64);
+    using C = SpCfg<NO>;
+    constexpr uint32_t id3 = idesc_bf16(128, 3 * NO), id2 = idesc_bf16(128, 2 * NO), id1 = idesc_bf16(128, NO);
     constexpr uint64_t kPart16 = kSpPart >> 4;
 #pragma unroll
     for (int t = 0; t < NT; ++t, ++g) {
-        const uint32_t s = g % kSpStages, acc = chain & 1;
+        const uint32_t s = g % C::STAGES, acc = chain & 1;
         const bool head = t % kSpChain == 0, tail = t % kSpChain == kSpChain - 1 || t == NT - 1;
         if (head && !mbar_wait(&ctl.acc_empty[acc], ((chain >> 1) & 1) ^ 1, kSpWait)) return false;
-        if (!mbar_wait(&ctl.w_full[s], (g / kSpStages) & 1, kSpWait)) return false;
+        if (!mbar_wait(&ctl.w_full[s], (g / C::STAGES) & 1, kSpWait)) return false;
         tc_fence_after();
-        const uint32_t d = tmem + acc * 256;
-        const uint64_t w = w_desc + (uint64_t)(s * (uint32_t)(kSpStage >> 4));
+        const uint32_t d = tmem + acc * C::ACC;
+        const uint64_t w = w_desc + (uint64_t)(s * (uint32_t)(C::STAGE >> 4));
         const uint64_t xt = x + (uint64_t)((FIRST ? kSpPre5 + (t - 2) * kL5Pitch
                                                   : kSpPre3 + (t / 3 - 1) * kL3Pitch + (t % 3 - 1)) * 8);
         if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) mma_bf16(d, xt + 2 * kk, w + 2 * kk, id192, head && kk == 0 ? 0u : 1u);
+            for (int kk = 0; kk < 4; ++kk) mma_bf16(d, xt + 2 * kk, w + 2 * kk, id3, head && kk == 0 ? 0u : 1u);
             if (!FIRST) {
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk) mma_bf16(d + 64, xt + kPart16 + 2 * kk, w + 2 * kk, id128, 1u);
+                for (int kk = 0; kk < 4; ++kk) mma_bf16(d + NO, xt + kPart16 + 2 * kk, w + 2 * kk, id2, 1u);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk) mma_bf16(d + 128, xt + 2 * kPart16 + 2 * kk, w + 2 * kk, id64, 1u);
+                for (int kk = 0; kk < 4; ++kk) mma_bf16(d + 2 * NO, xt + 2 * kPart16 + 2 * kk, w + 2 * kk, id1, 1u);
             }
             mma_commit(&ctl.w_empty[s]);
             if (tail) mma_commit(&ctl.acc_full[group][acc]);
@@ -248,13 +263,15 @@ __device__ __forceinline__ bool issue_half(SpCtl &ctl, uint32_t tmem, uint64_t x
 
 }  // namespace
 
+template <int NO>
 __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid_constant__ SpParams p) {
+    using C = SpCfg<NO>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *win = smem;
     uint8_t *wst = smem + kSpSlots * kSpSlot;
-    uint8_t *stg = smem + kSpStgOff;
-    SpCtl &ctl = *reinterpret_cast<SpCtl *>(smem + kSpCtlOff);
+    uint8_t *stg = smem + C::STG_OFF;
+    SpCtl &ctl = *reinterpret_cast<SpCtl *>(smem + C::CTL_OFF);
     int &abort_flag = ctl.abort_flag;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid / 32, 0), lane = tid % 32;
     const int n3 = (p.rows + kSpTile - 1) / kSpTile, n5 = (p.rows5 + kSpTile - 1) / kSpTile;
@@ -265,7 +282,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
             mbar_init(&ctl.win_full[i], 1);
             mbar_init(&ctl.win_empty[i], 1);
         }
-        for (int i = 0; i < kSpStages; ++i) {
+        for (int i = 0; i < C::STAGES; ++i) {
             mbar_init(&ctl.w_full[i], 1);
             mbar_init(&ctl.w_empty[i], 1);
         }
@@ -316,14 +333,15 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
 
     if (warp == 2) {
         // ------------------------------------------------ item claims + windows
-        if (lane == 0) {
-            uint32_t wn = 0;
-            for (int q = 0;; ++q) {
+        // lane 0 claims and loads, the whole warp polls the dependencies
+        uint32_t wn = 0;
+        for (int q = 0;; ++q) {
+            int it = -1;
+            if (lane == 0) {
                 const int slot = q % kSpRing;
                 bool ok = mbar_wait(&ctl.item_empty[slot], ((uint32_t)(q / kSpRing) & 1) ^ 1, kSpWait);
                 // claimed once its first window slot is free, so that it is worked on at once
                 ok = ok && mbar_wait(&ctl.win_empty[wn % kSpSlots], ((wn / kSpSlots) & 1) ^ 1, kSpWait);
-                int it = -1;
                 if (ok && !abort_flag) {
                     it = atomicAdd(item_ctr, 1);
                     if (it >= p.nitems) it = -1;
@@ -332,36 +350,41 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                 }
                 ctl.item_id[slot] = it;
                 mbar_arrive(&ctl.item_full[slot]);
-                if (it < 0) break;
-                int l, j, g;
-                decode(it, l, j, g);
-                const SpLayerDev &L = p.L[l];
-                if (l > 0) {
-                    bool done = true;
-                    if (p.L[l - 1].first) {
-                        // L5 tiles whose rows land on L3 rows [lo3, hi3): an L5 row is
-                        // the L3 row minus (board + y), board + y <= rows / 400 + 19
-                        const int lo3 = max(0, j * kSpTile - kSpPre3);
-                        const int hi3 = min(p.rows, j * kSpTile + kSpTile + kSpPre3);
-                        const int lo5 = max(0, lo3 - (hi3 - 1) / kL3Board - kBoard), hi5 = min(p.rows5 - 1, hi3 - 1);
-                        for (int jj = lo5 / kSpTile; jj <= hi5 / kSpTile && done; ++jj)
-                            done = sp_poll(flags5 + jj, L.need);
-                    } else {
-                        for (int jj = max(0, j - 1); jj <= min(n3 - 1, j + 1) && done; ++jj)
-                            done = sp_poll(flags3 + jj, L.need);
-                    }
-                    if (!done) {
-                        fail(102);
-                        break;
-                    }
-                    fence_proxy_async_global();
+            }
+            it = __shfl_sync(0xffffffffu, it, 0);
+            if (it < 0) break;
+            int l, j, g;
+            decode(it, l, j, g);
+            const SpLayerDev &L = p.L[l];
+            if (l > 0) {
+                const int *f;
+                int n;
+                if (p.L[l - 1].first) {
+                    // L5 tiles whose rows land on L3 rows [lo3, hi3): an L5 row is
+                    // the L3 row minus (board + y), board + y <= rows / 400 + 19
+                    const int lo3 = max(0, j * kSpTile - kSpPre3);
+                    const int hi3 = min(p.rows, j * kSpTile + kSpTile + kSpPre3);
+                    const int lo5 = max(0, lo3 - (hi3 - 1) / kL3Board - kBoard) / kSpTile;
+                    f = flags5 + lo5;
+                    n = min(p.rows5 - 1, hi3 - 1) / kSpTile - lo5 + 1;
+                } else {
+                    const int lo = max(0, j - 1);
+                    f = flags3 + lo;
+                    n = min(n3 - 1, j + 1) - lo + 1;
                 }
-                bool bad = false;
-                for (int h = 0; h < L.halves; ++h, ++wn) {
-                    const int ws = wn % kSpSlots;
-                    if (h > 0 && !mbar_wait(&ctl.win_empty[ws], ((wn / kSpSlots) & 1) ^ 1, kSpWait)) {
+                if (!sp_poll(f, n, L.need)) {
+                    if (lane == 0) fail(102);
+                    break;
+                }
+                fence_proxy_async_global();
+                __syncwarp();
+            }
+            if (lane == 0) {
+                for (int h = 0; h < L.halves; ++h) {
+                    const uint32_t w = wn + h;
+                    const int ws = w % kSpSlots;
+                    if (h > 0 && !mbar_wait(&ctl.win_empty[ws], ((w / kSpSlots) & 1) ^ 1, kSpWait)) {
                         fail(103);
-                        bad = true;
                         break;
                     }
                     uint8_t *dst = win + ws * kSpSlot;
@@ -375,8 +398,8 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                                         j * kSpTile - kSpPre3, pt);
                     }
                 }
-                if (bad) break;
             }
+            wn += L.halves;
         }
     } else if (warp == 0) {
         // ------------------------------------------------ weight stages
@@ -393,15 +416,20 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                 bool bad = false;
                 for (int h = 0; h < L.halves && !bad; ++h)
                     for (int t = 0; t < ntaps; ++t, ++g) {
-                        const int s = g % kSpStages;
-                        if (!mbar_wait(&ctl.w_empty[s], ((g / kSpStages) & 1) ^ 1, kSpWait)) {
+                        const int s = g % C::STAGES;
+                        if (!mbar_wait(&ctl.w_empty[s], ((g / C::STAGES) & 1) ^ 1, kSpWait)) {
                             fail(105);
                             bad = true;
                             break;
                         }
-                        mbar_arrive_expect_tx(&ctl.w_full[s], kSpStage);
-                        tma_load_2d(wst + s * kSpStage, &p.w, &ctl.w_full[s], 0,
-                                    L.wrow + ((t * L.halves + h) * L.groups + og) * (3 * kSpNO));
+                        mbar_arrive_expect_tx(&ctl.w_full[s], C::STAGE);
+                        const int row = L.wrow + ((t * L.halves + h) * L.wgroups + og * NO / 64) * 192 + og * NO % 64;
+                        if (NO == 64) {
+                            tma_load_2d(wst + s * C::STAGE, &p.w, &ctl.w_full[s], 0, row);
+                        } else {
+                            for (int pt = 0; pt < 3; ++pt)
+                                tma_load_2d(wst + s * C::STAGE + pt * NO * 128, &p.w, &ctl.w_full[s], 0, row + 64 * pt);
+                        }
                     }
                 if (bad) break;
             }
@@ -428,8 +456,8 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                 const int ws = wn % kSpSlots;
                 if (!mbar_wait(&ctl.win_full[ws], (wn / kSpSlots) & 1, kSpWait)) { fail(107); ok = false; break; }
                 const uint64_t x = x_desc + (uint64_t)(ws * (kSpSlot >> 4));
-                ok = first ? issue_half<true>(ctl, tmem, x, w_desc, q % kSpGroups, g, chain)
-                           : issue_half<false>(ctl, tmem, x, w_desc, q % kSpGroups, g, chain);
+                ok = first ? issue_half<NO, true>(ctl, tmem, x, w_desc, q % kSpGroups, g, chain)
+                           : issue_half<NO, false>(ctl, tmem, x, w_desc, q % kSpGroups, g, chain);
                 if (!ok) { fail(108); break; }
                 if (elect_one()) mma_commit(&ctl.win_empty[ws]);
             }
@@ -443,7 +471,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
         }
     } else if (warp >= 4) {
         // ------------------------------------------------ epilogue
-        const int quarter = warp & 3, ch = (((warp - 4) >> 2) & 1) * 32, group = (warp - 4) / kSpEpiWarps;
+        const int quarter = warp & 3, ch = (((warp - 4) >> 2) & 1) * C::CH, group = (warp - 4) / kSpEpiWarps;
         const int row = quarter * 32 + lane;
         const uint32_t t_row = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)ch;
         const size_t ps = (size_t)p.cap_rows * p.pitch;
@@ -461,9 +489,9 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                 g += chains;
                 continue;
             }
-            float v[32];
+            float v[C::CH];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0.0f;
+            for (int i = 0; i < C::CH; ++i) v[i] = 0.0f;
             bool bad = false;
             for (int c = 0; c < chains; ++c, ++g) {
                 const int acc = g & 1;
@@ -471,13 +499,13 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                 if (!mbar_wait(&ctl.acc_full[group][acc], use & 1, kSpWait)) { fail(111); bad = true; break; }
                 tc_fence_after();
 #pragma unroll
-                for (int c0 = 0; c0 < 32; c0 += 8) {
+                for (int c0 = 0; c0 < C::CH; c0 += 8) {
                     uint32_t a2[8], a1[8], a0[8];
-                    tmem_ld8(t_row + acc * 256 + 128 + c0, a2);
-                    tmem_ld8(t_row + acc * 256 + 64 + c0, a1);
-                    tmem_ld8(t_row + acc * 256 + c0, a0);
+                    tmem_ld8(t_row + acc * C::ACC + 2 * NO + c0, a2);
+                    tmem_ld8(t_row + acc * C::ACC + NO + c0, a1);
+                    tmem_ld8(t_row + acc * C::ACC + c0, a0);
                     tmem_ld_wait();
-                    if (c0 == 24) {
+                    if (c0 == C::CH - 8) {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&ctl.acc_empty[acc]);
@@ -489,9 +517,9 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
             }
             if (bad) break;
             const int q0 = j * kSpTile + row;
-            const int o0 = og * kSpNO + ch;
+            const int o0 = og * NO + ch;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < C::CH / 4; ++i) {
                 const float4 bv = __ldg(reinterpret_cast<const float4 *>(L.bias + o0) + i);
                 v[4 * i] += bv.x;
                 v[4 * i + 1] += bv.y;
@@ -500,10 +528,10 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
             }
             if (L.act == LG_ACT_RELU) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = act_fn(v[i], LG_ACT_RELU);
+                for (int i = 0; i < C::CH; ++i) v[i] = act_fn(v[i], LG_ACT_RELU);
             } else {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
+                for (int i = 0; i < C::CH; ++i) {
                     const float e = expf(v[i]) - 1.0f;  // as act_fn, without a branch a value
                     v[i] = v[i] > 0.0f ? v[i] : e;
                 }
@@ -520,29 +548,30 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                     float *dst = L.out32 + ((size_t)b * kPoints + y * kBoard + x) * L.cout + o0;
                     if ((L.cout & 3) == 0) {
 #pragma unroll
-                        for (int i = 0; i < 8; ++i)
+                        for (int i = 0; i < C::CH / 4; ++i)
                             if (o0 + 4 * i < L.cout)
                                 reinterpret_cast<float4 *>(dst)[i] =
                                     make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
                     } else {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
+                        for (int i = 0; i < C::CH; ++i)
                             if (o0 + i < L.cout) dst[i] = v[i];
                     }
                 }
             } else {
                 const int tgt = in_range && y < 20 ? b * kL3Board + y * kL3Pitch + x : -1;
                 uint4 *tile = reinterpret_cast<uint4 *>(stg + (warp - 4) * kSpTileBytes);
-                store_parts(v, tgt, point, tile, lane, L.out + o0, ps, p.pitch);
-                store_parts(v + 16, tgt, point, tile, lane, L.out + o0 + 16, ps, p.pitch);
-                if (L.first && tgt >= 0 && x == kBoard - 1)
-                    store_zero_parts(L.out + (size_t)(tgt + 1) * p.pitch + o0, ps);
+#pragma unroll
+                for (int c0 = 0; c0 < C::CH; c0 += 16) {
+                    store_parts(v + c0, tgt, point, tile, lane, L.out + o0 + c0, ps, p.pitch);
+                    if (L.first && tgt >= 0 && x == kBoard - 1)
+                        store_zero_parts(L.out + (size_t)(tgt + 1) * p.pitch + o0 + c0, ps);
+                }
             }
             // publish: the generic stores, ordered before other SMs' TMA reads
             fence_proxy_async_global();
             __syncwarp();
             if (lane == 0) {
-                __threadfence();
                 asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"((L.first ? flags5 : flags3) + j) : "memory");
             }
         }
@@ -554,7 +583,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
             mbar_wait(&ctl.win_full[i], 0, 1u << 16);
             mbar_wait(&ctl.win_full[i], 1, 1u << 16);
         }
-        for (int i = 0; i < kSpStages; ++i) {
+        for (int i = 0; i < C::STAGES; ++i) {
             mbar_wait(&ctl.w_full[i], 0, 1u << 16);
             mbar_wait(&ctl.w_full[i], 1, 1u << 16);
         }
@@ -620,7 +649,10 @@ void launch_split_weights(const float *wt, int k, int cin, int cout, __nv_bfloat
 }
 
 int split_init_device() {
-    cudaError_t e = cudaFuncSetAttribute(split_trunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpSmem);
+    cudaError_t e = cudaFuncSetAttribute(split_trunk_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SpCfg<64>::SMEM);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(split_trunk_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, SpCfg<32>::SMEM);
     if (e != cudaSuccess) {
         lg_set_error("cudaFuncSetAttribute(split trunk): %s", cudaGetErrorString(e));
         return LG_ERR_CUDA;
@@ -642,13 +674,22 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
     p.flags = T.flags;
     p.err = T.err;
     const int n3 = (p.rows + kSpTile - 1) / kSpTile, n5 = (p.rows5 + kSpTile - 1) / kSpTile;
+    int wide = 0;
+    for (int l = 0; l < T.nl; ++l) wide = std::max(wide, T.L[l].groups);
+    // 32-channel items while 64-channel ones would leave a third of the SMs
+    // without any: their MMAs (N = 96, 64, 32) run at two thirds of the rate,
+    // but twice as many SMs work on a layer.  Policy + value pair of the
+    // benchmark nets, us, 32 / 64 channels: 5 positions 322 / 422, 16 positions
+    // (100 wide items) 357 / 431, 24 positions (150) 475 / 441.
+    const int no = 3 * n3 * wide <= 2 * sm_count ? 32 : 64;
     int wrows = 0, items = 0;
     for (int l = 0; l < T.nl; ++l) {
         const SplitLayer &S = T.L[l];
         SpLayerDev &L = p.L[l];
         L.first = l == 0;
         L.halves = S.halves;
-        L.groups = S.groups;
+        L.groups = S.groups * 64 / no;
+        L.wgroups = S.groups;
         L.wrow = wrows;
         L.item0 = items;
         // a tile's counter once the layer before is complete there (the first
@@ -660,19 +701,19 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
         L.out = last ? nullptr : T.buf[(l + 1) & 1];
         L.out32 = last ? T.out32 : nullptr;
         L.cout = S.cout;
-        wrows += (l == 0 ? 5 : 9) * S.halves * S.groups * 3 * kSpNO;
-        items += (l == 0 ? n5 : n3) * S.groups;
+        wrows += (l == 0 ? 5 : 9) * S.halves * S.groups * 192;
+        items += (l == 0 ? n5 : n3) * L.groups;
     }
     p.nitems = items;
     int rc = encode_map_3d_bf16(&p.in[0], T.buf[0], T.pitch, p.rows, 3, T.cap_rows, 64, kSpWin3);
     if (!rc) rc = encode_map_3d_bf16(&p.in[1], T.buf[1], T.pitch, p.rows, 3, T.cap_rows, 64, kSpWin3);
     if (!rc) rc = encode_map_2d_bf16(&p.in5, T.l5, (uint64_t)T.L[0].halves * 64, (uint64_t)p.rows5, 64, kSpWin5);
-    if (!rc) rc = encode_map_2d_bf16(&p.w, T.w, 64, (uint64_t)wrows, 64, 3 * kSpNO);
+    if (!rc) rc = encode_map_2d_bf16(&p.w, T.w, 64, (uint64_t)wrows, 64, no == 64 ? 192 : 32);
     if (rc) return rc;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(std::min(items, sm_count));
     cfg.blockDim = dim3(kSpThreads);
-    cfg.dynamicSmemBytes = kSpSmem;
+    cfg.dynamicSmemBytes = no == 64 ? SpCfg<64>::SMEM : SpCfg<32>::SMEM;
     cfg.stream = s;
     // items are claimed in order, so what an item waits for belongs to a
     // running CTA: no co-residency needed
@@ -681,7 +722,7 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, split_trunk_kernel, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, no == 64 ? split_trunk_kernel<64> : split_trunk_kernel<32>, p);
     if (e != cudaSuccess) {
         lg_set_error("split trunk launch: %s", cudaGetErrorString(e));
         return LG_ERR_CUDA;
