@@ -18,6 +18,7 @@
 //     softmax and the value FC chain that follow are finish.cu's.
 #include "lg_kernels.h"
 
+#include <algorithm>
 #include <cfloat>
 
 namespace lg {
@@ -303,6 +304,145 @@ __global__ void __launch_bounds__(256, 2) conv_f32_big_kernel(const float *__res
     }
 }
 
+// Layers of 64k output channels over enough rows: 192 x 64 tiles, 12 x 8
+// outputs a thread (five float4 loads of the operands per 96 FMAs), K steps of
+// one tap and 8 input channels double-buffered.  What bounds tiles with fewer
+// outputs a thread is shared memory: a float4 load is four wavefronts a warp
+// whatever its lanes share (packed fma.rn.f32x2 on 8 x 8 outputs, one operand
+// stored twice, was slower than the 64 x 64 kernel).  Every output is still
+// one FMA chain over (tap, channel) in order, as in the other two kernels: the
+// same bits.
+//
+// Three CTAs an SM, each over an even share of the 64-row blocks in tiles of
+// three, the rest in one of two or one.  A 3x3 layer 64 -> 64 over 512 boards:
+// 440 us on the 64 x 64 kernel, 378 with one 256-row tile a CTA (2.4 waves
+// taking 3), 312 with shares of 16 x 8 outputs and two CTAs an SM, 296 so (46
+// TFLOP/s of a 70 TFLOP/s peak).
+constexpr int BM3 = 192, BN3 = 64, BKC3 = 8, kN64Threads = 128, kN64Ctas = 3;
+
+struct N64Smem {
+    float A[2][BKC3][BM3 + 4];
+    float B[2][BKC3][BN3 + 4];
+};
+
+__device__ __forceinline__ float4 ldg_nc4(const float *p) {
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+// One tile of 64 R rows from row m0.
+template <int KS, int R>
+__device__ __forceinline__ void n64_tile(const float *__restrict__ in, const float *__restrict__ wt,
+                                         const float *__restrict__ bias, float *__restrict__ out, int M, int C, int O,
+                                         int act, int m0, int n0, N64Smem &sm) {
+    const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
+    constexpr int PAD = KS / 2;
+    // A loader: rows ar + 64 i, channels ac .. ac+3; a bit per tap inside the board
+    const int ar = tid / 2, ac = (tid % 2) * 4;
+    uint32_t inside[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int m = m0 + ar + 64 * i, p = m % kPoints, y = p / kBoard, x = p - y * kBoard;
+        uint32_t bits = 0;
+        for (int t = 0; t < KS * KS; ++t) {
+            const int sy = y + t / KS - PAD, sx = x + t % KS - PAD;
+            if (m < M && sy >= 0 && sy < kBoard && sx >= 0 && sx < kBoard) bits |= 1u << t;
+        }
+        inside[i] = bits;
+    }
+    const float *src = in + (size_t)(m0 + ar) * C + ac;
+    // B loader: channel bk, columns bn .. bn+3
+    const int bk = tid / 16, bn = (tid % 16) * 4;
+    const float *wsrc = wt + (size_t)bk * O + n0 + bn;
+    const int cchunks = (C + BKC3 - 1) / BKC3, ksteps = KS * KS * cchunks;
+    float4 va[R], vb;
+    int tap = 0, c0 = 0;  // of the step to load
+    auto load = [&]() {
+        const float *s = src + ((tap / KS - PAD) * kBoard + tap % KS - PAD) * C + c0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            va[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if ((inside[i] >> tap & 1) && c0 + ac < C) va[i] = ldg_nc4(s + (size_t)(64 * i) * C);
+        }
+        vb = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c0 + bk < C) vb = ldg_nc4(wsrc + ((size_t)tap * C + c0) * O);
+        c0 += BKC3;
+        if (c0 >= C) {
+            c0 = 0;
+            ++tap;
+        }
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            sm.A[buf][ac + 0][ar + 64 * i] = va[i].x;
+            sm.A[buf][ac + 1][ar + 64 * i] = va[i].y;
+            sm.A[buf][ac + 2][ar + 64 * i] = va[i].z;
+            sm.A[buf][ac + 3][ar + 64 * i] = va[i].w;
+        }
+        *reinterpret_cast<float4 *>(&sm.B[buf][bk][bn]) = vb;
+    };
+    // rows ty*4 + 64 i + r, columns tx*4 + 32 h + j
+    float acc[4 * R][8];
+#pragma unroll
+    for (int i = 0; i < 4 * R; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+    load();
+    store(0);
+    __syncthreads();
+    for (int ks = 0; ks < ksteps; ++ks) {
+        const int cur = ks & 1;
+        const bool more = ks + 1 < ksteps;
+        if (more) load();
+#pragma unroll
+        for (int kk = 0; kk < BKC3; ++kk) {
+            float a[4 * R], b[8];
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                *reinterpret_cast<float4 *>(a + 4 * i) = *reinterpret_cast<const float4 *>(&sm.A[cur][kk][ty * 4 + 64 * i]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float4 *>(b + 4 * h) = *reinterpret_cast<const float4 *>(&sm.B[cur][kk][tx * 4 + 32 * h]);
+#pragma unroll
+            for (int i = 0; i < 4 * R; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        if (more) store(cur ^ 1);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4 * R; ++i) {
+        const int m = m0 + ty * 4 + 64 * (i / 4) + i % 4;
+        if (m >= M) continue;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int n = n0 + 32 * h + tx * 4;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = act_fn(bias[n + j] + acc[i][4 * h + j], act);
+            *reinterpret_cast<float4 *>(out + (size_t)m * O + n) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+    }
+}
+
+template <int KS>
+__global__ void __launch_bounds__(kN64Threads, kN64Ctas) conv_f32_n64_kernel(const float *__restrict__ in,
+                                                                      const float *__restrict__ wt,
+                                                                      const float *__restrict__ bias,
+                                                                      float *__restrict__ out, int M, int C, int O,
+                                                                      int act) {
+    __shared__ __align__(16) N64Smem sm;
+    const int nblk = (M + 63) / 64, n0 = blockIdx.y * BN3;
+    int b = (int)((long long)nblk * blockIdx.x / gridDim.x);
+    const int e = (int)((long long)nblk * (blockIdx.x + 1) / gridDim.x);
+    for (; b + 2 < e; b += 3) n64_tile<KS, 3>(in, wt, bias, out, M, C, O, act, b * 64, n0, sm);
+    if (b + 1 < e) n64_tile<KS, 2>(in, wt, bias, out, M, C, O, act, b * 64, n0, sm);
+    else if (b < e) n64_tile<KS, 1>(in, wt, bias, out, M, C, O, act, b * 64, n0, sm);
+}
+
 // Fixed-order reduction of the split-K partial sums, then bias + activation.
 __global__ void splitk_reduce_f32(const float *__restrict__ partial, int nsplit, size_t MO, int O,
                                   const float *__restrict__ bias, int act,
@@ -355,6 +495,11 @@ struct F32Plan {
     bool big;
     int bm, bn, bkc;
 };
+// The 12 x 8-output kernel where every CTA slot gets at least half a tile (the
+// 64 x 64 kernel would not split K there either) and float4 loads are aligned.
+bool f32_n64(const F32Plan &pl, int M, int C, int O) {
+    return !pl.big && O % BN3 == 0 && C % 4 == 0 && (long long)M * (O / BN3) >= 152 * 256;
+}
 F32Plan f32_plan(int M, int O) {
     return (O % BN2 == 0 && M >= 152 * BM2) ? F32Plan{true, BM2, BN2, BKC2} : F32Plan{false, BM, BN, BKC};
 }
@@ -381,6 +526,15 @@ void launch_conv_f32(const float *in, const float *wt, const float *bias, float 
                      int C, int O, int k, int act, float *partial, cudaStream_t s) {
     int M = B * kPoints;
     const F32Plan pl = f32_plan(M, O);
+    if (f32_n64(pl, M, C, O) && (((uintptr_t)in | (uintptr_t)wt | (uintptr_t)out) & 15) == 0) {
+        const dim3 grid(std::min(kN64Ctas * 152, (M + 63) / 64), O / BN3);
+        switch (k) {
+        case 1: conv_f32_n64_kernel<1><<<grid, kN64Threads, 0, s>>>(in, wt, bias, out, M, C, O, act); break;
+        case 3: conv_f32_n64_kernel<3><<<grid, kN64Threads, 0, s>>>(in, wt, bias, out, M, C, O, act); break;
+        default: conv_f32_n64_kernel<5><<<grid, kN64Threads, 0, s>>>(in, wt, bias, out, M, C, O, act); break;
+        }
+        return;
+    }
     int nsplit = conv_f32_splits(M, O, C, k);
     int ksteps = k * k * ((C + pl.bkc - 1) / pl.bkc);
     int per = (ksteps + nsplit - 1) / nsplit;

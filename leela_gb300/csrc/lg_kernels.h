@@ -22,6 +22,27 @@ __device__ __forceinline__ uint16_t round16(float v, bool f16) {
     return f16 ? __half_as_ushort(__float2half_rn(v)) : __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
 
+// x as three BF16 parts, h = rn(x), m = rn(x - h), l = x - h - m (exact).
+// Values that would round to infinity are truncated; infinities and NaN are
+// all in h.
+__device__ __forceinline__ void split3(float x, float &h, float &m, float &l) {
+    h = __bfloat162float(__float2bfloat16_rn(x));
+    float r = x - h;
+    if (!(fabsf(x) < 3.3895e38f)) {
+        const bool fin = fabsf(x) <= 3.402823466e38f;
+        if (fin) h = __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
+        r = fin ? x - h : 0.0f;
+    }
+    m = __bfloat162float(__float2bfloat16_rn(r));
+    l = r - m;
+}
+
+__device__ __forceinline__ uint32_t pack2_bf16(float lo, float hi) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
+
 // ------------------------------------------------------------ FP32 path
 int conv_f32_splits(int M, int O, int C, int k);
 size_t conv_f32_partial_floats(int B, int C, int O, int k);
@@ -44,7 +65,7 @@ struct SplitLayer {
 struct SplitTrunk {
     SplitLayer L[kSpMaxLayers];
     int nl, B, act;
-    const void *l5;          // [B * 399][L[0].halves * 64] BF16
+    const void *l5;          // [B * 399][L[0].halves * 64] BF16; null: no 5x5 layer, layer 0 is a 3x3 one reading buf[0]
     __nv_bfloat16 *buf[2];   // [3][cap_rows][pitch] parts, L3 rows
     int cap_rows, pitch;
     const void *w;           // per layer [tap][half][group][part][64][64] BF16
@@ -56,11 +77,28 @@ size_t split_flag_ints(int B);
 int split_pad(int channels);  // channels rounded up to whole groups
 // A layer's weights in that layout, made on the device from the FP32 path's
 // wt [k*k][cin][cout] (k = 5 for the first layer, else 3): elements, launch.
+// flip: from the wt [9][cout][cin] of a 3x3 conv, the weights of its input
+// gradient.
 size_t split_weight_elems(int k, int cin, int cout);
-void launch_split_weights(const float *wt, int k, int cin, int cout, __nv_bfloat16 *out, cudaStream_t s);
+void launch_split_weights(const float *wt, int k, int cin, int cout, __nv_bfloat16 *out, cudaStream_t s,
+                          bool flip = false);
 int split_init_device();
 // A programmatic dependent of the previous kernel in the stream.
 int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count);
+
+// Weight gradients of 64-wide conv layers from such parts (wgrad_tc.cu): dW
+// [taps][channels][64] += X^T dY over all rows.  x, d: [3][cap_rows][64] parts
+// in L3 rows; the 5x5 first layer: l5 the expanded planes [B*399][128] (5 c_in
+// <= 128 real channels), d in L5 rows.
+int wgrad_init_device();
+// FP32 [B*361][64] -> parts (L3 rows, or L5 rows with l5); with Y, masked by
+// Y > 0 and summed over rows into db[64].
+void launch_to_parts(const float *src, const float *Y, int B, bool l5, size_t cap_rows, __nv_bfloat16 *parts, float *db,
+                     cudaStream_t s);
+int launch_wgrad_3x3(const __nv_bfloat16 *x, const __nv_bfloat16 *d, int B, size_t cap_rows, float *dW, int *err,
+                     cudaStream_t s);
+int launch_wgrad_first(const __nv_bfloat16 *l5, const __nv_bfloat16 *d, int B, int c_in, size_t cap_rows, float *dW,
+                       int *err, cudaStream_t s);
 
 // Input of the finish kernels: the head output of point (b, p) is
 //   act_head?(sum_k parts[k * part_stride + b * 361 + p] + head_b).

@@ -144,27 +144,6 @@ __device__ __forceinline__ bool sp_poll(const int *f, int n, int want) {
     return __all_sync(0xffffffffu, ok);
 }
 
-// x as three BF16 parts, h = rn(x), m = rn(x - h), l = x - h - m (exact).
-// Values that would round to infinity are truncated; infinities and NaN are
-// all in h.
-__device__ __forceinline__ void split3(float x, float &h, float &m, float &l) {
-    h = __bfloat162float(__float2bfloat16_rn(x));
-    float r = x - h;
-    if (!(fabsf(x) < 3.3895e38f)) {
-        const bool fin = fabsf(x) <= 3.402823466e38f;
-        if (fin) h = __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
-        r = fin ? x - h : 0.0f;
-    }
-    m = __bfloat162float(__float2bfloat16_rn(r));
-    l = r - m;
-}
-
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-    uint32_t d;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
-    return d;
-}
-
 // 16 channels of 32 rows (lane = row) as parts into L3 rows `tgt` (-1: not
 // stored), through a 1 KB staging tile so that two lanes store the 32 bytes
 // of a row (a 16-byte store per lane and row would write half sectors of 32
@@ -180,12 +159,12 @@ __device__ __forceinline__ void store_parts(const float *v, int tgt, bool point,
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const float x0 = point ? v[2 * k] : 0.0f, x1 = point ? v[2 * k + 1] : 0.0f;
-            const uint32_t h = pack_bf16x2(x0, x1);
+            const uint32_t h = pack2_bf16(x0, x1);
             const float r0 = x0 - __uint_as_float(h << 16), r1 = x1 - __uint_as_float(h & 0xFFFF0000u);
-            const uint32_t m = pack_bf16x2(r0, r1);
+            const uint32_t m = pack2_bf16(r0, r1);
             w[0][k] = h;
             w[1][k] = m;
-            w[2][k] = pack_bf16x2(r0 - __uint_as_float(m << 16), r1 - __uint_as_float(m & 0xFFFF0000u));
+            w[2][k] = pack2_bf16(r0 - __uint_as_float(m << 16), r1 - __uint_as_float(m & 0xFFFF0000u));
         }
     } else {
 #pragma unroll
@@ -193,9 +172,9 @@ __device__ __forceinline__ void store_parts(const float *v, int tgt, bool point,
             float h0, m0, l0, h1, m1, l1;
             split3(point ? v[2 * k] : 0.0f, h0, m0, l0);
             split3(point ? v[2 * k + 1] : 0.0f, h1, m1, l1);
-            w[0][k] = pack_bf16x2(h0, h1);
-            w[1][k] = pack_bf16x2(m0, m1);
-            w[2][k] = pack_bf16x2(l0, l1);
+            w[0][k] = pack2_bf16(h0, h1);
+            w[1][k] = pack2_bf16(m0, m1);
+            w[2][k] = pack2_bf16(l0, l1);
         }
     }
     const int sub = lane >> 1, c = lane & 1, sw = (lane >> 2) & 1;
@@ -529,7 +508,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
             if (L.act == LG_ACT_RELU) {
 #pragma unroll
                 for (int i = 0; i < C::CH; ++i) v[i] = act_fn(v[i], LG_ACT_RELU);
-            } else {
+            } else if (L.act == LG_ACT_ELU) {
 #pragma unroll
                 for (int i = 0; i < C::CH; ++i) {
                     const float e = expf(v[i]) - 1.0f;  // as act_fn, without a branch a value
@@ -609,14 +588,19 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
 // past the real channels.  Parts by truncation; a part that comes out zero is
 // the smallest normal number with the weight's sign (unless the weight is
 // below 1e-25), so that no part turns an infinite activation into a NaN.
+// flip (k = 3): wt is [9][cout][cin], the weights of the conv whose input
+// gradient this is -- taps in reverse, channels transposed.
 __global__ void __launch_bounds__(256) split_weights_kernel(const float *__restrict__ wt, int k, int cin, int cout,
-                                                            int kpad, int opad, __nv_bfloat16 *__restrict__ out, int n) {
+                                                            int kpad, int opad, bool flip, __nv_bfloat16 *__restrict__ out,
+                                                            int n) {
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
     const int kk = i % kpad, o = i / kpad % opad, t = i / kpad / opad;
     const int dx = k == 5 ? kk / cin : 0, ci = k == 5 ? kk - dx * cin : kk;
     float w = 0.0f;
-    if (o < cout && kk < (k == 5 ? 5 * cin : cin)) w = wt[((size_t)(k == 5 ? t * 5 + dx : t) * cin + ci) * cout + o];
+    if (o < cout && kk < (k == 5 ? 5 * cin : cin))
+        w = flip ? wt[((size_t)(k * k - 1 - t) * cout + o) * cin + ci]
+                 : wt[((size_t)(k == 5 ? t * 5 + dx : t) * cin + ci) * cout + o];
     const float tiny = fabsf(w) > 1e-25f ? copysignf(1.17549435e-38f, w) : 0.0f;
     uint16_t *dst = reinterpret_cast<uint16_t *>(out) +
                     (((size_t)t * (kpad / 64) + kk / 64) * (opad / 64) + o / 64) * 3 * 4096 + (size_t)(o % 64) * 64 + kk % 64;
@@ -642,10 +626,10 @@ size_t split_weight_elems(int k, int cin, int cout) {
     return (size_t)taps * split_pad(kper) * split_pad(cout) * 3;
 }
 
-void launch_split_weights(const float *wt, int k, int cin, int cout, __nv_bfloat16 *out, cudaStream_t s) {
+void launch_split_weights(const float *wt, int k, int cin, int cout, __nv_bfloat16 *out, cudaStream_t s, bool flip) {
     const int n = (int)(split_weight_elems(k, cin, cout) / 3);
     split_weights_kernel<<<(n + 255) / 256, 256, 0, s>>>(wt, k, cin, cout, split_pad(k == 5 ? 5 * cin : cin),
-                                                         split_pad(cout), out, n);
+                                                         split_pad(cout), flip, out, n);
 }
 
 int split_init_device() {
@@ -668,7 +652,7 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
     SpParams p{};
     p.nl = T.nl;
     p.rows = T.B * kL3Board;
-    p.rows5 = T.B * kL5Board;
+    p.rows5 = T.l5 ? T.B * kL5Board : 0;
     p.cap_rows = T.cap_rows;
     p.pitch = T.pitch;
     p.flags = T.flags;
@@ -682,11 +666,11 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
     // benchmark nets, us, 32 / 64 channels: 5 positions 322 / 422, 16 positions
     // (100 wide items) 357 / 431, 24 positions (150) 475 / 441.
     const int no = 3 * n3 * wide <= 2 * sm_count ? 32 : 64;
-    int wrows = 0, items = 0;
+    int wrows = 0, items = 0, done3 = 0;
     for (int l = 0; l < T.nl; ++l) {
         const SplitLayer &S = T.L[l];
         SpLayerDev &L = p.L[l];
-        L.first = l == 0;
+        L.first = l == 0 && T.l5;
         L.halves = S.halves;
         L.groups = S.groups * 64 / no;
         L.wgroups = S.groups;
@@ -694,20 +678,24 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
         L.item0 = items;
         // a tile's counter once the layer before is complete there (the first
         // layer counts in its own tiles)
-        L.need = l == 0 ? 0 : (l < 3 ? 0 : p.L[l - 1].need) + kSpEpiWarps * p.L[l - 1].groups;
+        if (l > 0) {
+            const int n = kSpEpiWarps * p.L[l - 1].groups;
+            L.need = p.L[l - 1].first ? n : done3 += n;
+        }
         L.act = T.act;
         L.bias = S.bias;
         const bool last = l + 1 == T.nl;
         L.out = last ? nullptr : T.buf[(l + 1) & 1];
         L.out32 = last ? T.out32 : nullptr;
         L.cout = S.cout;
-        wrows += (l == 0 ? 5 : 9) * S.halves * S.groups * 192;
-        items += (l == 0 ? n5 : n3) * L.groups;
+        wrows += (L.first ? 5 : 9) * S.halves * S.groups * 192;
+        items += (L.first ? n5 : n3) * L.groups;
     }
     p.nitems = items;
     int rc = encode_map_3d_bf16(&p.in[0], T.buf[0], T.pitch, p.rows, 3, T.cap_rows, 64, kSpWin3);
     if (!rc) rc = encode_map_3d_bf16(&p.in[1], T.buf[1], T.pitch, p.rows, 3, T.cap_rows, 64, kSpWin3);
-    if (!rc) rc = encode_map_2d_bf16(&p.in5, T.l5, (uint64_t)T.L[0].halves * 64, (uint64_t)p.rows5, 64, kSpWin5);
+    p.in5 = p.in[0];
+    if (!rc && T.l5) rc = encode_map_2d_bf16(&p.in5, T.l5, (uint64_t)T.L[0].halves * 64, (uint64_t)p.rows5, 64, kSpWin5);
     if (!rc) rc = encode_map_2d_bf16(&p.w, T.w, 64, (uint64_t)wrows, 64, no == 64 ? 192 : 32);
     if (rc) return rc;
     cudaLaunchConfig_t cfg{};
