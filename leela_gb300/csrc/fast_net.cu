@@ -35,13 +35,21 @@
 //     MMA of that slot's layer has completed, and the slot's next layer
 //     starts once all epilogue warps have written and fenced their rows;
 //   * the last layer's epilogue applies both 1x1 heads to its row and
-//     writes two partial sums per head (one per 32-channel half) to global
+//     writes four partial sums per head (one per 16 channels) to global
 //     memory; the softmax and the value FC run as the library's finish
 //     kernels, which add the parts in a fixed order.
 //
+// A batch with an SM for every board runs one board a CTA (152 boards: 55 us
+// against 89 in pairs).  8,192 boards: 1.63 ms with four epilogue warps per
+// TMEM lane quarter and a warp-uniform MMA issuer, 1.85 with two and a
+// one-lane issuer: a pair of boards takes 111k cycles, 84k of them the MMAs'
+// own (N = 64: 48 cycles each, shared-memory reads), 6k the epilogue's stores
+// in the same shared memory, 11k waits for weight slices (a deeper ring does
+// not shorten them).
+//
 // Warps: 0 = TMA producer of the weight slices, 1 = TMEM owner and MMA
-// issuer (one thread), 2..9 = plane staging, epilogue (two warps per TMEM
-// lane quarter, 32 channels each).  Every wait is bounded; a wait that runs
+// issuer, 2..17 = plane staging, epilogue (four warps per TMEM lane quarter,
+// 16 channels each).  Every wait is bounded; a wait that runs
 // out records an error word, and the CTA drains what it issued and frees
 // its tensor memory.
 #include "lg_kernels.h"
@@ -70,9 +78,10 @@ constexpr int kFStages = 4;
 constexpr int kFSlice = kFW * 128;                   // 64 outputs x 64 K, BF16
 constexpr int kFMaxCin = 24;
 constexpr int kFMaxLayers = 17;                      // first layer + up to 16 3x3
-constexpr int kFEpiWarps = 8;
+constexpr int kFEpiWarps = 16;
 constexpr int kFEpiThreads = kFEpiWarps * 32;
-constexpr int kFThreads = 64 + kFEpiThreads;         // 320
+constexpr int kFThreads = 64 + kFEpiThreads;         // 576
+constexpr int kFParts = 4;                           // head partial sums: one per 16 channels
 constexpr uint32_t kFWaitLimit = 1u << 26;
 
 constexpr int OFF_BUF = 0;                                             // kFSlots x 592 rows
@@ -80,7 +89,7 @@ constexpr int OFF_WST = OFF_BUF + kFSlots * kFBufBytes;                // 151,55
 constexpr int OFF_PL = OFF_WST + kFStages * kFSlice;                   // planes of a group
 constexpr int OFF_MASK = OFF_PL + ((kFSlots * kFMaxCin * kPoints + 127) / 128) * 128;
 constexpr int OFF_LUT = OFF_MASK + ((kFSlots * kPoints * 4 + 127) / 128) * 128;
-constexpr int OFF_BIAS = OFF_LUT + 256 * 16;
+constexpr int OFF_BIAS = OFF_LUT + 256 * 16;  // 16-byte aligned
 constexpr int OFF_HEAD = OFF_BIAS + kFMaxLayers * kFW * 4;
 constexpr int SMEM_USED = OFF_HEAD + 2 * kFW * 4;
 constexpr int kFSmem = 1024 + SMEM_USED;
@@ -91,9 +100,10 @@ static_assert(kFSlots * kFTiles * kFW <= 512, "accumulators fit the tensor memor
 struct FastParams {
     const uint8_t *planes;   // [B][c_in][361]
     int B, c_in, n3;         // positions, input planes, 3x3 layers
+    int slots;               // boards in flight per CTA (1 or kFSlots)
     const float *bias;       // [n3 + 1][64]
     const float *wp, *wv;    // [64] policy / value head weights
-    float *parts_p, *parts_v;  // [2][part_stride]: head sums over channels 0..31 / 32..63
+    float *parts_p, *parts_v;  // [kFParts][part_stride]: head sums over 16 channels each
     size_t part_stride;
     int *err;
     uint32_t wait_limit;
@@ -152,8 +162,9 @@ __global__ void __launch_bounds__(kFThreads, 1)
     __shared__ uint32_t tmem_base;
     __shared__ int abort_flag;
 
-    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const int ngroups = (p.B + kFSlots - 1) / kFSlots;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid / 32, 0), lane = tid % 32;
+    const int NS = p.slots;
+    const int ngroups = (p.B + NS - 1) / NS;
     const int nl = p.n3 + 1;
     const int nslices = 10 + 9 * p.n3;
     const int G = gridDim.x;
@@ -193,6 +204,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
+    grid_dep_launch();  // the finish kernels may be scheduled as CTAs leave (they wait for this grid)
 
     auto fail = [&](int code) {
         atomicCAS(p.err, 0, code);
@@ -207,14 +219,14 @@ __global__ void __launch_bounds__(kFThreads, 1)
         if (lane == 0) {
             uint32_t g = 0;
             for (int grp = blockIdx.x; grp < ngroups; grp += G) {
-                for (int j = 0; j < kFSlots * nslices; ++j, ++g) {
+                for (int j = 0; j < NS * nslices; ++j, ++g) {
                     if (aborted()) goto done_producer;
                     int s;
-                    if (j < 10 * kFSlots) {
-                        const int h = j / (5 * kFSlots), dy = j % 5;
+                    if (j < 10 * NS) {
+                        const int h = j / (5 * NS), dy = j % 5;
                         s = h * 5 + dy;
                     } else {
-                        const int r = j - 10 * kFSlots, l = r / (9 * kFSlots), tap = r % 9;
+                        const int r = j - 10 * NS, l = r / (9 * NS), tap = r % 9;
                         s = 10 + 9 * l + tap;
                     }
                     const int st = g % kFStages;
@@ -227,62 +239,68 @@ __global__ void __launch_bounds__(kFThreads, 1)
         done_producer:;
         }
     } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16(128, kFW);
-            const uint64_t b_base = sdesc_sw128(smem_u32(wst));
-            uint32_t g = 0, n_stage[kFSlots] = {0, 0}, n_act[kFSlots] = {0, 0};
-            for (int grp = blockIdx.x; grp < ngroups; grp += G) {
-                // first layer: two 64-channel halves of the expanded rows
-                for (int h = 0; h < 2; ++h)
-                    for (int sl = 0; sl < kFSlots; ++sl) {
-                        if (!mbar_wait(&stage_full[sl], n_stage[sl] & 1, WL)) { fail(92); goto done_mma; }
-                        ++n_stage[sl];
+        // ------------------------------------------------ MMA issuer: the
+        // whole warp walks the jobs, one elected lane issues
+        const uint32_t idesc = idesc_bf16(128, kFW);
+        const uint64_t b_base = sdesc_sw128(smem_u32(wst));
+        uint32_t g = 0, n_stage[kFSlots] = {0, 0}, n_act[kFSlots] = {0, 0};
+        for (int grp = blockIdx.x; grp < ngroups; grp += G) {
+            // first layer: two 64-channel halves of the expanded rows
+            for (int h = 0; h < 2; ++h)
+                for (int sl = 0; sl < NS; ++sl) {
+                    if (!mbar_wait(&stage_full[sl], n_stage[sl] & 1, WL)) { fail(92); goto done_mma; }
+                    ++n_stage[sl];
+                    const uint64_t a_base = sdesc_sw128(smem_u32(buf + sl * kFBufBytes));
+                    const uint32_t tm = tmem + (uint32_t)(sl * kFTiles * kFW);
+#pragma unroll
+                    for (int dy = 0; dy < 5; ++dy, ++g) {
+                        const uint32_t st = g % kFStages;
+                        if (!mbar_wait(&w_full[st], (g / kFStages) & 1, WL)) { fail(93); goto done_mma; }
                         tc_fence_after();
-                        const uint64_t a_base = sdesc_sw128(smem_u32(buf + sl * kFBufBytes));
-                        const uint32_t tm = tmem + (uint32_t)(sl * kFTiles * kFW);
-                        for (int dy = 0; dy < 5; ++dy, ++g) {
-                            const int st = g % kFStages;
-                            const uint32_t k = g / kFStages;
-                            if (!mbar_wait(&w_full[st], k & 1, WL)) { fail(93); goto done_mma; }
-                            tc_fence_after();
-                            const uint64_t a0 = a_base + (uint64_t)((kFPre + kFPitch * (dy - 2)) * 8);
-                            const uint64_t b0 = b_base + (uint64_t)(st * (kFSlice >> 4));
+                        const uint64_t a0 = a_base + (uint64_t)((kFPre + kFPitch * (dy - 2)) * 8);
+                        const uint64_t b0 = b_base + (uint64_t)(st * (uint32_t)(kFSlice >> 4));
+                        if (elect_one()) {
                             if (h == 0 && dy == 0)
                                 fast_slice<true>(tm, a0, b0, idesc);
                             else
                                 fast_slice<false>(tm, a0, b0, idesc);
                             mma_commit(&w_empty[st]);
+                            if (dy == 4) mma_commit(h == 0 ? &half_done[sl] : &acc_full[sl]);
                         }
-                        mma_commit(h == 0 ? &half_done[sl] : &acc_full[sl]);
+                        __syncwarp();
                     }
-                for (int l = 1; l < nl; ++l)
-                    for (int sl = 0; sl < kFSlots; ++sl) {
-                        if (!mbar_wait(&act_ready[sl], n_act[sl] & 1, WL)) { fail(94); goto done_mma; }
-                        ++n_act[sl];
+                }
+            for (int l = 1; l < nl; ++l)
+                for (int sl = 0; sl < NS; ++sl) {
+                    if (!mbar_wait(&act_ready[sl], n_act[sl] & 1, WL)) { fail(94); goto done_mma; }
+                    ++n_act[sl];
+                    const uint64_t a_base = sdesc_sw128(smem_u32(buf + sl * kFBufBytes));
+                    const uint32_t tm = tmem + (uint32_t)(sl * kFTiles * kFW);
+#pragma unroll
+                    for (int tap = 0; tap < 9; ++tap, ++g) {
+                        const uint32_t st = g % kFStages;
+                        if (!mbar_wait(&w_full[st], (g / kFStages) & 1, WL)) { fail(95); goto done_mma; }
                         tc_fence_after();
-                        const uint64_t a_base = sdesc_sw128(smem_u32(buf + sl * kFBufBytes));
-                        const uint32_t tm = tmem + (uint32_t)(sl * kFTiles * kFW);
-                        for (int tap = 0; tap < 9; ++tap, ++g) {
-                            const int st = g % kFStages;
-                            const uint32_t k = g / kFStages;
-                            if (!mbar_wait(&w_full[st], k & 1, WL)) { fail(95); goto done_mma; }
-                            tc_fence_after();
-                            const int shift = kFPitch * (tap / 3 - 1) + (tap % 3 - 1);
-                            const uint64_t a0 = a_base + (uint64_t)((kFPre + shift) * 8);
-                            const uint64_t b0 = b_base + (uint64_t)(st * (kFSlice >> 4));
+                        const int shift = kFPitch * (tap / 3 - 1) + (tap % 3 - 1);
+                        const uint64_t a0 = a_base + (uint64_t)((kFPre + shift) * 8);
+                        const uint64_t b0 = b_base + (uint64_t)(st * (uint32_t)(kFSlice >> 4));
+                        if (elect_one()) {
                             if (tap == 0)
                                 fast_slice<true>(tm, a0, b0, idesc);
                             else
                                 fast_slice<false>(tm, a0, b0, idesc);
                             mma_commit(&w_empty[st]);
+                            if (tap == 8) mma_commit(&acc_full[sl]);
                         }
-                        mma_commit(&acc_full[sl]);
+                        __syncwarp();
                     }
-            }
-        done_mma:
-            // every MMA this thread issued has completed before the CTA can
-            // free its tensor memory (also after a wait gave up)
+                }
+        }
+    done_mma:
+        // every MMA issued has completed before the CTA can free its tensor
+        // memory (also after a wait gave up)
+        __syncwarp();
+        if (elect_one()) {
             mma_commit(&mma_done);
             mbar_wait(&mma_done, 0, 1u << 20);
         }
@@ -290,12 +308,12 @@ __global__ void __launch_bounds__(kFThreads, 1)
         // ------------------------------------------------ staging + epilogue
         const int e = tid - 64;
         const int qd = warp & 3;          // TMEM lane quarter this warp may read
-        const int chh = (warp - 2) >> 2;  // channels 32*chh .. 32*chh + 31
+        const int chq = (warp - 2) >> 2;  // channels 16*chq .. 16*chq + 15
         const int c_in = p.c_in;
         uint32_t n_half[kFSlots] = {0, 0}, n_acc[kFSlots] = {0, 0}, n_epi = 0;
-        auto boards = [&](int grp) { return min(kFSlots, p.B - grp * kFSlots); };
+        auto boards = [&](int grp) { return min(NS, p.B - grp * NS); };
 
-        // barrier of the 8 staging / epilogue warps (bounded)
+        // barrier of the staging / epilogue warps (bounded)
         auto epi_sync = [&]() -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(&epi_bar);
@@ -305,7 +323,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
             return ok;
         };
         auto copy_planes = [&](int grp) {
-            const uint8_t *src = p.planes + (size_t)grp * kFSlots * c_in * kPoints;
+            const uint8_t *src = p.planes + (size_t)grp * NS * c_in * kPoints;
             const int words = boards(grp) * c_in * kPoints / 4;
             for (int i = e; i < words; i += kFEpiThreads) cp_async4(pl + 4 * i, src + 4 * i);
             cp_async_commit();
@@ -368,7 +386,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
         // both halves of group grp's first-layer rows, slot by slot, each
         // second half once that slot's first-half MMAs have completed
         auto stage_second_halves = [&](int grp) -> bool {
-            for (int sl = 0; sl < kFSlots; ++sl) {
+            for (int sl = 0; sl < NS; ++sl) {
                 if (!mbar_wait(&half_done[sl], n_half[sl] & 1, WL)) { fail(97); return false; }
                 ++n_half[sl];
                 stage(sl, 1, boards(grp));
@@ -382,7 +400,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
             copy_planes(g0);
             if (!build_masks(g0)) goto done_epi;
             if (g0 + G < ngroups) copy_planes(g0 + G);
-            for (int sl = 0; sl < kFSlots; ++sl) {
+            for (int sl = 0; sl < NS; ++sl) {
                 stage(sl, 0, boards(g0));
                 stage_done(sl);
             }
@@ -406,51 +424,56 @@ __global__ void __launch_bounds__(kFThreads, 1)
             }
             for (int l = 0; l < nl; ++l) {
                 const bool last = l == nl - 1;
-                const float *bias = s_bias + l * kFW + chh * 32;
-                for (int sl = 0; sl < kFSlots; ++sl) {
+                // (read once: the stores below may not be moved over them)
+                float bias[16];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    *reinterpret_cast<float4 *>(bias + 4 * i) =
+                        *reinterpret_cast<const float4 *>(s_bias + l * kFW + chq * 16 + 4 * i);
+                for (int sl = 0; sl < NS; ++sl) {
                     if (!mbar_wait(&acc_full[sl], n_acc[sl] & 1, WL)) { fail(98); goto done_epi; }
                     ++n_acc[sl];
                     tc_fence_after();
                     const uint32_t vm = sl < nb ? vmask : 0u;
                     const uint32_t t_row = tmem + ((uint32_t)(32 * qd) << 16) +
-                                           (uint32_t)(sl * kFTiles * kFW + 32 * chh);
+                                           (uint32_t)(sl * kFTiles * kFW + 16 * chq);
                     uint8_t *sbuf = buf + sl * kFBufBytes;
 #pragma unroll
                     for (int t0 = 0; t0 < kFTiles; t0 += 2) {
-                        uint32_t v[2][32];
-                        tmem_ld32(t_row + (uint32_t)(kFW * t0), v[0]);
-                        tmem_ld32(t_row + (uint32_t)(kFW * (t0 + 1)), v[1]);
+                        uint32_t v[2][16];
+                        tmem_ld16(t_row + (uint32_t)(kFW * t0), v[0]);
+                        tmem_ld16(t_row + (uint32_t)(kFW * (t0 + 1)), v[1]);
                         tmem_ld_wait();
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
                             const int q = 128 * (t0 + u) + 32 * qd + lane;
                             const bool valid = (vm >> (t0 + u)) & 1u;
                             if (!last) {
-                                uint32_t w[16];
+                                uint32_t w[8];
 #pragma unroll
-                                for (int i = 0; i < 16; ++i)
+                                for (int i = 0; i < 8; ++i)
                                     w[i] = valid ? relu_bf16x2(__uint_as_float(v[u][2 * i]) + bias[2 * i],
                                                                __uint_as_float(v[u][2 * i + 1]) + bias[2 * i + 1])
                                                  : 0u;
                                 const int R = q + kFPre;
                                 uint8_t *row = sbuf + R * 128;
 #pragma unroll
-                                for (int k = 0; k < 4; ++k)
-                                    *reinterpret_cast<uint4 *>(row + (((4 * chh + k) ^ (R & 7)) << 4)) =
+                                for (int k = 0; k < 2; ++k)
+                                    *reinterpret_cast<uint4 *>(row + (((2 * chq + k) ^ (R & 7)) << 4)) =
                                         make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
                             } else {
                                 float sp = 0.0f, sv = 0.0f;
 #pragma unroll
-                                for (int i = 0; i < 32; ++i) {
+                                for (int i = 0; i < 16; ++i) {
                                     const float f = fmaxf(__uint_as_float(v[u][i]) + bias[i], 0.0f);
-                                    sp = fmaf(f, s_wp[32 * chh + i], sp);
-                                    sv = fmaf(f, s_wv[32 * chh + i], sv);
+                                    sp = fmaf(f, s_wp[16 * chq + i], sp);
+                                    sv = fmaf(f, s_wv[16 * chq + i], sv);
                                 }
                                 if (valid) {
                                     const int y = q / kFPitch, x = q - y * kFPitch;
-                                    const size_t idx = (size_t)(grp * kFSlots + sl) * kPoints + y * kBoard + x;
-                                    p.parts_p[chh * p.part_stride + idx] = sp;
-                                    p.parts_v[chh * p.part_stride + idx] = sv;
+                                    const size_t idx = (size_t)(grp * NS + sl) * kPoints + y * kBoard + x;
+                                    p.parts_p[chq * p.part_stride + idx] = sp;
+                                    p.parts_v[chq * p.part_stride + idx] = sv;
                                 }
                             }
                         }
@@ -601,7 +624,7 @@ struct lg_fast {
     float bp = 0.0f, bv = 0.0f;
     float *w1s = nullptr, *b1 = nullptr, *w2 = nullptr;  // FC1 sliced [H/64][361][64], b1, w2
     float b2 = 0.0f;
-    float *parts = nullptr;      // [4][max_batch * 361]: policy halves, value halves
+    float *parts = nullptr;      // [2][kFParts][max_batch * 361]: policy, value
     float *fcpart = nullptr;
     int *fccnt = nullptr;        // value-head group counters, zero between launches
     float *entropy = nullptr;    // [max_batch]
@@ -734,16 +757,19 @@ int fast_forward(lg_fast *f, const uint8_t *planes, int B, float T, float *probs
     p.wv = f->wv;
     p.part_stride = (size_t)f->max_batch * kPoints;
     p.parts_p = f->parts;
-    p.parts_v = f->parts + 2 * p.part_stride;
+    p.parts_v = f->parts + kFParts * p.part_stride;
     p.err = f->err;
     p.wait_limit = kFWaitLimit;
-    const int groups = (B + kFSlots - 1) / kFSlots;
+    // one board a CTA while every board has an SM of its own
+    p.slots = B <= f->sm_count ? 1 : kFSlots;
+    const int groups = (B + p.slots - 1) / p.slots;
     const int grid = groups < f->sm_count ? groups : f->sm_count;
     fast_trunk_kernel<<<grid, kFThreads, kFSmem, s>>>(f->w_map, p);
-    HeadIn hp{p.parts_p, 2, p.part_stride, f->bp, 0, LG_ACT_RELU, logits};
-    launch_softmax(hp, B, T, probs, s, entropy ? entropy : f->entropy);
-    HeadIn hv{p.parts_v, 2, p.part_stride, f->bv, 0, LG_ACT_RELU, nullptr};
-    launch_value_fc(hv, B, f->w1s, f->b1, f->w2, f->b2, f->H, LG_ACT_RELU, 0, value, f->fcpart, f->fccnt, s);
+    HeadIn hp{p.parts_p, kFParts, p.part_stride, f->bp, 0, LG_ACT_RELU, logits};
+    launch_softmax(hp, B, T, probs, s, entropy ? entropy : f->entropy, true);
+    HeadIn hv{p.parts_v, kFParts, p.part_stride, f->bv, 0, LG_ACT_RELU, nullptr};
+    launch_value_fc(hv, B, f->w1s, f->b1, f->w2, f->b2, f->H, LG_ACT_RELU, 0, value, f->fcpart, f->fccnt, s,
+                    true);
     *nlaunch = 3;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -846,7 +872,7 @@ extern "C" LG_API int lg_fast_create(int device, int c_in, int n3x3, int fc_hidd
     if (!rc) rc = fast_alloc(f, &f->w1s, (size_t)slices * kPoints * 64);
     if (!rc) rc = fast_alloc(f, &f->b1, fc_hidden);
     if (!rc) rc = fast_alloc(f, &f->w2, fc_hidden);
-    if (!rc) rc = fast_alloc(f, &f->parts, 4 * (size_t)max_batch * kPoints);
+    if (!rc) rc = fast_alloc(f, &f->parts, 2 * kFParts * (size_t)max_batch * kPoints);
     if (!rc) rc = fast_alloc(f, &f->fcpart, value_fc_part_floats(max_batch, fc_hidden));
     if (!rc) rc = fast_alloc(f, &f->fccnt, value_fc_counter_ints(max_batch, fc_hidden));
     if (!rc && cudaMemset(f->fccnt, 0, sizeof(int) * value_fc_counter_ints(max_batch, fc_hidden)) != cudaSuccess)
