@@ -96,7 +96,7 @@ __device__ __forceinline__ void gather_board(const int8_t *__restrict__ squares,
     __shared__ uint32_t rowc[2][kBoard];  // row bitboard: bit x of rowc[c][y] = stone of colour c at (y, x)
     __shared__ short cand[kCand];         // ladder candidates: point | kind << 9 (0 ladder, 1 ladder win)
     __shared__ uint8_t lad_yes[extra ? kPoints : 1], win_yes[extra ? kPoints : 1];
-    __shared__ int ncand;
+    __shared__ int ncand, next_cand;
     __shared__ int8_t sq[kPoints];
     __shared__ short lab[kPoints];
     __shared__ __align__(16) uint32_t stones[kPoints][kWords];
@@ -129,7 +129,7 @@ __device__ __forceinline__ void gather_board(const int8_t *__restrict__ squares,
     }
     if (p < kWords) empty[p] = 0;
     if (extra && p < 2 * kBoard) rowc[p / kBoard][p % kBoard] = 0;
-    if (extra && p == 0) ncand = 0;
+    if (extra && p == 0) ncand = next_cand = 0;
     __syncthreads();
     // string labels: the minimum point index of the string, by union-find:
     // every stone links to its left and upper neighbours of its colour (the
@@ -293,13 +293,18 @@ __device__ __forceinline__ void gather_board(const int8_t *__restrict__ squares,
     }
     if (extra) {
         __syncthreads();
-        // one warp per candidate; the row board in registers (lane y = row y)
-        const int lane = p & 31, warp = p >> 5, nwarps = blockDim.x >> 5;
+        // One warp per candidate, taken one by one (a ladder is read in 2 to
+        // 60 us); the row board in registers (lane y = row y).
+        const int lane = p & 31;
         lad::Board wb;
         wb.c[0] = lane < kBoard ? rowc[0][lane] : 0u;
         wb.c[1] = lane < kBoard ? rowc[1][lane] : 0u;
         const int n = ncand;
-        for (int i = warp; i < n; i += nwarps) {
+        for (;;) {
+            int i = 0;
+            if (lane == 0) i = atomicAdd(&next_cand, 1);
+            i = __shfl_sync(0xffffffffu, i, 0);
+            if (i >= n) break;
             const int e = cand[i], q = e & 0x1ff;
             if (e >> 9) {
                 const bool yes = lad::winning_ladder(wb, tomove, q);
@@ -397,12 +402,15 @@ __device__ __forceinline__ void gather_board(const int8_t *__restrict__ squares,
     for (int i = 0; i < nplanes; ++i) dst[(size_t)i * kPoints] = (uint8_t)((bits >> i) & 1u);
 }
 
+// (With the ladder reader two CTAs an SM: its eight floods at once want 80
+// registers; at 56, three CTAs, they spill and 1,000 boards take 327 us for
+// both sets against 301.)
 // Launched as a programmatic dependent of a trunk, the gather runs on the
 // SMs the trunk's CTAs leave (its output must be rows that trunk does not
 // read) and waits for the trunk only before it exits, so that a kernel which
 // waits for the gather has the trunk's results too.
 template <int WHICH, bool EXTRA, bool L5>
-__global__ void __launch_bounds__(384, 3) gather_kernel(const int8_t *__restrict__ squares,
+__global__ void __launch_bounds__(384, EXTRA ? 2 : 3) gather_kernel(const int8_t *__restrict__ squares,
                                                      const int8_t *__restrict__ to_move,
                                                      const int32_t *__restrict__ moves, int B,
                                                      int nplanes, uint8_t *__restrict__ planes, int halves,

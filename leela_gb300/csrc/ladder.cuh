@@ -18,6 +18,16 @@
 // Every function here is called by all 32 lanes of a warp with the same
 // (warp-uniform) arguments and returns the same value on every lane.
 //
+// What bounds it is one warp's latency: a step of a ladder looks at the
+// strings around two liberties and an escape, each found by a flood of
+// dependent shuffles.  They are flooded side by side, each once (the hunted
+// string is carried along), and every question -- captures, suicide, self-
+// atari, liberties after a move -- is answered from those masks: 1,000 boards,
+// both plane sets, 301 us against 595 with a flood per question and neighbour;
+// 8,192 boards 1.79 against 6.5 ms.  Tried and slower: a kernel of one-warp
+// CTAs for the candidates (330 us), lines shared between the CTA's warps at
+// even choices (347), floods started from the gathered board's strings (357).
+//
 // check_losing_ladder recurses on even choices (both ataris tried, result
 // OR-ed, at most 5 levels of branching); here that is a depth-first search
 // with an explicit stack of at most 6 pending lines, stopping at the first
@@ -80,164 +90,182 @@ __device__ __forceinline__ uint32_t runs_of(uint32_t x, uint32_t r) {
     return run_up(x, r) | __brev(run_up(__brev(x), __brev(r)));
 }
 
-// the string of colour-mask `st` through point p (p must be in st): whole
-// runs of a row at a time, then a step to the rows above and below
-__device__ __forceinline__ uint32_t string_of(uint32_t st, int p) {
-    uint32_t s = point_mask(p);
+// N strings at once: each s[k], seeded inside colour-mask st[k], grown to the
+// strings it touches.  Whole runs of a row at a time, then a step to the rows
+// above and below; the floods share a step's latency (75 cycles of dependent
+// shuffles, and a vote).
+template <int N>
+__device__ __forceinline__ void flood(uint32_t (&s)[N], const uint32_t (&st)[N]) {
     for (int it = 0; it < 400; ++it) {
-        s = runs_of(s, st);
-        uint32_t up = __shfl_up_sync(kAll, s, 1);
-        const uint32_t dn = __shfl_down_sync(kAll, s, 1);
-        if (lane_id() == 0) up = 0;
-        const uint32_t n = s | ((up | dn) & st);
-        if (!any(n ^ s)) break;
-        s = n;
-    }
-    return s;
-}
-
-// liberties of string s (as a mask)
-__device__ __forceinline__ uint32_t liberty_mask(const Board &b, uint32_t s) { return dilate(s) & empties(b); }
-
-__device__ __forceinline__ int nbr(int p, int k) {
-    const int x = p % kBoard, y = p / kBoard;
-    switch (k) {
-    case 0: return x > 0 ? p - 1 : -1;
-    case 1: return x < kBoard - 1 ? p + 1 : -1;
-    case 2: return y > 0 ? p - kBoard : -1;
-    default: return y < kBoard - 1 ? p + kBoard : -1;
+        uint32_t changed = 0;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const uint32_t t = runs_of(s[k], st[k]);
+            uint32_t up = __shfl_up_sync(kAll, t, 1);
+            const uint32_t dn = __shfl_down_sync(kAll, t, 1);
+            if (lane_id() == 0) up = 0;
+            s[k] = t | ((up | dn) & st[k]);
+            changed |= s[k] ^ t;
+        }
+        if (!any(changed)) break;
     }
 }
 
-// colour at p: 0, 1, or 2 (empty)
-__device__ __forceinline__ int color_at(const Board &b, int p) {
-    const int y = p / kBoard, x = p % kBoard;
-    const uint32_t r0 = row_of(b.c[0], y), r1 = row_of(b.c[1], y);
-    return ((r0 >> x) & 1u) ? 0 : (((r1 >> x) & 1u) ? 1 : 2);
+// The four neighbours of a point: colour (0, 1, 2 empty, 3 off the board),
+// the strings through its stones (0 elsewhere) and their liberties.
+struct Around {
+    int v;
+    int c[4];
+    uint32_t s[4], l[4];
+};
+
+__device__ __forceinline__ void neighbour_colours(const Board &b, int v, int (&c)[4]) {
+    const int y = v / kBoard, x = v - y * kBoard;
+    const int yu = y > 0 ? y - 1 : y, yd = y < kBoard - 1 ? y + 1 : y;
+    const uint32_t b0 = row_of(b.c[0], y), w0 = row_of(b.c[1], y);
+    const uint32_t bu = row_of(b.c[0], yu), wu = row_of(b.c[1], yu);
+    const uint32_t bd = row_of(b.c[0], yd), wd = row_of(b.c[1], yd);
+    auto at = [](uint32_t bl, uint32_t wh, int i) { return (bl >> i & 1u) ? 0 : ((wh >> i & 1u) ? 1 : 2); };
+    c[0] = x > 0 ? at(b0, w0, x - 1) : 3;
+    c[1] = x < kBoard - 1 ? at(b0, w0, x + 1) : 3;
+    c[2] = y > 0 ? at(bu, wu, x) : 3;
+    c[3] = y < kBoard - 1 ? at(bd, wd, x) : 3;
 }
 
-// liberties of the string through the stone at p
-__device__ __forceinline__ int libs_at(const Board &b, int p) {
-    return popc(liberty_mask(b, string_of(stones(b, color_at(b, p)), p)));
+__device__ __forceinline__ uint32_t neighbour_mask(int v, int k) {
+    return point_mask(k == 0 ? v - 1 : (k == 1 ? v + 1 : (k == 2 ? v - kBoard : v + kBoard)));
 }
 
-__device__ __forceinline__ int count_empty_nbrs(const Board &b, int v) {
-    const uint32_t e = empties(b);
-    const int y = v / kBoard, x = v % kBoard;
-    const uint32_t r0 = row_of(e, y);
-    const uint32_t ru = row_of(e, y > 0 ? y - 1 : y), rd = row_of(e, y < kBoard - 1 ? y + 1 : y);
-    int n = 0;
-    if (x > 0) n += (r0 >> (x - 1)) & 1u;
-    if (x < kBoard - 1) n += (r0 >> (x + 1)) & 1u;
-    if (y > 0) n += (ru >> x) & 1u;
-    if (y < kBoard - 1) n += (rd >> x) & 1u;
-    return n;
-}
-
-// FastBoard::update_board_fast: place, capture opponent strings without
-// liberties, remove the new string if it has none
-__device__ void play(Board &b, int color, int v) {
-    const uint32_t own = stones(b, color) | point_mask(v);
-    set_stones(b, color, own);
-    uint32_t opp = stones(b, 1 - color);
-#pragma unroll 1
-    for (int k = 0; k < 4; ++k) {
-        const int q = nbr(v, k);
-        if (q < 0 || !test(opp, q)) continue;
-        const uint32_t s = string_of(opp, q);
-        if (!any(liberty_mask(b, s))) {
-            opp &= ~s;
-            set_stones(b, 1 - color, opp);
+// Around of N points at once.  known: a whole string of the board (or 0),
+// taken as it is where a neighbour belongs to it.
+template <int N>
+__device__ __forceinline__ void look(const Board &b, const int (&v)[N], uint32_t known, Around (&a)[N]) {
+    uint32_t s[4 * N], st[4 * N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        a[i].v = v[i];
+        neighbour_colours(b, v[i], a[i].c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int c = a[i].c[k], j = 4 * i + k;
+            st[j] = c < 2 ? stones(b, c) : 0u;
+            s[j] = c < 2 ? neighbour_mask(v[i], k) : 0u;
+            if (any(s[j] & known)) s[j] = known;
         }
     }
-    const uint32_t s = string_of(own, v);
-    if (!any(liberty_mask(b, s))) set_stones(b, color, own & ~s);
+    flood(s, st);
+    const uint32_t e = empties(b);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            a[i].s[k] = s[4 * i + k];
+            a[i].l[k] = dilate(s[4 * i + k]) & e;
+        }
+}
+
+__device__ __forceinline__ int empty_neighbours(const Around &a) {
+    return (a.c[0] == 2) + (a.c[1] == 2) + (a.c[2] == 2) + (a.c[3] == 2);
+}
+
+// FastBoard::update_board_fast at a.v (a: taken on b): place, capture opponent
+// strings without liberties, remove the new string if it has none.  The new
+// string in own_out (0 if it was removed), its liberties in libs_out.
+__device__ __forceinline__ void play(Board &b, int color, const Around &a, uint32_t &own_out, uint32_t &libs_out) {
+    const uint32_t pt = point_mask(a.v);
+    uint32_t own = pt, dead = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (a.c[k] == color) own |= a.s[k];
+        if (a.c[k] == 1 - color && !any(a.l[k] & ~pt)) dead |= a.s[k];
+    }
+    set_stones(b, 1 - color, stones(b, 1 - color) & ~dead);
+    set_stones(b, color, stones(b, color) | pt);
+    uint32_t l = dilate(own) & empties(b);
+    if (!any(l)) {
+        set_stones(b, color, stones(b, color) & ~own);
+        own = 0;
+    }
+    own_out = own;
+    libs_out = l;
+}
+
+// FastBoard::after_liberties_color: liberties of the string formed by playing
+// a.v, 0 for a suicide
+__device__ __forceinline__ int after_libs(const Board &b, int color, const Around &a) {
+    Board t = b;
+    uint32_t own, l;
+    play(t, color, a, own, l);
+    return popc(l);
 }
 
 // FastBoard::minimum_elib_count: fewest liberties among the opponent strings
-// next to the point v itself (100 if none)
-__device__ int min_elib(const Board &b, int color, int v) {
+// next to the point itself (100 if none)
+__device__ __forceinline__ int min_elib(const Around &a, int color) {
     int best = 100;
-    const uint32_t opp = stones(b, 1 - color);
-#pragma unroll 1
-    for (int k = 0; k < 4; ++k) {
-        const int q = nbr(v, k);
-        if (q < 0 || !test(opp, q)) continue;
-        best = min(best, popc(liberty_mask(b, string_of(opp, q))));
-    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (a.c[k] == 1 - color) best = min(best, popc(a.l[k]));
     return best;
-}
-
-// FastBoard::is_suicide
-__device__ bool is_suicide(const Board &b, int v, int color) {
-    if (count_empty_nbrs(b, v) > 0) return false;
-#pragma unroll 1
-    for (int k = 0; k < 4; ++k) {
-        const int q = nbr(v, k);
-        if (q < 0) continue;
-        const int cq = color_at(b, q);  // a stone: v has no empty neighbour
-        const int l = popc(liberty_mask(b, string_of(stones(b, cq), q)));
-        if (cq == color ? l > 1 : l <= 1) return false;
-    }
-    return true;
 }
 
 // FastBoard::self_atari (fewer than two empty neighbours, no capture, no
 // connection to 3+ liberties, and v + empty neighbours + liberties of the own
-// neighbour strings with 2+ liberties number at most two)
-__device__ bool self_atari(const Board &b, int color, int v) {
-    if (count_empty_nbrs(b, v) >= 2) return false;
-    uint32_t set = point_mask(v);
-#pragma unroll 1
+// neighbour strings with 2+ liberties number at most two); with suicide,
+// FastBoard::is_suicide (no empty neighbour, no own string next to it with
+// another liberty, no opponent string in atari) counts too
+__device__ __forceinline__ bool self_atari(const Around &a, int color, bool suicide) {
+    const int ne = empty_neighbours(a);
+    if (ne >= 2) return false;
+    uint32_t set = point_mask(a.v);
+    bool safe = false, escapes = false;
+#pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int q = nbr(v, k);
-        if (q < 0) continue;
-        const int c = color_at(b, q);
-        if (c == 2) {
-            set |= point_mask(q);
-            continue;
-        }
-        const uint32_t l = liberty_mask(b, string_of(stones(b, c), q));
-        const int nl = popc(l);
-        if ((c == 1 - color && nl <= 1) || (c == color && nl >= 3)) return false;
-        if (c == color && nl > 1) set |= l;
+        if (a.c[k] == 2) set |= neighbour_mask(a.v, k);
+        if (a.c[k] >= 2) continue;
+        const int n = popc(a.l[k]);
+        const bool own = a.c[k] == color;
+        safe = safe || (own ? n >= 3 : n <= 1);
+        escapes = escapes || (own ? n > 1 : n <= 1);
+        if (own && n > 1) set |= a.l[k];
     }
-    return popc(set) <= 2;
+    if (suicide && ne == 0 && !escapes) return true;
+    return !safe && popc(set) <= 2;
 }
 
-// FastBoard::after_liberties_color: liberties of the string formed by playing
-// v, 0 for a suicide
-__device__ int after_libs(const Board &b, int color, int v) {
-    if (is_suicide(b, v, color)) return 0;
-    Board t = b;
-    play(t, color, v);
-    return libs_at(t, v);
-}
-
-// the own strings in atari next to vtx: exactly one, which cannot capture
+// the own strings in atari next to a.v: exactly one, which cannot capture
 // an attacker (check_losing_ladder's opening tests)
-__device__ bool lone_critical_string(const Board &b, int color, int vtx) {
-    const uint32_t own = stones(b, color), opp = stones(b, 1 - color);
+__device__ __forceinline__ bool lone_critical_string(const Board &b, int color, const Around &a) {
+    const uint32_t opp = stones(b, 1 - color);
     uint32_t crit = 0;
     int ncrit = 0;
-#pragma unroll 1
+#pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int q = nbr(vtx, k);
-        if (q < 0 || !test(own, q) || test(crit, q)) continue;
-        const uint32_t s = string_of(own, q);
-        if (popc(liberty_mask(b, s)) > 1) continue;
+        if (a.c[k] != color || any(crit & a.s[k]) || popc(a.l[k]) > 1) continue;
         ++ncrit;
-        crit |= s;
+        crit |= a.s[k];
     }
     if (ncrit != 1) return false;
-    // any attacker string next to it in atari?
+    // any attacker string next to it in atari?  Three at a time, from three
+    // points next to it (of one string, perhaps)
     uint32_t d = dilate(crit) & opp;
+    const uint32_t e = empties(b);
     for (int it = 0; it < kPoints; ++it) {
-        const int q = first_point(d);
-        if (q < 0) break;
-        const uint32_t s = string_of(opp, q);
-        if (popc(liberty_mask(b, s)) <= 1) return false;
-        d &= ~s;
+        uint32_t s[3], st[3] = {opp, opp, opp};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int q = first_point(d);
+            s[k] = q >= 0 ? point_mask(q) : 0u;
+            d &= ~s[k];
+        }
+        if (!any(s[0])) break;
+        flood(s, st);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int n = popc(dilate(s[k]) & e);
+            if (n <= 1 && any(s[k])) return false;
+            d &= ~s[k];
+        }
     }
     return true;
 }
@@ -249,7 +277,9 @@ struct Alt {
 
 // FastBoard::check_losing_ladder(color, vtx): `color` (to move) saves its
 // string in atari next to vtx by playing there; true if the attacker can
-// keep it in atari until it dies.  Depth-first over the even choices.
+// keep it in atari until it dies.  Depth-first over the even choices.  The
+// hunted string is carried from move to move, so a step floods only the
+// other strings next to its two liberties and to the escape.
 __device__ bool losing_ladder(const Board &start, int color, int vtx0) {
     Alt stack[6];
     int top = 0;
@@ -261,81 +291,109 @@ __device__ bool losing_ladder(const Board &start, int color, int vtx0) {
         --top;
         Board b = stack[top].b;
         const int vtx = stack[top].vtx, branching = stack[top].branching;
-        bool result = false;
-        if (branching <= 5) {
-            const int elib = min_elib(b, color, vtx);
-            if (elib != 0 && elib != 1 && lone_critical_string(b, color, vtx)) {
-                int atari = vtx;
-                play(b, color, vtx);
-                for (int step = 0; step < 400; ++step) {
-                    const uint32_t own = stones(b, color);
-                    if (!test(own, atari)) { result = true; break; }   // the escape was a suicide
-                    uint32_t l = liberty_mask(b, string_of(own, atari));
-                    const int nl = popc(l);
-                    if (nl == 1) { result = true; break; }              // self-atari
-                    if (nl >= 3) break;                                  // escaped
-                    if (min_elib(b, color, atari) == 1) break;           // counter-atari
-                    const int lib0 = first_point(l);
-                    l &= ~point_mask(lib0);
-                    const int lib1 = first_point(l);
-                    if (count_empty_nbrs(b, lib0) == 3 && count_empty_nbrs(b, lib1) == 3) break;
-                    int l0 = after_libs(b, color, lib0), l1 = after_libs(b, color, lib1);
-                    const bool s0 = is_suicide(b, lib0, 1 - color) || self_atari(b, 1 - color, lib0);
-                    const bool s1 = is_suicide(b, lib1, 1 - color) || self_atari(b, 1 - color, lib1);
-                    if (s0 && s1) break;
-                    if (s0) l1 = l0 + 1;
-                    if (s1) l0 = l1 + 1;
-                    if (l0 == l1) {
-                        // both ataris, each followed by the escape at the
-                        // other liberty; lines at branching depth 6 fail at
-                        // once, so a depth-5 branch is a failed line (and the
-                        // stack holds at most one pending line per depth)
-                        if (branching + 1 > 5) break;
-                        stack[top].b = b;
-                        play(stack[top].b, 1 - color, lib1);
-                        stack[top].vtx = lib0;
-                        stack[top].branching = branching + 1;
-                        ++top;
-                        stack[top].b = b;
-                        play(stack[top].b, 1 - color, lib0);
-                        stack[top].vtx = lib1;
-                        stack[top].branching = branching + 1;
-                        ++top;
-                        break;
-                    }
-                    play(b, 1 - color, l0 > l1 ? lib0 : lib1);
-                    // the string is back in atari: its one liberty is the next saving move
-                    l = liberty_mask(b, string_of(stones(b, color), atari));
-                    if (popc(l) != 1) break;
-                    const int next = first_point(l);
-                    play(b, color, next);
-                    atari = next;
-                }
-            }
+        if (branching > 5) continue;
+        Around at[1];
+        {
+            const int v[1] = {vtx};
+            look<1>(b, v, 0u, at);
         }
-        if (result) return true;
+        const int elib = min_elib(at[0], color);
+        if (elib == 0 || elib == 1 || !lone_critical_string(b, color, at[0])) continue;
+        uint32_t own, l;
+        play(b, color, at[0], own, l);
+        for (int step = 0; step < 400; ++step) {
+            const int nl = popc(l);
+            if (nl <= 1) return true;  // the escape was a suicide, or a self-atari
+            if (nl >= 3) break;        // escaped
+            {
+                // fewest liberties of the attacker's strings next to the escape
+                // point, as they are after it
+                const uint32_t e = empties(b), opp = stones(b, 1 - color);
+                int best = 100;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t s = at[0].c[k] == 1 - color ? at[0].s[k] & opp : 0u;
+                    const int n = popc(dilate(s) & e);
+                    if (any(s)) best = min(best, n);
+                }
+                if (best == 1) break;  // counter-atari
+            }
+            const int lib0 = first_point(l);
+            const int lib1 = first_point(l & ~point_mask(lib0));
+            Around a[2];
+            {
+                const int v[2] = {lib0, lib1};
+                look<2>(b, v, own, a);
+            }
+            if (empty_neighbours(a[0]) == 3 && empty_neighbours(a[1]) == 3) break;
+            const bool s0 = self_atari(a[0], 1 - color, true), s1 = self_atari(a[1], 1 - color, true);
+            if (s0 && s1) break;
+            int first = s0 ? 1 : 0;  // the liberty that the attacker takes
+            if (!s0 && !s1) {
+                const int l0 = after_libs(b, color, a[0]), l1 = after_libs(b, color, a[1]);
+                if (l0 == l1) {
+                    // both ataris, each followed by the escape at the other
+                    // liberty; lines at branching depth 6 fail at once, so a
+                    // depth-5 branch is a failed line (and the stack holds at
+                    // most one pending line per depth)
+                    if (branching + 1 > 5) break;
+                    uint32_t o, f;
+                    stack[top].b = b;
+                    play(stack[top].b, 1 - color, a[1], o, f);
+                    stack[top].vtx = lib0;
+                    stack[top].branching = branching + 1;
+                    ++top;
+                    stack[top].b = b;
+                    play(stack[top].b, 1 - color, a[0], o, f);
+                    stack[top].vtx = lib1;
+                    stack[top].branching = branching + 1;
+                    ++top;
+                    break;
+                }
+                first = l0 > l1 ? 0 : 1;
+            }
+            uint32_t o, f;
+            if (first)
+                play(b, 1 - color, a[1], o, f);
+            else
+                play(b, 1 - color, a[0], o, f);
+            // the string is back in atari: its one liberty is the next saving move
+            l = dilate(own) & empties(b);
+            if (popc(l) != 1) break;
+            {
+                const int v[1] = {first_point(l)};
+                look<1>(b, v, own, at);
+            }
+            play(b, color, at[0], own, l);
+        }
     }
     return false;
 }
 
 // FastBoard::check_winning_ladder(color, vtx)
 __device__ bool winning_ladder(const Board &b, int color, int vtx) {
-    bool sa_known = false, sa = false;
-    const uint32_t opp = stones(b, 1 - color);
+    Around at[1];
+    {
+        const int v[1] = {vtx};
+        look<1>(b, v, 0u, at);
+    }
+    if (self_atari(at[0], color, false)) return false;
+    Board t = b;
+    uint32_t o, f;
+    play(t, color, at[0], o, f);
+    uint32_t done = 0;
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
-        const int q = nbr(vtx, k);
-        if (q < 0 || !test(opp, q)) continue;
-        if (popc(liberty_mask(b, string_of(opp, q))) != 2) continue;
-        if (!sa_known) {
-            sa = self_atari(b, color, vtx);
-            sa_known = true;
-        }
-        if (sa) continue;
-        Board t = b;
-        play(t, color, vtx);
-        const int esc = first_point(liberty_mask(t, string_of(stones(t, 1 - color), q)));
-        if (esc < 0 || count_empty_nbrs(t, esc) != 2) continue;
+        const int c = k == 0 ? at[0].c[0] : (k == 1 ? at[0].c[1] : (k == 2 ? at[0].c[2] : at[0].c[3]));
+        const uint32_t s = k == 0 ? at[0].s[0] : (k == 1 ? at[0].s[1] : (k == 2 ? at[0].s[2] : at[0].s[3]));
+        const uint32_t l = k == 0 ? at[0].l[0] : (k == 1 ? at[0].l[1] : (k == 2 ? at[0].l[2] : at[0].l[3]));
+        if (c != 1 - color || any(s & done) || popc(l) != 2) continue;
+        done |= s;
+        const int esc = first_point(dilate(s) & empties(t));
+        if (esc < 0) continue;
+        int ec[4];
+        neighbour_colours(t, esc, ec);
+        if ((ec[0] == 2) + (ec[1] == 2) + (ec[2] == 2) + (ec[3] == 2) != 2) continue;
         if (losing_ladder(t, 1 - color, esc)) return true;
     }
     return false;
