@@ -152,6 +152,7 @@ struct lg_ctx {
     float *d_parts = nullptr;  // fused-head partial sums, [4][max_batch * 361]
     float *d_fcpart = nullptr; // value-head FC partial sums
     int *d_fccnt = nullptr;    // value-head group counters, zero between launches
+    int cluster_boards = 0;    // boards whose clusters run side by side (cluster_trunk.cu)
     int *d_flags = nullptr;    // chunk flags and item counter of the persistent trunk kernel
     // pinned staging of the blocking calls, two slots so that chunk k+1 is
     // packed while chunk k runs: planes, outputs, logits, completion events
@@ -797,6 +798,16 @@ bool trunk_fusable(const Net &n) {
            n.tc[0].cout == 128;
 }
 
+// Choice 3 with a cluster of four CTAs a board while all of them run side by
+// side (36 boards: four 227 KB CTAs of a cluster must share a GPC): policy +
+// value pair 148 to 158 us from 1 to 36 positions, against 201 to 250 on the
+// trunk's items; in a second wave the clusters would take 300.  The same
+// results bit for bit.  Nets with another activation than ReLU, device-side
+// batch sizes and the stall hook stay on the trunk.
+bool use_cluster(const lg_ctx *c, const Net &n, int B, const TcTrunk &t) {
+    return B <= c->cluster_boards && t.buf5 && t.head_w && !t.count && t.stall_item < 0 && n.d.act == LG_ACT_RELU;
+}
+
 // next (optional): the following batch's planes, packed by CTAs of this
 // batch's finish launch into next->out, which must not be this batch's l5.
 // mid (optional): launches made between the layers and the finish (the
@@ -871,7 +882,9 @@ int forward_tc(lg_ctx *c, Net &n, const uint8_t *planes, int B, float T, float *
             int rc;
             {
                 ProfScope ps(c, prof, LG_PROF_TC_TRUNK, s);
-                rc = launch_tc_trunk(tt, c->d_parts, part_stride, c->d_flags, c->d_err, s, c->sm_count);
+                rc = use_cluster(c, n, B, tt)
+                         ? launch_cluster_trunk(tt, B, c->d_parts, part_stride, c->d_err, s)
+                         : launch_tc_trunk(tt, c->d_parts, part_stride, c->d_flags, c->d_err, s, c->sm_count);
             }
             if (rc) return rc;
             L += 1;
@@ -1625,6 +1638,7 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
             }
         } else {
             if ((rc = tc_init_device())) return fail(rc);
+            if (trunk_fusable(n) && (rc = cluster_trunk_init_device(&c->cluster_boards))) return fail(rc);
             max_tc_l3 = std::max(max_tc_l3, (size_t)n.d.width);
             max_tc_l5 = std::max(max_tc_l5, (size_t)n.tc[0].halves * 64);
         }

@@ -262,6 +262,11 @@ int launch_tc_trunk(const TcTrunk &T, float *parts, size_t part_stride, int *fla
 size_t trunk_flag_ints(int rows, int rows5);
 // index of the first work item of 3x3 layer k (rows5 = 0: no fused first layer)
 int trunk_layer_item(int rows, int rows5, int k);
+// The same layers (5x5 first layer, 3x3 ReLU layers, fused head; T.buf_a/b not
+// used) with a board's activations kept in the shared memory of a cluster, for
+// batches of up to *max_boards (cluster_trunk.cu).  parts as launch_tc_trunk.
+int cluster_trunk_init_device(int *max_boards);
+int launch_cluster_trunk(const TcTrunk &T, int B, float *parts, size_t part_stride, int *err, cudaStream_t s);
 size_t tc_conv_smem_bytes(int n, int ntaps, int cin_halves);
 int tc_init_device();
 // Head kernels for the tensor-core path (logits already produced by the

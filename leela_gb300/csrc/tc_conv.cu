@@ -1381,7 +1381,8 @@ int tc_head_parts(int n, int variant) { return (n == 128 && variant != 1) ? 4 : 
 // stores: ~5 us, the same for every size) and 72 MMAs of N = rows.  64-row
 // items while every SM has at most one (24 positions), 128-row items while
 // 256-row ones would leave SMs without any (97); then the largest, whose MMAs
-// run at the full rate and read each weight stage for the most rows.  Policy +
+// run at the full rate and read each weight stage for the most rows.  (ReLU nets
+// of up to 36 positions run in clusters instead, cluster_trunk.cu.)  Policy +
 // value pair, us, with 64 / 128 / 256 rows: 8 positions 217 / 220 / 253, 24
 // positions 233 / 235 / 269, 48 positions 277 / 252 / 283, 96 positions
 // 486 / 294 / 300, 128 positions 633 / 356 / 316.  Every output is the same
