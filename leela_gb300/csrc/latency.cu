@@ -21,7 +21,7 @@
 //
 // CTA c (grid G, a multiple of 8, one CTA per SM) always takes split
 // s = c % 8 and rows c/8, c/8 + G/8, ...; its weight slice of a layer is one
-// contiguous block, copied into shared memory with cp.async while the
+// contiguous block, brought into shared memory by one bulk copy while the
 // previous layer computes.  Units publish "row done" by a release add on a
 // per-(layer, row) counter; a unit waits (bounded acquire polls) until the
 // rows its taps read are complete in the layer before -- and, so that it
@@ -29,6 +29,14 @@
 // that read the same rows of the layer before it are complete.  No
 // grid-wide barrier; the last CTA to leave resets the counters for the next
 // launch.
+//
+// What bounds it at one position: the hand-over of a layer (~5k of 7.7k cycles
+// in 16-bit nets, 12k in FP32: the release's fence, the counters' polls, a
+// round trip for the partial sums).  BF16 policy + value pair 121 us, 128 with
+// the weights copied by every thread and bias and scale read after the partial
+// sums.  Tried and not kept: each partial sum with a tag in one 64-bit word,
+// no counters or fences (128 us: twice the bytes to read); two inputs' halves
+// per thread with ten points each in FP32 (same time).
 //
 // Arithmetic per thread: 5 points x 2 output channels, the 5 + k - 1 input
 // values of one (channel, tap row) read once into registers (every lane of
@@ -70,13 +78,6 @@ __device__ __forceinline__ int atom_acq_rel_add(int *p, int v) {
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
     return old;
 }
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_u32(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
 // Polls one counter until it reaches `want`: spins, then sleeps between
 // polls; gives up after `limit` polls or as soon as another CTA has
 // reported an error.  Returns false on either.
@@ -98,11 +99,16 @@ __device__ __forceinline__ bool wait_rows(const int *cnt, int lo, int hi, int wa
     return !__syncthreads_or(bad || !alive);
 }
 
-// The weight slice of split s of layer L into shared memory (cp.async, 16 B
-// per copy; slices are padded to 4 floats so every copy is aligned).
-__device__ __forceinline__ void copy_slice(const LatConv &L, int s, float *dst) {
+// The weight slice of split s of layer L into shared memory: one bulk copy by
+// one thread, completing on `bar` (copied by all threads 16 bytes at a time,
+// its issue was 1 to 1.7k cycles of every layer's critical path).
+__device__ __forceinline__ void copy_slice(const LatConv &L, int s, float *dst, uint64_t *bar) {
     const float *src = static_cast<const float *>(L.w) + (size_t)s * L.slice;
-    for (int i = threadIdx.x * 4; i < L.slice; i += kLT * 4) cp_async16(dst + i, src + i);
+    ptx::mbar_arrive_expect_tx(bar, (uint32_t)L.slice * 4u);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     ptx::smem_u32(dst)),
+                 "l"(src), "r"(L.slice * 4), "r"(ptx::smem_u32(bar))
+                 : "memory");
 }
 
 // Partial sums of one unit: acc[j][h] for point 5 pg + j and channel
@@ -194,7 +200,8 @@ __global__ void __launch_bounds__(kLT, 1) lat_kernel(const LatParams p) {
     float *in_s = sm + 2 * kLatSliceMax;                      // [cg][K][kPitch] FP32, or in16 [K][nx][16]
     uint16_t *in16 = reinterpret_cast<uint16_t *>(in_s);
     float *fin = in_s + kLatMaxCg * 5 * kPitch;                // finish stage: 361 head outputs + 8 x 32 sums
-    __shared__ int s_last;
+    __shared__ uint64_t w_bar[2];                              // weights of even / odd layers
+    __shared__ int s_last, s_bad;
     __shared__ float red[32];
 
     const int tid = threadIdx.x, G = gridDim.x, cta = blockIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -207,17 +214,26 @@ __global__ void __launch_bounds__(kLT, 1) lat_kernel(const LatParams p) {
         alive = false;
     };
 
-    copy_slice(p.L[0], s, wbuf0);
-    cp_async_commit();
+    if (tid == 0) {
+        s_bad = 0;
+        ptx::mbar_init(&w_bar[0], 1);
+        ptx::mbar_init(&w_bar[1], 1);
+        ptx::fence_mbar_init();
+        ptx::fence_proxy_async();
+        copy_slice(p.L[0], s, wbuf0, &w_bar[0]);
+    }
+    __syncthreads();
+    int w_issued = 0, w_have = -1;  // layers whose weights were asked for, waited for
     for (int l = 0; l < p.nl; ++l) {
         const LatConv &L = p.L[l];
         const bool mma = MODE != 0 && L.mma;
         float *w_s = (l & 1) ? wbuf1 : wbuf0;
-        __syncthreads();  // the other buffer's last reader (layer l - 1) is done
-        if (l + 1 < p.nl) copy_slice(p.L[l + 1], s, (l & 1) ? wbuf0 : wbuf1);
-        cp_async_commit();
-        cp_async_wait1();
-        __syncthreads();
+        // (the other buffer's last reads, layer l - 1's, were before the
+        // barrier at the end of its last unit)
+        if (alive && l + 1 < p.nl) {
+            if (tid == kLT - 32) copy_slice(p.L[l + 1], s, (l & 1) ? wbuf0 : wbuf1, &w_bar[(l + 1) & 1]);
+            w_issued = l + 1;
+        }
         const int r = L.k / 2;
         const int rp = l > 0 ? p.L[l - 1].k / 2 : 0;
         const int rw = max(r, rp);                             // rows to wait for
@@ -226,6 +242,23 @@ __global__ void __launch_bounds__(kLT, 1) lat_kernel(const LatParams p) {
         // staged columns: x = -r .. 19 + r (FFMA: 20 points), or .. 23 + r
         // (MMA: three 8-point column tiles)
         const int nx = (mma ? 24 : kRowPts) + 2 * r;
+        // This thread's staged item of every row (l > 0): 8 channels (4 when
+        // cg is not a multiple of 8) of one point; a layer has at most 4 x 3 x
+        // 22 of them, fewer than threads by the channel groups.  Its bias and
+        // scale are read here, while the rows it waits for are on their way.
+        const int c0 = s * L.cg, cw = (L.cg % 8 == 0) ? 8 : 4, n_items = (L.cg / cw) * L.k * nx;
+        const int ci = tid / (L.k * nx), idy = (tid - ci * (L.k * nx)) / nx, ixx = tid - ci * (L.k * nx) - idy * nx;
+        const int ich = c0 + cw * ci;
+        float ib[8], is[8];
+        if (l > 0 && tid < n_items) {
+            const LatConv &P = p.L[l - 1];
+#pragma unroll
+            for (int e = 0; e < 8; e += 4) {
+                if (e >= cw) break;
+                *reinterpret_cast<float4 *>(ib + e) = __ldg(reinterpret_cast<const float4 *>(P.bias + ich + e));
+                if (P.scale) *reinterpret_cast<float4 *>(is + e) = __ldg(reinterpret_cast<const float4 *>(P.scale + ich + e));
+            }
+        }
         for (int row = cta / kLatSplits; row < rows; row += rstep) {
             const int b = row / kBoard, y = row % kBoard;
             // (test hook: the stalled row of layer 1 waits for a count no
@@ -238,7 +271,6 @@ __global__ void __launch_bounds__(kLT, 1) lat_kernel(const LatParams p) {
             }
             if (!alive) continue;
             // ---- stage the input rows y - r .. y + r of this split's channels
-            const int c0 = s * L.cg;
             if (l == 0) {
                 const int n = L.cg * L.k * nx;
                 for (int i = tid; i < n; i += kLT) {
@@ -249,64 +281,64 @@ __global__ void __launch_bounds__(kLT, 1) lat_kernel(const LatParams p) {
                         v = (float)p.planes[((size_t)b * p.c_in + c0 + c) * kPoints + yy * kBoard + x];
                     in_s[(c * L.k + dy) * kPitch + xx] = v;
                 }
-            } else {
-                // 8 channels per item (4 when cg is not a multiple of 8): sum
-                // of the 8 partials, scale, bias, act; every load of an item
-                // is issued before the first add, and at most two items a
-                // thread for a 3x3 layer (one round trip each)
-                const LatConv &P = p.L[l - 1];
-                const int cw = (L.cg % 8 == 0) ? 8 : 4, nc = L.cg / cw, n = nc * L.k * nx;
-                for (int i = tid; i < n; i += kLT) {
-                    const int ci = i / (L.k * nx), rem = i - ci * (L.k * nx), dy = rem / nx, xx = rem - dy * nx;
-                    const int yy = y + dy - r, x = xx - r;
-                    float v[8];
+            } else if (tid < n_items) {
+                // the sum of the 8 partials, scale, bias, act; every load is
+                // issued before the first add (one round trip)
+                const int yy = y + idy - r, x = ixx - r;
+                float v[8];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = 0.0f;
-                    const int ch = c0 + cw * ci;
-                    if (yy >= 0 && yy < kBoard && x >= 0 && x < kBoard) {
-                        const float *q = src + ((size_t)(b * kBoard + yy) * kRowPts + x) * 128 + ch;
-                        float4 t[kLatSplits][2];
+                for (int e = 0; e < 8; ++e) v[e] = 0.0f;
+                if (yy >= 0 && yy < kBoard && x >= 0 && x < kBoard) {
+                    const float *q = src + ((size_t)(b * kBoard + yy) * kRowPts + x) * 128 + ich;
+                    float4 t[kLatSplits][2];
 #pragma unroll
-                        for (int ss = 0; ss < kLatSplits; ++ss) {
-                            const float4 *qq = reinterpret_cast<const float4 *>(q + (size_t)ss * kLatMaxRows * kRowPts * 128);
-                            t[ss][0] = __ldcg(qq);
-                            t[ss][1] = cw == 8 ? __ldcg(qq + 1) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        }
-#pragma unroll
-                        for (int ss = 0; ss < kLatSplits; ++ss) {
-                            v[0] += t[ss][0].x;
-                            v[1] += t[ss][0].y;
-                            v[2] += t[ss][0].z;
-                            v[3] += t[ss][0].w;
-                            v[4] += t[ss][1].x;
-                            v[5] += t[ss][1].y;
-                            v[6] += t[ss][1].z;
-                            v[7] += t[ss][1].w;
-                        }
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            if (e >= cw) break;
-                            const float bb = __ldg(P.bias + ch + e);
-                            v[e] = lat_act(P.scale ? fmaf(v[e], __ldg(P.scale + ch + e), bb) : v[e] + bb, p.act);
-                        }
+                    for (int ss = 0; ss < kLatSplits; ++ss) {
+                        const float4 *qq = reinterpret_cast<const float4 *>(q + (size_t)ss * kLatMaxRows * kRowPts * 128);
+                        t[ss][0] = __ldcg(qq);
+                        t[ss][1] = cw == 8 ? __ldcg(qq + 1) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
-                    if (mma) {
-                        // cw == 8 (cg = 16): one 16-byte store of 8 channels
-                        uint4 h;
-                        h.x = (uint32_t)to16(v[0], F16) | ((uint32_t)to16(v[1], F16) << 16);
-                        h.y = (uint32_t)to16(v[2], F16) | ((uint32_t)to16(v[3], F16) << 16);
-                        h.z = (uint32_t)to16(v[4], F16) | ((uint32_t)to16(v[5], F16) << 16);
-                        h.w = (uint32_t)to16(v[6], F16) | ((uint32_t)to16(v[7], F16) << 16);
-                        *reinterpret_cast<uint4 *>(in16 + (dy * nx + xx) * 16 + 8 * ci) = h;
-                    } else {
-                        float *d = in_s + ((cw * ci) * L.k + dy) * kPitch + xx;
 #pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (e < cw) d[e * L.k * kPitch] = v[e];
+                    for (int ss = 0; ss < kLatSplits; ++ss) {
+                        v[0] += t[ss][0].x;
+                        v[1] += t[ss][0].y;
+                        v[2] += t[ss][0].z;
+                        v[3] += t[ss][0].w;
+                        v[4] += t[ss][1].x;
+                        v[5] += t[ss][1].y;
+                        v[6] += t[ss][1].z;
+                        v[7] += t[ss][1].w;
+                    }
+                    const bool scaled = p.L[l - 1].scale != nullptr;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        if (e >= cw) break;
+                        v[e] = lat_act(scaled ? fmaf(v[e], is[e], ib[e]) : v[e] + ib[e], p.act);
                     }
                 }
+                if (mma) {
+                    // cw == 8 (cg = 16): one 16-byte store of 8 channels
+                    uint4 h;
+                    h.x = (uint32_t)to16(v[0], F16) | ((uint32_t)to16(v[1], F16) << 16);
+                    h.y = (uint32_t)to16(v[2], F16) | ((uint32_t)to16(v[3], F16) << 16);
+                    h.z = (uint32_t)to16(v[4], F16) | ((uint32_t)to16(v[5], F16) << 16);
+                    h.w = (uint32_t)to16(v[6], F16) | ((uint32_t)to16(v[7], F16) << 16);
+                    *reinterpret_cast<uint4 *>(in16 + (idy * nx + ixx) * 16 + 8 * ci) = h;
+                } else {
+                    float *d = in_s + ((cw * ci) * L.k + idy) * kPitch + ixx;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (e < cw) d[e * L.k * kPitch] = v[e];
+                }
+            }
+            if (w_have < l) {
+                w_have = l;
+                if (!ptx::mbar_wait(&w_bar[l & 1], (uint32_t)(l >> 1) & 1, p.poll_limit)) s_bad = 1;
             }
             __syncthreads();
+            if (s_bad) {
+                fail(93);
+                continue;
+            }
             // ---- partial sums of this unit
             float *o_row = dst + ((size_t)s * kLatMaxRows + row) * kRowPts * 128;
             if (mma) {
@@ -346,13 +378,15 @@ __global__ void __launch_bounds__(kLT, 1) lat_kernel(const LatParams p) {
                         *reinterpret_cast<float2 *>(o + x * 128) = make_float2(acc[j][0], acc[j][1]);
                 }
             }
-            // publish: the barrier orders every thread's stores before thread
-            // 0's release add
+            // publish: the barrier orders every thread's stores before the
+            // release add (by a thread of a warp that polls nothing, so that
+            // the polls of the next rows do not start behind its fence)
             __syncthreads();
-            if (tid == 0) red_release_add(p.cnt + l * kLatMaxRows + row, 1);
+            if (tid == kLT - 64) red_release_add(p.cnt + l * kLatMaxRows + row, 1);
         }
     }
-    cp_async_wait0();
+    // (after a wait that ran out: no copy outlives the CTA)
+    for (int l = w_have + 1; l <= w_issued; ++l) ptx::mbar_wait(&w_bar[l & 1], (uint32_t)(l >> 1) & 1, 1u << 20);
 
     // ---- finish: softmax (one unit per board) or the value head (8 units
     // per board: a slice of the FC1 units each; the last to finish adds the
