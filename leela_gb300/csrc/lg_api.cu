@@ -2336,7 +2336,7 @@ extern "C" int lg_policy_avg8_device(lg_ctx *c, const uint8_t *planes, int B, fl
     launch_rotate8(planes, B, n.d.c_in, c->d_planes, s);
     int nl = 0;
     rc = forward(c, LG_NET_POLICY, c->d_planes, 8 * B, temperature, c->d_probs, nullptr, nullptr, s, &nl,
-                 c->profiling);
+                 c->profiling, false, nullptr, nullptr, true);
     if (rc) return rc;
     launch_unrotate_avg8(c->d_probs, B, probs, s);
     c->launches += nl + 2;
@@ -2366,7 +2366,8 @@ extern "C" int lg_value_avg8_device(lg_ctx *c, const uint8_t *planes, int B, flo
     cudaStream_t s = (cudaStream_t)stream;
     launch_rotate8(planes, B, n.d.c_in, c->d_planes, s);
     int nl = 0;
-    rc = forward(c, LG_NET_VALUE, c->d_planes, 8 * B, 1.0f, nullptr, nullptr, c->d_value, s, &nl, c->profiling);
+    rc = forward(c, LG_NET_VALUE, c->d_planes, 8 * B, 1.0f, nullptr, nullptr, c->d_value, s, &nl, c->profiling, false,
+                 nullptr, nullptr, true);
     if (rc) return rc;
     launch_avg8(c->d_value, B, value, s);
     c->launches += nl + 2;
