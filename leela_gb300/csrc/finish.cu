@@ -20,6 +20,7 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <utility>
 
@@ -593,6 +594,19 @@ __global__ void __launch_bounds__(kSoftmaxThreads, 5)
     if (b < head_boards(h, B)) softmax_board(h, b, temperature, probs, entropy, sm.red);
 }
 
+// Results of a small host call straight into pinned host memory: up to two
+// arrays of n floats and the error word.
+__global__ void __launch_bounds__(256) export_kernel(const float *__restrict__ a, float *__restrict__ ha,
+                                                     const float *__restrict__ b, float *__restrict__ hb, int n,
+                                                     const int *__restrict__ err, int *__restrict__ herr) {
+    ptx::grid_dep_wait();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        ha[i] = a[i];
+        if (b) hb[i] = b[i];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *herr = *err;
+}
+
 // ------------------------------------------------------------ host launchers
 
 namespace {
@@ -692,6 +706,11 @@ size_t value_fc_counter_ints(int B, int H) {
 }
 
 int value_fc_slice_units() { return kFcUnits; }
+
+void launch_export(const float *a, float *ha, const float *b, float *hb, int n, const int *err, int *herr,
+                   cudaStream_t s) {
+    launch_ex(export_kernel, std::max(1, std::min(64, (n + 255) / 256)), 256, s, true, a, ha, b, hb, n, err, herr);
+}
 
 void launch_pack_planes_l5(const uint8_t *planes, int B, int C, int halves, bool f16, __nv_bfloat16 *out,
                            cudaStream_t s, const int *count, int count_base, bool pdl) {

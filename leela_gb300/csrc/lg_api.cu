@@ -159,6 +159,7 @@ struct lg_ctx {
     uint8_t *h_planes = nullptr, *h_planes_b = nullptr;
     float *h_out = nullptr, *h_out2 = nullptr, *h_out_b = nullptr, *h_out2_b = nullptr;
     cudaEvent_t host_done[2] = {nullptr, nullptr};
+    int *h_err = nullptr;  // pinned: the error word as of each slot's results (blocking calls, then the server's)
     // board calls over several chunks of a tensor-core net (allocated on the
     // first such call): a ring of kPipe slots, each holding one super-chunk's
     // boards (pinned, device), input planes (device) and results (device,
@@ -1135,6 +1136,21 @@ int run_host_boards_pipe(lg_ctx *c, int net, int B, float T, float *probs, float
     return rc;
 }
 
+// A chunk's results and the error word into pinned memory (captured into its
+// graph).  Up to 32 KB an array by one kernel: a copy per array and a
+// synchronous one for the error word after the chunk were 16 us of a
+// one-position call (109 -> 93 us; the copy in, by a kernel as well, gave
+// less than 1 us).
+void results_out(lg_ctx *c, const float *a, float *ha, const float *b, float *hb, int n, int *herr) {
+    if (n <= 8192) {
+        launch_export(a, ha, b, hb, n, c->d_err, herr, c->stream);
+        return;
+    }
+    cudaMemcpyAsync(ha, a, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    if (b) cudaMemcpyAsync(hb, b, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+}
+
 // Host call: chunks of up to max_batch positions go through a cached CUDA
 // graph of copy-in + forward + copy-out (one graph per chunk size and
 // staging slot).  Two pinned slots alternate, so the host packs chunk k+1
@@ -1190,8 +1206,7 @@ int run_host(lg_ctx *c, int net, const uint8_t *planes, int B, float T, float *p
         if (!q.live) return LG_OK;
         q.live = false;
         LG_CUDA_TRY(cudaEventSynchronize(c->host_done[slot]));
-        int herr = 0;
-        LG_CUDA_TRY(cudaMemcpy(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+        const int herr = c->h_err[slot];
         if (herr) {
             cudaMemset(c->d_err, 0, sizeof(int));
             lg_set_error("kernel reported error status %d", herr);
@@ -1255,16 +1270,8 @@ int run_host(lg_ctx *c, int net, const uint8_t *planes, int B, float T, float *p
                 rc = forward(c, net, c->d_planes, nb, T, c->d_probs, want_logits ? c->d_logits : nullptr,
                              c->d_value, c->stream, &nf, false, l5_direct);
             nl += nf;
-            if (n.d.value_head) {
-                cudaMemcpyAsync(ho[slot], c->d_value, (size_t)nb * sizeof(float), cudaMemcpyDeviceToHost,
-                                c->stream);
-            } else {
-                cudaMemcpyAsync(ho[slot], c->d_probs, (size_t)nb * kPoints * sizeof(float),
-                                cudaMemcpyDeviceToHost, c->stream);
-                if (want_logits)
-                    cudaMemcpyAsync(hl[slot], c->d_logits, (size_t)nb * kPoints * sizeof(float),
-                                    cudaMemcpyDeviceToHost, c->stream);
-            }
+            results_out(c, n.d.value_head ? c->d_value : c->d_probs, ho[slot], want_logits ? c->d_logits : nullptr,
+                        hl[slot], n.d.value_head ? nb : nb * kPoints, &c->h_err[slot]);
             if (direct) {
                 if (rc) {
                     finish(slot ^ 1);
@@ -1393,12 +1400,8 @@ int server_launch(lg_ctx *c, int slot, int net, int nb, float T) {
         int nl = 0;
         int rc = forward(c, logits ? LG_NET_POLICY : net, c->d_planes, nb, T, c->d_probs,
                          logits ? c->d_logits : nullptr, c->d_value, c->stream, &nl);
-        if (n.d.value_head)
-            cudaMemcpyAsync(c->srv_out[slot], c->d_value, (size_t)nb * sizeof(float), cudaMemcpyDeviceToHost,
-                            c->stream);
-        else
-            cudaMemcpyAsync(c->srv_out[slot], logits ? c->d_logits : c->d_probs, (size_t)nb * kPoints * sizeof(float),
-                            cudaMemcpyDeviceToHost, c->stream);
+        results_out(c, n.d.value_head ? c->d_value : (logits ? c->d_logits : c->d_probs), c->srv_out[slot], nullptr,
+                    nullptr, n.d.value_head ? nb : nb * kPoints, &c->h_err[2 + slot]);
         cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
         if (rc) {
             if (ce == cudaSuccess) cudaGraphDestroy(g);
@@ -1419,8 +1422,7 @@ int server_launch(lg_ctx *c, int slot, int net, int nb, float T) {
 
 int server_finish(lg_ctx *c, int slot) {
     LG_CUDA_TRY(cudaEventSynchronize(c->srv_done[slot]));
-    int herr = 0;
-    LG_CUDA_TRY(cudaMemcpy(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+    const int herr = c->h_err[2 + slot];
     if (herr) {
         cudaMemset(c->d_err, 0, sizeof(int));
         lg_set_error("kernel reported error status %d", herr);
@@ -1563,6 +1565,7 @@ extern "C" void lg_destroy(lg_ctx *c) {
     if (c->h_planes_b) cudaFreeHost(c->h_planes_b);
     if (c->h_out_b) cudaFreeHost(c->h_out_b);
     if (c->h_out2_b) cudaFreeHost(c->h_out2_b);
+    if (c->h_err) cudaFreeHost(c->h_err);
     for (int i = 0; i < 2; ++i)
         if (c->host_done[i]) cudaEventDestroy(c->host_done[i]);
     if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
@@ -1712,6 +1715,7 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
         cudaMallocHost(&c->h_planes_b, mb * max_c_in * kPoints) != cudaSuccess ||
         cudaMallocHost(&c->h_out_b, mb * kPoints * sizeof(float)) != cudaSuccess ||
         cudaMallocHost(&c->h_out2_b, mb * kPoints * sizeof(float)) != cudaSuccess ||
+        cudaMallocHost(&c->h_err, 4 * sizeof(int)) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->host_done[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->host_done[1], cudaEventDisableTiming) != cudaSuccess) {
         lg_set_error("cudaMallocHost failed");
