@@ -119,15 +119,17 @@ __global__ void st_softmax(const float *__restrict__ logits, int B, float *__res
 //   dlogits = (softmax - target) / B
 //   du = 2 vw (v - vt)(1 - v^2) / B;  dpre[h] = du W2[h] [hid > 0];  dx361 = W1^T dpre
 // Writes dlogits[B][361], du[B], dpre[B][H], dx361[B][361]; adds the batch
-// losses into loss[0] (KL) and loss[1] (value MSE, before vw).
+// losses into loss[0] (KL) and loss[1] (value MSE, before vw), the head convs'
+// bias gradients sum_p dlogits and sum_p dx361 into dbp and dbv.
 __global__ void __launch_bounds__(384) st_loss_bwd(const float *__restrict__ logits, const float *__restrict__ target,
                             const float *__restrict__ v, const float *__restrict__ vt,
                             const float *__restrict__ hid, const float *__restrict__ W1,
                             const float *__restrict__ W2, int B, int H, float vw,
                             float *__restrict__ dlogits, float *__restrict__ du_out,
                             float *__restrict__ dpre, float *__restrict__ dx361,
-                            float *__restrict__ loss) {
+                            float *__restrict__ dbp, float *__restrict__ dbv, float *__restrict__ loss) {
     __shared__ float red[32];
+    __shared__ double red64[12], inv_s;
     __shared__ float s_dpre[512];
     const int b = blockIdx.x, p = threadIdx.x;
     const float invB = 1.0f / (float)B;
@@ -141,21 +143,36 @@ __global__ void __launch_bounds__(384) st_loss_bwd(const float *__restrict__ log
     for (int w = 1; w < 12; ++w) m = fmaxf(m, red[w]);
     __syncthreads();
     const float e = p < kPoints ? expf(x - m) : 0.0f;
-    float s = e;
+    // over the CTA, the same value in every thread of warp 0
+    auto sum = [&](double x) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (p % 32 == 0) red[p / 32] = s;
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        __syncthreads();
+        if (p % 32 == 0) red64[p / 32] = x;
+        __syncthreads();
+        x = p % 32 < 12 && p < 32 ? red64[p] : 0.0;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    };
+    const double s64 = sum(e);
+    if (p == 0) {
+        inv_s = 1.0 / s64;
+        red[31] = (float)s64;
+    }
     __syncthreads();
-    s = 0.0f;
-    for (int w = 0; w < 12; ++w) s += red[w];
-    __syncthreads();
-    float kl = 0.0f;
+    float kl = 0.0f, dl = 0.0f;
     if (p < kPoints) {
         const float t = target[(size_t)b * kPoints + p];
-        const float logq = (x - m) - logf(s);
-        dlogits[(size_t)b * kPoints + p] = (e / s - t) * invB;
+        const float logq = (x - m) - logf(red[31]);
+        dl = ((float)(e * inv_s) - t) * invB;
+        dlogits[(size_t)b * kPoints + p] = dl;
         if (t > 0.0f) kl = t * (logf(t) - logq);
     }
+    // a board's sum of p - t is rounding alone where both sum to 1, so neither
+    // the softmax's sum nor this one may add rounding of its own
+    const double dl_sum = sum(dl);
+    if (p == 0) atomicAdd(dbp, (float)dl_sum);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) kl += __shfl_xor_sync(0xffffffffu, kl, o);
     if (p % 32 == 0) red[p / 32] = kl;
@@ -178,11 +195,13 @@ __global__ void __launch_bounds__(384) st_loss_bwd(const float *__restrict__ log
         dpre[(size_t)b * H + h] = g;
     }
     __syncthreads();
+    float dx = 0.0f;
     if (p < kPoints) {
-        float acc = 0.0f;
-        for (int h = 0; h < H; ++h) acc = fmaf(s_dpre[h], W1[(size_t)h * kPoints + p], acc);
-        dx361[(size_t)b * kPoints + p] = acc;
+        for (int h = 0; h < H; ++h) dx = fmaf(s_dpre[h], W1[(size_t)h * kPoints + p], dx);
+        dx361[(size_t)b * kPoints + p] = dx;
     }
+    const double dx_sum = sum(dx);
+    if (p == 0) atomicAdd(dbv, (float)dx_sum);
 }
 
 // Value FC weight gradients, reduced over the batch (a CTA per hidden unit and
@@ -225,36 +244,28 @@ __global__ void __launch_bounds__(384) st_fc_wgrad(const float *__restrict__ dpr
 }
 
 // Head backward into the trunk: dX[m][c] = dlogits[m] wp[c] + dx361[m] wv[c];
-// head weight gradients dwp[c] = sum_m dlogits[m] X[m][c] (dwv alike),
-// dbp = sum_m dlogits[m], dbv = sum_m dx361[m].  C <= 128.
+// head weight gradients dwp[c] = sum_m dlogits[m] X[m][c] (dwv alike).  C <= 128.
 __global__ void __launch_bounds__(256) st_heads_bwd(const float *__restrict__ X, const float *__restrict__ dlogits,
                              const float *__restrict__ dx361, const float *__restrict__ wp,
                              const float *__restrict__ wv, int M, int C, float *__restrict__ dX,
-                             float *__restrict__ dwp, float *__restrict__ dbp,
-                             float *__restrict__ dwv, float *__restrict__ dbv) {
-    __shared__ float swp[128], swv[128], sdp[256][2];
+                             float *__restrict__ dwp, float *__restrict__ dwv) {
+    __shared__ float swp[128], swv[128];
     const int tid = threadIdx.x;
     // Each thread owns channel c = tid % C of rows m = row0 + tid / C + k*(256/C).
     const int per = 256 / C;
     const int c = tid % C, r = tid / C;
-    float gp = 0.0f, gv = 0.0f, bpp = 0.0f, bvv = 0.0f;
+    float gp = 0.0f, gv = 0.0f;
     for (int m = blockIdx.x * per + r; m < M && r < per; m += gridDim.x * per) {
         const float dl = dlogits[m], dx = dx361[m];
         const float x = X[(size_t)m * C + c];
         dX[(size_t)m * C + c] = dl * wp[c] + dx * wv[c];
         gp = fmaf(dl, x, gp);
         gv = fmaf(dx, x, gv);
-        if (c == 0) {
-            bpp += dl;
-            bvv += dx;
-        }
     }
     if (tid < C) {
         swp[tid] = 0.0f;
         swv[tid] = 0.0f;
     }
-    sdp[tid][0] = bpp;
-    sdp[tid][1] = bvv;
     __syncthreads();
     if (r < per) {
         atomicAdd(&swp[c], gp);
@@ -264,15 +275,6 @@ __global__ void __launch_bounds__(256) st_heads_bwd(const float *__restrict__ X,
     if (tid < C) {
         atomicAdd(&dwp[tid], swp[tid]);
         atomicAdd(&dwv[tid], swv[tid]);
-    }
-    if (tid == 0) {
-        float a = 0.0f, b = 0.0f;
-        for (int i = 0; i < 256; ++i) {
-            a += sdp[i][0];
-            b += sdp[i][1];
-        }
-        atomicAdd(dbp, a);
-        atomicAdd(dbv, b);
     }
 }
 
@@ -492,13 +494,13 @@ int st_backward(lg_student *s, int B, const float *target, const float *vt, floa
     cudaMemsetAsync(s->grads, 0, s->nparam * sizeof(float), st);
     cudaMemsetAsync(s->loss, 0, 2 * sizeof(float), st);
     st_loss_bwd<<<B, 384, 0, st>>>(s->logits, target, s->vout, vt, s->hid, P(s, s->W1), P(s, s->W2), B, s->H,
-                                   vw, s->dlogits, s->du, s->dpre, s->dx361, s->loss);
+                                   vw, s->dlogits, s->du, s->dpre, s->dx361, G(s, s->bp), G(s, s->bv), s->loss);
     st_fc_wgrad<<<dim3(s->H, (B + kFcShare - 1) / kFcShare), 384, 0, st>>>(s->dpre, s->du, s->x361, s->hid, B, s->H, G(s, s->W1), G(s, s->b1),
                                       G(s, s->W2), G(s, s->b2));
     const float *Xlast = s->Y.back();
     int hblocks = std::min(1024, (M + (256 / s->width) - 1) / (256 / s->width));
     st_heads_bwd<<<hblocks, 256, 0, st>>>(Xlast, s->dlogits, s->dx361, P(s, s->wp), P(s, s->wv), M, s->width,
-                                          s->dA, G(s, s->wp), G(s, s->bp), G(s, s->wv), G(s, s->bv));
+                                          s->dA, G(s, s->wp), G(s, s->wv));
     if (s->tc) return st_backward_tc(s, B, st);
     float *dY = s->dA, *dX = s->dB;
     for (int l = (int)s->convs.size() - 1; l >= 0; --l) {
