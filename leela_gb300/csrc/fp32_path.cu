@@ -304,31 +304,37 @@ __global__ void __launch_bounds__(256, 2) conv_f32_big_kernel(const float *__res
     }
 }
 
-// Layers of 64k output channels over enough rows: 192 x 64 tiles, 12 x 8
-// outputs a thread (five float4 loads of the operands per 96 FMAs), K steps of
-// one tap and 8 input channels double-buffered.  What bounds tiles with fewer
-// outputs a thread is shared memory: a float4 load is four wavefronts a warp
-// whatever its lanes share (packed fma.rn.f32x2 on 8 x 8 outputs, one operand
-// stored twice, was slower than the 64 x 64 kernel).  Every output is still
-// one FMA chain over (tap, channel) in order, as in the other two kernels: the
-// same bits.
+// Layers of 64k output channels over enough rows: 256 x 64 tiles, 16 x 8
+// outputs a thread as pairs of rows (fma.rn.f32x2; six float4 loads of the
+// operands per 64 of them), K steps of one tap and 8 input channels brought in
+// by cp.async, double-buffered.  What bounds tiles with fewer outputs a thread
+// is shared memory: a float4 load is four wavefronts a warp whatever its lanes
+// share (8 x 8 outputs with one operand stored twice were slower than the
+// 64 x 64 kernel).  Every output is still one FMA chain over (tap, channel) in
+// order, as in the other two kernels: the same bits.
 //
-// Three CTAs an SM, each over an even share of the 64-row blocks in tiles of
-// three, the rest in one of two or one.  A 3x3 layer 64 -> 64 over 512 boards:
-// 440 us on the 64 x 64 kernel, 378 with one 256-row tile a CTA (2.4 waves
-// taking 3), 312 with shares of 16 x 8 outputs and two CTAs an SM, 296 so (46
-// TFLOP/s of a 70 TFLOP/s peak).
-constexpr int BM3 = 192, BN3 = 64, BKC3 = 8, kN64Threads = 128, kN64Ctas = 3;
+// Two CTAs an SM, each over an even share of the 64-row blocks in tiles of
+// four, the rest in one of three, two or one.  A 3x3 layer 64 -> 64 over 512
+// boards: 440 us on the 64 x 64 kernel; with single FMAs 378 with one 256-row
+// tile a CTA (2.4 waves taking 3), 312 with these shares, 296 with 12 x 8
+// outputs and three CTAs an SM (issue slots 77% busy); with pairs 278 so (49
+// TFLOP/s of a 70 TFLOP/s peak, the FMA pipe 69% busy where an SM has work).
+// Inputs through registers cost 10 us more, 12 x 8 pairs in three CTAs spill,
+// three stages or a loader spread over the step's channels were slower.
+constexpr int kN64Rows = 4, BM3 = 64 * kN64Rows, BN3 = 64, BKC3 = 8, kN64Threads = 128, kN64Ctas = 2;
 
 struct N64Smem {
     float A[2][BKC3][BM3 + 4];
     float B[2][BKC3][BN3 + 4];
+    uint32_t inside[BM3];
 };
 
-__device__ __forceinline__ float4 ldg_nc4(const float *p) {
-    float4 v;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
+// A float (16 bytes) from global to shared memory, or zeros.
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float *src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float *src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
 // One tile of 64 R rows from row m0.
@@ -338,80 +344,79 @@ __device__ __forceinline__ void n64_tile(const float *__restrict__ in, const flo
                                          int act, int m0, int n0, N64Smem &sm) {
     const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
     constexpr int PAD = KS / 2;
-    // A loader: rows ar + 64 i, channels ac .. ac+3; a bit per tap inside the board
-    const int ar = tid / 2, ac = (tid % 2) * 4;
-    uint32_t inside[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const int m = m0 + ar + 64 * i, p = m % kPoints, y = p / kBoard, x = p - y * kBoard;
+    // a bit per tap inside the board for each row of the tile
+    __syncthreads();
+    for (int r = tid; r < 64 * R; r += kN64Threads) {
+        const int m = m0 + r, p = m % kPoints, y = p / kBoard, x = p - y * kBoard;
         uint32_t bits = 0;
         for (int t = 0; t < KS * KS; ++t) {
             const int sy = y + t / KS - PAD, sx = x + t % KS - PAD;
             if (m < M && sy >= 0 && sy < kBoard && sx >= 0 && sx < kBoard) bits |= 1u << t;
         }
-        inside[i] = bits;
+        sm.inside[r] = bits;
     }
-    const float *src = in + (size_t)(m0 + ar) * C + ac;
-    // B loader: channel bk, columns bn .. bn+3
+    __syncthreads();
+    // A loader: rows ar + 16 i, channel ac; B loader: channel bk, columns bn .. bn+3
+    const int ar = tid / 8, ac = tid % 8;
     const int bk = tid / 16, bn = (tid % 16) * 4;
-    const float *wsrc = wt + (size_t)bk * O + n0 + bn;
     const int cchunks = (C + BKC3 - 1) / BKC3, ksteps = KS * KS * cchunks;
-    float4 va[R], vb;
     int tap = 0, c0 = 0;  // of the step to load
-    auto load = [&]() {
-        const float *s = src + ((tap / KS - PAD) * kBoard + tap % KS - PAD) * C + c0;
+    uint32_t rows = 0;    // a bit per row of the loader inside the board at this tap
+    auto load = [&](int buf) {
+        if (c0 == 0) {
+            rows = 0;
 #pragma unroll
-        for (int i = 0; i < R; ++i) {
-            va[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if ((inside[i] >> tap & 1) && c0 + ac < C) va[i] = ldg_nc4(s + (size_t)(64 * i) * C);
+            for (int i = 0; i < 4 * R; ++i) rows |= (sm.inside[ar + 16 * i] >> tap & 1) << i;
         }
-        vb = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c0 + bk < C) vb = ldg_nc4(wsrc + ((size_t)tap * C + c0) * O);
+        const float *s = in + (ptrdiff_t)(m0 + ar + (tap / KS - PAD) * kBoard + tap % KS - PAD) * C + c0 + ac;
+        const uint32_t ok = c0 + ac < C ? rows : 0u, da = ptx::smem_u32(&sm.A[buf][ac][ar]);
+#pragma unroll
+        for (int i = 0; i < 4 * R; ++i) {
+            const bool in_i = ok >> i & 1;
+            cp_async4(da + 64 * i, in_i ? s : in, in_i);
+            s += 16 * C;
+        }
+        const bool bok = c0 + bk < C;
+        cp_async16(ptx::smem_u32(&sm.B[buf][bk][bn]), wt + (bok ? (size_t)(tap * C + c0 + bk) * O + n0 + bn : 0), bok);
+        asm volatile("cp.async.commit_group;" ::: "memory");
         c0 += BKC3;
         if (c0 >= C) {
             c0 = 0;
             ++tap;
         }
     };
-    auto store = [&](int buf) {
+    // rows ty*4 + 64 i + r, columns tx*4 + 32 h + j; two rows to an accumulator pair
+    float2 acc[2 * R][8];
 #pragma unroll
-        for (int i = 0; i < R; ++i) {
-            sm.A[buf][ac + 0][ar + 64 * i] = va[i].x;
-            sm.A[buf][ac + 1][ar + 64 * i] = va[i].y;
-            sm.A[buf][ac + 2][ar + 64 * i] = va[i].z;
-            sm.A[buf][ac + 3][ar + 64 * i] = va[i].w;
-        }
-        *reinterpret_cast<float4 *>(&sm.B[buf][bk][bn]) = vb;
-    };
-    // rows ty*4 + 64 i + r, columns tx*4 + 32 h + j
-    float acc[4 * R][8];
+    for (int i = 0; i < 2 * R; ++i)
 #pragma unroll
-    for (int i = 0; i < 4 * R; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-    load();
-    store(0);
-    __syncthreads();
+        for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+    load(0);
     for (int ks = 0; ks < ksteps; ++ks) {
         const int cur = ks & 1;
-        const bool more = ks + 1 < ksteps;
-        if (more) load();
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (ks + 1 < ksteps) load(cur ^ 1);
 #pragma unroll
         for (int kk = 0; kk < BKC3; ++kk) {
-            float a[4 * R], b[8];
+            float2 a[2 * R];
 #pragma unroll
-            for (int i = 0; i < R; ++i)
-                *reinterpret_cast<float4 *>(a + 4 * i) = *reinterpret_cast<const float4 *>(&sm.A[cur][kk][ty * 4 + 64 * i]);
+            for (int i = 0; i < R; ++i) {
+                const float4 v = *reinterpret_cast<const float4 *>(&sm.A[cur][kk][ty * 4 + 64 * i]);
+                a[2 * i] = make_float2(v.x, v.y);
+                a[2 * i + 1] = make_float2(v.z, v.w);
+            }
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *reinterpret_cast<float4 *>(b + 4 * h) = *reinterpret_cast<const float4 *>(&sm.B[cur][kk][tx * 4 + 32 * h]);
+            for (int h = 0; h < 2; ++h) {
+                const float4 v = *reinterpret_cast<const float4 *>(&sm.B[cur][kk][tx * 4 + 32 * h]);
+                const float b[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int i = 0; i < 4 * R; ++i)
+                for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                    for (int i = 0; i < 2 * R; ++i)
+                        acc[i][4 * h + j] = __ffma2_rn(a[i], make_float2(b[j], b[j]), acc[i][4 * h + j]);
+            }
         }
-        if (more) store(cur ^ 1);
-        __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < 4 * R; ++i) {
@@ -422,7 +427,7 @@ __device__ __forceinline__ void n64_tile(const float *__restrict__ in, const flo
             const int n = n0 + 32 * h + tx * 4;
             float v[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = act_fn(bias[n + j] + acc[i][4 * h + j], act);
+            for (int j = 0; j < 4; ++j) v[j] = act_fn(bias[n + j] + (i % 2 ? acc[i / 2][4 * h + j].y : acc[i / 2][4 * h + j].x), act);
             *reinterpret_cast<float4 *>(out + (size_t)m * O + n) = make_float4(v[0], v[1], v[2], v[3]);
         }
     }
@@ -438,8 +443,9 @@ __global__ void __launch_bounds__(kN64Threads, kN64Ctas) conv_f32_n64_kernel(con
     const int nblk = (M + 63) / 64, n0 = blockIdx.y * BN3;
     int b = (int)((long long)nblk * blockIdx.x / gridDim.x);
     const int e = (int)((long long)nblk * (blockIdx.x + 1) / gridDim.x);
-    for (; b + 2 < e; b += 3) n64_tile<KS, 3>(in, wt, bias, out, M, C, O, act, b * 64, n0, sm);
-    if (b + 1 < e) n64_tile<KS, 2>(in, wt, bias, out, M, C, O, act, b * 64, n0, sm);
+    for (; b + kN64Rows - 1 < e; b += kN64Rows) n64_tile<KS, kN64Rows>(in, wt, bias, out, M, C, O, act, b * 64, n0, sm);
+    if (b + 2 < e) n64_tile<KS, 3>(in, wt, bias, out, M, C, O, act, b * 64, n0, sm);
+    else if (b + 1 < e) n64_tile<KS, 2>(in, wt, bias, out, M, C, O, act, b * 64, n0, sm);
     else if (b < e) n64_tile<KS, 1>(in, wt, bias, out, M, C, O, act, b * 64, n0, sm);
 }
 
@@ -495,10 +501,12 @@ struct F32Plan {
     bool big;
     int bm, bn, bkc;
 };
-// The 12 x 8-output kernel where every CTA slot gets at least half a tile (the
-// 64 x 64 kernel would not split K there either) and float4 loads are aligned.
+// The 16 x 8-output kernel from the size on at which the 64 x 64 one would not
+// split K (304 of its tiles), so that sums keep their order, where loads are
+// aligned.  Training passes of 64-wide nets just above the line, 64 x 64 kernel
+// -> this one: 54 boards 1,147 -> 959 us, 107 boards 1,439 -> 1,165.
 bool f32_n64(const F32Plan &pl, int M, int C, int O) {
-    return !pl.big && O % BN3 == 0 && C % 4 == 0 && (long long)M * (O / BN3) >= 152 * 256;
+    return !pl.big && O % BN3 == 0 && C % 4 == 0 && (long long)((M + BM - 1) / BM) * (O / BN3) >= 2 * 152;
 }
 F32Plan f32_plan(int M, int O) {
     return (O % BN2 == 0 && M >= 152 * BM2) ? F32Plan{true, BM2, BN2, BKC2} : F32Plan{false, BM, BN, BKC};
