@@ -40,12 +40,13 @@
 //     kernels, which add the parts in a fixed order.
 //
 // A batch with an SM for every board runs one board a CTA (152 boards: 55 us
-// against 89 in pairs).  8,192 boards: 1.63 ms with four epilogue warps per
-// TMEM lane quarter and a warp-uniform MMA issuer, 1.85 with two and a
-// one-lane issuer: a pair of boards takes 111k cycles, 84k of them the MMAs'
-// own (N = 64: 48 cycles each, shared-memory reads), 6k the epilogue's stores
-// in the same shared memory, 11k waits for weight slices (a deeper ring does
-// not shorten them).
+// against 89 in pairs).  8,192 boards, with softmax and value head: 1.57 ms
+// with four epilogue warps per TMEM lane quarter, a warp-uniform MMA issuer and
+// each slice's wait before the last MMAs of the slice ahead of it; 1.62 with
+// the waits between the slices; 1.85 also with two epilogue warps and a
+// one-lane issuer.  Of ~107k cycles a pair of boards 84k are the MMAs' own (N
+// = 64: 48 cycles each, shared-memory reads), 6k the epilogue's stores in the
+// same shared memory (a deeper ring of slices gains nothing).
 //
 // Warps: 0 = TMA producer of the weight slices, 1 = TMEM owner and MMA
 // issuer, 2..17 = plane staging, epilogue (four warps per TMEM lane quarter,
@@ -127,11 +128,14 @@ __device__ __forceinline__ uint32_t relu_bf16x2(float lo, float hi) {
 // 16 bytes), B = the slice at b0; K steps of 16 channels = 32 bytes = 2
 // units.  The descriptors are a base plus compile-time offsets, so the
 // issuing thread spends an add per operand and MMA.  FIRST: the slice
-// starts every accumulator.
-template <bool FIRST>
+// starts every accumulator.  Tiles T0 .. T1 - 1: the issuer waits for the
+// next slice before the last tile of the one ahead of it, so that the tensor
+// pipe does not run dry meanwhile (8,192 positions: waits between the slices
+// 1,620 us, before the last tile 1,568, before the last two 1,575).
+template <int T0, int T1, bool FIRST>
 __device__ __forceinline__ void fast_slice(uint32_t tmem, uint64_t a0, uint64_t b0, uint32_t idesc) {
 #pragma unroll
-    for (int t = 0; t < kFTiles; ++t)
+    for (int t = T0; t < T1; ++t)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
             mma_bf16(tmem + (uint32_t)(kFW * t), a0 + (uint64_t)(t * 1024 + 2 * kk), b0 + (uint64_t)(2 * kk), idesc,
@@ -244,6 +248,11 @@ __global__ void __launch_bounds__(kFThreads, 1)
         const uint32_t idesc = idesc_bf16(128, kFW);
         const uint64_t b_base = sdesc_sw128(smem_u32(wst));
         uint32_t g = 0, n_stage[kFSlots] = {0, 0}, n_act[kFSlots] = {0, 0};
+        auto slice_ready = [&](uint32_t i) {
+            if (!mbar_wait(&w_full[i % kFStages], (i / kFStages) & 1, WL)) return false;
+            tc_fence_after();
+            return true;
+        };
         for (int grp = blockIdx.x; grp < ngroups; grp += G) {
             // first layer: two 64-channel halves of the expanded rows
             for (int h = 0; h < 2; ++h)
@@ -252,18 +261,24 @@ __global__ void __launch_bounds__(kFThreads, 1)
                     ++n_stage[sl];
                     const uint64_t a_base = sdesc_sw128(smem_u32(buf + sl * kFBufBytes));
                     const uint32_t tm = tmem + (uint32_t)(sl * kFTiles * kFW);
+                    if (!slice_ready(g)) { fail(93); goto done_mma; }
 #pragma unroll
                     for (int dy = 0; dy < 5; ++dy, ++g) {
                         const uint32_t st = g % kFStages;
-                        if (!mbar_wait(&w_full[st], (g / kFStages) & 1, WL)) { fail(93); goto done_mma; }
-                        tc_fence_after();
                         const uint64_t a0 = a_base + (uint64_t)((kFPre + kFPitch * (dy - 2)) * 8);
                         const uint64_t b0 = b_base + (uint64_t)(st * (uint32_t)(kFSlice >> 4));
                         if (elect_one()) {
                             if (h == 0 && dy == 0)
-                                fast_slice<true>(tm, a0, b0, idesc);
+                                fast_slice<0, kFTiles - 1, true>(tm, a0, b0, idesc);
                             else
-                                fast_slice<false>(tm, a0, b0, idesc);
+                                fast_slice<0, kFTiles - 1, false>(tm, a0, b0, idesc);
+                        }
+                        if (dy < 4 && !slice_ready(g + 1)) { fail(93); goto done_mma; }
+                        if (elect_one()) {
+                            if (h == 0 && dy == 0)
+                                fast_slice<kFTiles - 1, kFTiles, true>(tm, a0, b0, idesc);
+                            else
+                                fast_slice<kFTiles - 1, kFTiles, false>(tm, a0, b0, idesc);
                             mma_commit(&w_empty[st]);
                             if (dy == 4) mma_commit(h == 0 ? &half_done[sl] : &acc_full[sl]);
                         }
@@ -276,19 +291,25 @@ __global__ void __launch_bounds__(kFThreads, 1)
                     ++n_act[sl];
                     const uint64_t a_base = sdesc_sw128(smem_u32(buf + sl * kFBufBytes));
                     const uint32_t tm = tmem + (uint32_t)(sl * kFTiles * kFW);
+                    if (!slice_ready(g)) { fail(95); goto done_mma; }
 #pragma unroll
                     for (int tap = 0; tap < 9; ++tap, ++g) {
                         const uint32_t st = g % kFStages;
-                        if (!mbar_wait(&w_full[st], (g / kFStages) & 1, WL)) { fail(95); goto done_mma; }
-                        tc_fence_after();
                         const int shift = kFPitch * (tap / 3 - 1) + (tap % 3 - 1);
                         const uint64_t a0 = a_base + (uint64_t)((kFPre + shift) * 8);
                         const uint64_t b0 = b_base + (uint64_t)(st * (uint32_t)(kFSlice >> 4));
                         if (elect_one()) {
                             if (tap == 0)
-                                fast_slice<true>(tm, a0, b0, idesc);
+                                fast_slice<0, kFTiles - 1, true>(tm, a0, b0, idesc);
                             else
-                                fast_slice<false>(tm, a0, b0, idesc);
+                                fast_slice<0, kFTiles - 1, false>(tm, a0, b0, idesc);
+                        }
+                        if (tap < 8 && !slice_ready(g + 1)) { fail(95); goto done_mma; }
+                        if (elect_one()) {
+                            if (tap == 0)
+                                fast_slice<kFTiles - 1, kFTiles, true>(tm, a0, b0, idesc);
+                            else
+                                fast_slice<kFTiles - 1, kFTiles, false>(tm, a0, b0, idesc);
                             mma_commit(&w_empty[st]);
                             if (tap == 8) mma_commit(&acc_full[sl]);
                         }
