@@ -639,10 +639,10 @@ int bucket_of(int B) {
 
 // Where nobody chose, FP32 nets that the split trunk covers leave the
 // small-batch kernel for it from 3 positions on: that kernel's time grows
-// with the batch (benchmark nets, policy + value pair: 179, 313, 447, 715,
-// 1118 us at 1, 2, 3, 5, 8 positions), the split trunk's items run side by
-// side (317 to 328 us over the same sizes).  A hand-set choice 0 stays the
-// FFMA kernels per layer (at 256 positions 14.3 ms a pair against 3.0).
+// with the batch (benchmark nets, policy + value pair: 162, 276, 398, 643,
+// 1010 us at 1, 2, 3, 5, 8 positions), the split trunk's items run side by
+// side (307 to 316 us over the same sizes).  A hand-set choice 0 stays the
+// FFMA kernels per layer (at 256 positions 14.3 ms a pair against 2.6).
 constexpr int kLatSplitB = 2;
 bool use_lat(lg_ctx *c, const Net &n, int B) {
     const int bl = bucket_of(B);
@@ -657,10 +657,11 @@ bool use_split(lg_ctx *c, const Net &n, int B) {
 // Kernel choices without tuning (measured on GB300, policy + value pairs,
 // device-resident inputs): FP32 nets run the small-batch kernel up to 8
 // positions (but see use_lat) and the split trunk above; 16-bit
-// nets run it up to 2 (B = 2: 220 against 254 us on the persistent trunk;
-// B = 3: 314 against 256 us) and the persistent trunk with the first layer
-// inside from 3 positions on (B = 256: 0.43 against 0.76 ms a pair on the
-// per-layer kernels).  A context with a 16-bit net takes the 16-bit rule.
+// nets run it up to 2 and the trunk with the first layer inside from 3
+// positions on (B = 3: 273 against 150 us; B = 256: 0.43 against 0.76 ms a
+// pair on the per-layer kernels).  The cluster trunk would be faster at 2 as
+// well (191 against 150 us), but it rounds differently: the line stays, and
+// the tuner moves it.  A context with a 16-bit net takes the 16-bit rule.
 void default_tuning(lg_ctx *c) {
     bool lowp = false;
     for (const Net &n : c->nets) lowp = lowp || (n.present && n.d.precision != LG_FP32);

@@ -47,12 +47,16 @@
 //              channels): two groups of 8 taking items in turn, so that one's
 //              stores overlap the other's sums
 //
-// What bounds it: the tensor pipe (832 cycles a weight stage, of 1.0k spent),
-// then waits for weight stages.  With one epilogue group the MMAs waited 4.8k
-// of 26k cycles an item for the stores (13.4 ms below).  Policy + value nets
-// of 1,024 positions: 11.9 ms = 211 TFLOP/s of FP32 multiply-adds against
-// 53.2 ms on the FFMA kernels; 77 positions of the reference's shapes through
-// the host call 0.94 against 3.62 ms.
+// What bounds it: the tensor pipe (832 cycles a weight stage, of ~1,150
+// spent), then shared memory (131 KB of operands and writes a stage, 1,024
+// cycles at 128 B/clk) and stages that arrive late.  With one epilogue group
+// the MMAs waited 4.8k of 26k cycles an item for the stores.  Policy + value
+// nets of 1,024 positions: 10.2 to 10.6 ms = 240 TFLOP/s of FP32 multiply-adds
+// against 53.2 ms on the FFMA kernels; 77 positions of the reference's shapes
+// through the host call 0.83 against 3.62 ms.  Pairs of CTAs (M = 256 MMAs,
+// half of B's rows read and, with shared units, 20 KB of weights a stage) were
+// correct but slower (12.3 ms against 11.8, 14.2 against 10.4 with the waits
+// moved).
 //
 // Every wait is bounded; on a timeout the CTA records an error code, stops
 // issuing, drains what it issued and frees its TMEM.
@@ -204,7 +208,13 @@ __device__ __forceinline__ void store_zero_parts(__nv_bfloat16 *dst, size_t part
 
 // The MMAs of one 64-channel half of an item, chains of kSpChain taps: the
 // window in the slot of descriptor x, weight stages g, g + 1, ... of the
-// ring.  Called by a converged warp.  False if a wait ran out.
+// ring.  Called by a converged warp.  A stage's waits come between the MMAs of
+// the stage ahead of it: the tensor pipe has few MMAs queued, and ran dry while
+// the issuer polled between two stages.  Policy + value nets of 1,024
+// positions: waits between the stages 11.8 ms, before the last four of the 12
+// MMAs 10.3, before the last eight 10.2, before the last ten 11.1 (stages that
+// arrive late then hold up more); the next half's first stage and window
+// waited for as well: no gain.  False if a wait ran out.
 template <int NO, bool FIRST>
 __device__ __forceinline__ bool issue_half(SpCtl &ctl, uint32_t tmem, uint64_t x, uint64_t w_desc, int group,
                                            uint32_t &g, uint32_t &chain) {
@@ -212,21 +222,32 @@ __device__ __forceinline__ bool issue_half(SpCtl &ctl, uint32_t tmem, uint64_t x
     using C = SpCfg<NO>;
     constexpr uint32_t id3 = idesc_bf16(128, 3 * NO), id2 = idesc_bf16(128, 2 * NO), id1 = idesc_bf16(128, NO);
     constexpr uint64_t kPart16 = kSpPart >> 4;
+    auto ready = [&](uint32_t stage, bool head, uint32_t ch) {
+        if (head && !mbar_wait(&ctl.acc_empty[ch & 1], ((ch >> 1) & 1) ^ 1, kSpWait)) return false;
+        if (!mbar_wait(&ctl.w_full[stage % C::STAGES], (stage / C::STAGES) & 1, kSpWait)) return false;
+        tc_fence_after();
+        return true;
+    };
+    if (!ready(g, true, chain)) return false;
 #pragma unroll
     for (int t = 0; t < NT; ++t, ++g) {
         const uint32_t s = g % C::STAGES, acc = chain & 1;
         const bool head = t % kSpChain == 0, tail = t % kSpChain == kSpChain - 1 || t == NT - 1;
-        if (head && !mbar_wait(&ctl.acc_empty[acc], ((chain >> 1) & 1) ^ 1, kSpWait)) return false;
-        if (!mbar_wait(&ctl.w_full[s], (g / C::STAGES) & 1, kSpWait)) return false;
-        tc_fence_after();
         const uint32_t d = tmem + acc * C::ACC;
         const uint64_t w = w_desc + (uint64_t)(s * (uint32_t)(C::STAGE >> 4));
         const uint64_t xt = x + (uint64_t)((FIRST ? kSpPre5 + (t - 2) * kL5Pitch
                                                   : kSpPre3 + (t / 3 - 1) * kL3Pitch + (t % 3 - 1)) * 8);
         if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) mma_bf16(d, xt + 2 * kk, w + 2 * kk, id3, head && kk == 0 ? 0u : 1u);
-            if (!FIRST) {
+            for (int kk = 0; kk < (FIRST ? 2 : 4); ++kk)
+                mma_bf16(d, xt + 2 * kk, w + 2 * kk, id3, head && kk == 0 ? 0u : 1u);
+        }
+        if (t + 1 < NT && !ready(g + 1, tail, chain + 1)) return false;
+        if (elect_one()) {
+            if (FIRST) {
+#pragma unroll
+                for (int kk = 2; kk < 4; ++kk) mma_bf16(d, xt + 2 * kk, w + 2 * kk, id3, 1u);
+            } else {
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) mma_bf16(d + NO, xt + kPart16 + 2 * kk, w + 2 * kk, id2, 1u);
 #pragma unroll
@@ -663,8 +684,8 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
     // 32-channel items while 64-channel ones would leave a third of the SMs
     // without any: their MMAs (N = 96, 64, 32) run at two thirds of the rate,
     // but twice as many SMs work on a layer.  Policy + value pair of the
-    // benchmark nets, us, 32 / 64 channels: 5 positions 322 / 422, 16 positions
-    // (100 wide items) 357 / 431, 24 positions (150) 475 / 441.
+    // benchmark nets, us, 32 / 64 channels: 5 positions 311 / 364, 16 positions
+    // (100 wide items) 344 / 371, 20 positions (126) 391 / 375.
     const int no = 3 * n3 * wide <= 2 * sm_count ? 32 : 64;
     int wrows = 0, items = 0, done3 = 0;
     for (int l = 0; l < T.nl; ++l) {
