@@ -40,11 +40,11 @@
 //     kernels, which add the parts in a fixed order.
 //
 // A batch with an SM for every board runs one board a CTA (152 boards: 55 us
-// against 89 in pairs).  8,192 boards, with softmax and value head: 1.57 ms
+// against 89 in pairs).  8,192 boards, with softmax and value head: 1.54 ms
 // with four epilogue warps per TMEM lane quarter, a warp-uniform MMA issuer and
-// each slice's wait before the last MMAs of the slice ahead of it; 1.62 with
-// the waits between the slices; 1.85 also with two epilogue warps and a
-// one-lane issuer.  Of ~107k cycles a pair of boards 84k are the MMAs' own (N
+// each slice's and job's waits before the last MMAs ahead of it; 1.62 with the
+// waits between the slices; 1.85 also with two epilogue warps and a
+// one-lane issuer.  Of ~105k cycles a pair of boards 84k are the MMAs' own (N
 // = 64: 48 cycles each, shared-memory reads), 6k the epilogue's stores in the
 // same shared memory (a deeper ring of slices gains nothing).
 //
@@ -285,13 +285,19 @@ __global__ void __launch_bounds__(kFThreads, 1)
                         __syncwarp();
                     }
                 }
+            bool waited = false;  // by the job before
             for (int l = 1; l < nl; ++l)
                 for (int sl = 0; sl < NS; ++sl) {
-                    if (!mbar_wait(&act_ready[sl], n_act[sl] & 1, WL)) { fail(94); goto done_mma; }
+                    if (!waited && !mbar_wait(&act_ready[sl], n_act[sl] & 1, WL)) { fail(94); goto done_mma; }
                     ++n_act[sl];
                     const uint64_t a_base = sdesc_sw128(smem_u32(buf + sl * kFBufBytes));
                     const uint32_t tm = tmem + (uint32_t)(sl * kFTiles * kFW);
-                    if (!slice_ready(g)) { fail(95); goto done_mma; }
+                    if (!waited && !slice_ready(g)) { fail(95); goto done_mma; }
+                    // with two slots the next job is the other one's, whose
+                    // layer before does not wait for this job: its waits come
+                    // before this job's last MMAs too (8,192 positions 1,567
+                    // -> 1,537 us; the first layer's jobs as well: 1,556)
+                    waited = NS == 2 && (l + 1 < nl || sl == 0);
 #pragma unroll
                     for (int tap = 0; tap < 9; ++tap, ++g) {
                         const uint32_t st = g % kFStages;
@@ -304,7 +310,11 @@ __global__ void __launch_bounds__(kFThreads, 1)
                             else
                                 fast_slice<0, kFTiles - 1, false>(tm, a0, b0, idesc);
                         }
-                        if (tap < 8 && !slice_ready(g + 1)) { fail(95); goto done_mma; }
+                        if (tap == 8 && waited && !mbar_wait(&act_ready[sl ^ 1], n_act[sl ^ 1] & 1, WL)) {
+                            fail(94);
+                            goto done_mma;
+                        }
+                        if ((tap < 8 || waited) && !slice_ready(g + 1)) { fail(95); goto done_mma; }
                         if (elect_one()) {
                             if (tap == 0)
                                 fast_slice<kFTiles - 1, kFTiles, true>(tm, a0, b0, idesc);
