@@ -197,7 +197,7 @@ struct lg_ctx {
     std::atomic<long long> batches{0};
     std::atomic<int> fault_in{0};
     // test hook (lg_inject_stall): the next launch of kernel kind stall_kind
-    // (0 persistent trunk, 1 small-batch kernel) has one wait that nothing
+    // (0 trunk, 1 small-batch kernel) has one wait that nothing
     // satisfies, with its wait limits cut to stall_polls; -1 = disarmed
     int stall_kind = -1;
     uint32_t stall_polls = 0;
@@ -747,6 +747,11 @@ int forward_fp32(lg_ctx *c, Net &n, const uint8_t *planes, int B, float T, float
             T.out32 = c->act[0] + b0 * per_out;
             T.flags = c->sp_flags;
             T.err = c->d_err;
+            if (c->stall_kind == 0) {
+                T.stall = true;
+                T.wait_limit = T.poll_limit = c->stall_polls;
+                c->stall_kind = -1;
+            }
             {
                 ProfScope ps(c, prof, LG_PROF_FP32_CONV, s);
                 if (int rc = launch_split_trunk(T, s, c->sm_count)) return rc;

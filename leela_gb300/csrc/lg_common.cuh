@@ -119,6 +119,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t phase, uint32_
     return false;
 }
 
+// The same for a converged warp, one answer for all of its lanes: what
+// follows (elect.sync, tcgen05.ld, __syncwarp) needs every lane, also where a
+// barrier completes around the last poll.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t phase, uint32_t limit) {
+    for (uint32_t i = 0; i < limit; ++i)
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, phase))) return true;
+    return false;
+}
+
 // 2D tiled TMA load into shared memory, completion on an mbarrier.
 __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *map, uint64_t *bar,
                                             int x, int y) {

@@ -72,6 +72,10 @@ struct SplitTrunk {
     float *out32;            // the last layer's output, [B * 361][cout]
     int *flags;              // split_flag_ints(B) ints, zero between launches
     int *err;
+    // wait limits (0: the defaults) and the test hook that makes the second
+    // layer's first item wait for a count that nothing reaches
+    uint32_t wait_limit, poll_limit;
+    bool stall;
 };
 size_t split_flag_ints(int B);
 int split_pad(int channels);  // channels rounded up to whole groups

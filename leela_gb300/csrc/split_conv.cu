@@ -60,8 +60,9 @@
 // correct but slower (12.3 ms against 11.8, 14.2 against 10.4 with the waits
 // moved).
 //
-// Every wait is bounded; on a timeout the CTA records an error code, stops
-// issuing, drains what it issued and frees its TMEM.
+// Every wait is bounded (the limits are launch parameters); on a timeout the
+// CTA records an error code, stops issuing, drains what it issued and frees
+// its TMEM.  Warps that wait as a whole decide as a whole.
 #include "lg_kernels.h"
 
 #include <algorithm>
@@ -86,7 +87,7 @@ constexpr int kSpSlot = 3 * kSpPart;
 constexpr int kSpSlots = 2;
 constexpr int kSpChain = 2;                       // taps (of 64 channels) per accumulator chain
 constexpr int kSpRing = 4;                        // item descriptors in flight
-constexpr uint32_t kSpWait = 1u << 21;
+constexpr uint32_t kSpWait = 1u << 21;            // default limits: mbarrier polls, counter polls
 constexpr uint32_t kSpPolls = 1u << 22;
 static_assert(kSpWin5 * 128 <= kSpSlot, "a first-layer window fits a slot");
 static_assert(kSpPart % 1024 == 0 && kSpSlot % 1024 == 0, "swizzle alignment");
@@ -137,15 +138,17 @@ struct SpParams {
     int pitch;                // channels per activation row
     int *flags;               // [n3] tile counters, [n5] first-layer tile counters, item counter, exit counter
     int *err;
+    uint32_t wait_limit, poll_limit;
+    int stall_item;           // test hook: this item waits for a count no item reaches (-1: none)
 };
 
 // A converged warp waits until the n counters at f reach `want`, a lane each.
-__device__ __forceinline__ bool sp_poll(const int *f, int n, int want) {
+__device__ __forceinline__ bool sp_poll(const int *f, int n, int want, uint32_t limit) {
     bool ok = true;
     for (int i = threadIdx.x % 32; i < n; i += 32) {
         uint32_t k = 0;
-        while (ld_acquire_gpu(f + i) < want && ++k < kSpPolls) __nanosleep(32);
-        ok = ok && k < kSpPolls;
+        while (ld_acquire_gpu(f + i) < want && ++k < limit) __nanosleep(32);
+        ok = ok && k < limit;
     }
     return __all_sync(0xffffffffu, ok);
 }
@@ -219,14 +222,14 @@ __device__ __forceinline__ void store_zero_parts(__nv_bfloat16 *dst, size_t part
 // waited for as well: no gain.  False if a wait ran out.
 template <int NO, bool FIRST>
 __device__ __forceinline__ bool issue_half(SpCtl &ctl, uint32_t tmem, uint64_t x, uint64_t w_desc, int group,
-                                           uint32_t &g, uint32_t &chain) {
+                                           uint32_t &g, uint32_t &chain, uint32_t limit) {
     constexpr int NT = FIRST ? 5 : 9;
     using C = SpCfg<NO>;
     constexpr uint32_t id3 = idesc_bf16(128, 3 * NO), id2 = idesc_bf16(128, 2 * NO), id1 = idesc_bf16(128, NO);
     constexpr uint64_t kPart16 = kSpPart >> 4;
     auto ready = [&](uint32_t stage, bool head, uint32_t ch) {
-        if (head && !mbar_wait(&ctl.acc_empty[ch & 1], ((ch >> 1) & 1) ^ 1, kSpWait)) return false;
-        if (!mbar_wait(&ctl.w_full[stage % C::STAGES], (stage / C::STAGES) & 1, kSpWait)) return false;
+        if (head && !mbar_wait_warp(&ctl.acc_empty[ch & 1], ((ch >> 1) & 1) ^ 1, limit)) return false;
+        if (!mbar_wait_warp(&ctl.w_full[stage % C::STAGES], (stage / C::STAGES) & 1, limit)) return false;
         tc_fence_after();
         return true;
     };
@@ -323,10 +326,10 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
         j = r / p.L[l].groups;
         g = r - j * p.L[l].groups;
     };
-    // the next item of this warp's walk over the ring; -1 at the end
+    // the next item of this (converged) warp's walk over the ring; -1 at the end
     auto next_item = [&](int q, int code) -> int {
         const int slot = q % kSpRing;
-        if (!mbar_wait(&ctl.item_full[slot], (uint32_t)(q / kSpRing) & 1, kSpWait)) {
+        if (!mbar_wait_warp(&ctl.item_full[slot], (uint32_t)(q / kSpRing) & 1, p.wait_limit)) {
             fail(code);
             return -1;
         }
@@ -341,9 +344,9 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
             int it = -1;
             if (lane == 0) {
                 const int slot = q % kSpRing;
-                bool ok = mbar_wait(&ctl.item_empty[slot], ((uint32_t)(q / kSpRing) & 1) ^ 1, kSpWait);
+                bool ok = mbar_wait(&ctl.item_empty[slot], ((uint32_t)(q / kSpRing) & 1) ^ 1, p.wait_limit);
                 // claimed once its first window slot is free, so that it is worked on at once
-                ok = ok && mbar_wait(&ctl.win_empty[wn % kSpSlots], ((wn / kSpSlots) & 1) ^ 1, kSpWait);
+                ok = ok && mbar_wait(&ctl.win_empty[wn % kSpSlots], ((wn / kSpSlots) & 1) ^ 1, p.wait_limit);
                 if (ok && !abort_flag) {
                     it = atomicAdd(item_ctr, 1);
                     if (it >= p.nitems) it = -1;
@@ -374,7 +377,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                     f = flags3 + lo;
                     n = min(n3 - 1, j + 1) - lo + 1;
                 }
-                if (!sp_poll(f, n, L.need)) {
+                if (!sp_poll(f, n, it == p.stall_item ? 1 << 30 : L.need, p.poll_limit)) {
                     if (lane == 0) fail(102);
                     break;
                 }
@@ -385,7 +388,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                 for (int h = 0; h < L.halves; ++h) {
                     const uint32_t w = wn + h;
                     const int ws = w % kSpSlots;
-                    if (h > 0 && !mbar_wait(&ctl.win_empty[ws], ((w / kSpSlots) & 1) ^ 1, kSpWait)) {
+                    if (h > 0 && !mbar_wait(&ctl.win_empty[ws], ((w / kSpSlots) & 1) ^ 1, p.wait_limit)) {
                         fail(103);
                         break;
                     }
@@ -408,7 +411,11 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
         if (lane == 0) {
             uint32_t g = 0;
             for (int q = 0;; ++q) {
-                const int it = next_item(q, 104);
+                int it = -1;
+                if (mbar_wait(&ctl.item_full[q % kSpRing], (uint32_t)(q / kSpRing) & 1, p.wait_limit))
+                    it = ctl.item_id[q % kSpRing];
+                else
+                    fail(104);
                 mbar_arrive(&ctl.item_empty[q % kSpRing]);
                 if (it < 0) break;
                 int l, j, og;
@@ -419,7 +426,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
                 for (int h = 0; h < L.halves && !bad; ++h)
                     for (int t = 0; t < ntaps; ++t, ++g) {
                         const int s = g % C::STAGES;
-                        if (!mbar_wait(&ctl.w_empty[s], ((g / C::STAGES) & 1) ^ 1, kSpWait)) {
+                        if (!mbar_wait(&ctl.w_empty[s], ((g / C::STAGES) & 1) ^ 1, p.wait_limit)) {
                             fail(105);
                             bad = true;
                             break;
@@ -456,10 +463,10 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
             bool ok = true;
             for (int h = 0; h < halves && ok; ++h, ++wn) {
                 const int ws = wn % kSpSlots;
-                if (!mbar_wait(&ctl.win_full[ws], (wn / kSpSlots) & 1, kSpWait)) { fail(107); ok = false; break; }
+                if (!mbar_wait_warp(&ctl.win_full[ws], (wn / kSpSlots) & 1, p.wait_limit)) { fail(107); ok = false; break; }
                 const uint64_t x = x_desc + (uint64_t)(ws * (kSpSlot >> 4));
-                ok = first ? issue_half<NO, true>(ctl, tmem, x, w_desc, q % kSpGroups, g, chain)
-                           : issue_half<NO, false>(ctl, tmem, x, w_desc, q % kSpGroups, g, chain);
+                ok = first ? issue_half<NO, true>(ctl, tmem, x, w_desc, q % kSpGroups, g, chain, p.wait_limit)
+                           : issue_half<NO, false>(ctl, tmem, x, w_desc, q % kSpGroups, g, chain, p.wait_limit);
                 if (!ok) { fail(108); break; }
                 if (elect_one()) mma_commit(&ctl.win_empty[ws]);
             }
@@ -498,7 +505,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) split_trunk_kernel(const __grid
             for (int c = 0; c < chains; ++c, ++g) {
                 const int acc = g & 1;
                 const uint32_t use = acc ? used[1]++ : used[0]++;
-                if (!mbar_wait(&ctl.acc_full[group][acc], use & 1, kSpWait)) { fail(111); bad = true; break; }
+                if (!mbar_wait_warp(&ctl.acc_full[group][acc], use & 1, p.wait_limit)) { fail(111); bad = true; break; }
                 tc_fence_after();
 #pragma unroll
                 for (int c0 = 0; c0 < C::CH; c0 += 8) {
@@ -680,6 +687,9 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
     p.pitch = T.pitch;
     p.flags = T.flags;
     p.err = T.err;
+    p.wait_limit = T.wait_limit ? T.wait_limit : kSpWait;
+    p.poll_limit = T.poll_limit ? T.poll_limit : kSpPolls;
+    p.stall_item = -1;
     const int n3 = (p.rows + kSpTile - 1) / kSpTile, n5 = (p.rows5 + kSpTile - 1) / kSpTile;
     int wide = 0;
     for (int l = 0; l < T.nl; ++l) wide = std::max(wide, T.L[l].groups);
@@ -715,6 +725,7 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
         items += (L.first ? n5 : n3) * L.groups;
     }
     p.nitems = items;
+    if (T.stall && T.nl > 1) p.stall_item = p.L[1].item0;
     int rc = encode_map_3d_bf16(&p.in[0], T.buf[0], T.pitch, p.rows, 3, T.cap_rows, 64, kSpWin3);
     if (!rc) rc = encode_map_3d_bf16(&p.in[1], T.buf[1], T.pitch, p.rows, 3, T.cap_rows, 64, kSpWin3);
     p.in5 = p.in[0];

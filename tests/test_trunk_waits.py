@@ -1,0 +1,35 @@
+"""Waits of the trunk kernels that run out: whole warps give up together, the
+launch ends in bounded time with an error status, and the next call on the
+same context gives the same results as before."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _stalled_call_and_after(lg, c, call, polls=1 << 14):
+    """`call` with one wait that nothing satisfies, then without."""
+    good = call()
+    c.inject_stall(0, polls)
+    t0 = time.perf_counter()
+    with pytest.raises(lg.LeelaGPUError) as e:
+        call()
+    elapsed = time.perf_counter() - t0
+    assert e.value.code == -5, str(e.value)  # LG_ERR_DEVICE
+    assert elapsed < 20.0
+    assert np.array_equal(call(), good)
+    print(f"stalled call returned after {elapsed * 1e3:.1f} ms: {e.value}")
+
+
+# 32-channel items on few and on most SMs, 64-channel items
+@pytest.mark.parametrize("B", [1, 5, 40])
+def test_split_trunk_wait_runs_out(gpu_lib, weights, positions, B):
+    lg = gpu_lib
+    pp, pv = positions["planes_p"][:B], positions["planes_v"][:B]
+    with lg.Context(policy=lg.NetDesc.reference_policy(weights["ref_p"][1]),
+                    value=lg.NetDesc.reference_value(weights["ref_v"][1]), max_batch=40) as c:
+        c.set_tuning(B, 3, 0)
+        _stalled_call_and_after(lg, c, lambda: c.policy(pp))
+        _stalled_call_and_after(lg, c, lambda: c.value(pv))
