@@ -382,6 +382,10 @@ LG_API int lg_inject_fault(lg_ctx *ctx, int nth_call);
  * working.  kind -1 disarms.  No reference counterpart (the engine's own
  * final wait, OpenCL.cpp:575-577, is unbounded). */
 LG_API int lg_inject_stall(lg_ctx *ctx, int kind, int polls);
+/* The same for the student's serving kernel: its next launch's first CTA
+ * waits in the second layer for what comes only at its end; lg_fast_status
+ * then returns LG_ERR_DEVICE. */
+LG_API int lg_fast_inject_stall(lg_fast *f, int polls);
 
 #ifdef __cplusplus
 }

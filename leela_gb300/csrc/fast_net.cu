@@ -50,9 +50,9 @@
 //
 // Warps: 0 = TMA producer of the weight slices, 1 = TMEM owner and MMA
 // issuer, 2..17 = plane staging, epilogue (four warps per TMEM lane quarter,
-// 16 channels each).  Every wait is bounded; a wait that runs
-// out records an error word, and the CTA drains what it issued and frees
-// its tensor memory.
+// 16 channels each).  Every wait is bounded, and warps that wait as a whole
+// decide as a whole; a wait that runs out records an error word, and the CTA
+// drains what it issued and frees its tensor memory.
 #include "lg_kernels.h"
 
 #include <cfloat>
@@ -108,6 +108,7 @@ struct FastParams {
     size_t part_stride;
     int *err;
     uint32_t wait_limit;
+    int stall;               // test hook: the first CTA's second layer waits for what comes only later
 };
 
 __device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
         const uint64_t b_base = sdesc_sw128(smem_u32(wst));
         uint32_t g = 0, n_stage[kFSlots] = {0, 0}, n_act[kFSlots] = {0, 0};
         auto slice_ready = [&](uint32_t i) {
-            if (!mbar_wait(&w_full[i % kFStages], (i / kFStages) & 1, WL)) return false;
+            if (!mbar_wait_warp(&w_full[i % kFStages], (i / kFStages) & 1, WL)) return false;
             tc_fence_after();
             return true;
         };
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
             // first layer: two 64-channel halves of the expanded rows
             for (int h = 0; h < 2; ++h)
                 for (int sl = 0; sl < NS; ++sl) {
-                    if (!mbar_wait(&stage_full[sl], n_stage[sl] & 1, WL)) { fail(92); goto done_mma; }
+                    if (!mbar_wait_warp(&stage_full[sl], n_stage[sl] & 1, WL)) { fail(92); goto done_mma; }
                     ++n_stage[sl];
                     const uint64_t a_base = sdesc_sw128(smem_u32(buf + sl * kFBufBytes));
                     const uint32_t tm = tmem + (uint32_t)(sl * kFTiles * kFW);
@@ -288,7 +289,11 @@ __global__ void __launch_bounds__(kFThreads, 1)
             bool waited = false;  // by the job before
             for (int l = 1; l < nl; ++l)
                 for (int sl = 0; sl < NS; ++sl) {
-                    if (!waited && !mbar_wait(&act_ready[sl], n_act[sl] & 1, WL)) { fail(94); goto done_mma; }
+                    if (!waited && !mbar_wait_warp(&act_ready[sl], n_act[sl] & 1, WL)) { fail(94); goto done_mma; }
+                    if (p.stall && l == 1 && blockIdx.x == 0 && !mbar_wait_warp(&mma_done, 0, WL)) {
+                        fail(94);
+                        goto done_mma;
+                    }
                     ++n_act[sl];
                     const uint64_t a_base = sdesc_sw128(smem_u32(buf + sl * kFBufBytes));
                     const uint32_t tm = tmem + (uint32_t)(sl * kFTiles * kFW);
@@ -310,7 +315,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
                             else
                                 fast_slice<0, kFTiles - 1, false>(tm, a0, b0, idesc);
                         }
-                        if (tap == 8 && waited && !mbar_wait(&act_ready[sl ^ 1], n_act[sl ^ 1] & 1, WL)) {
+                        if (tap == 8 && waited && !mbar_wait_warp(&act_ready[sl ^ 1], n_act[sl ^ 1] & 1, WL)) {
                             fail(94);
                             goto done_mma;
                         }
@@ -348,7 +353,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
         auto epi_sync = [&]() -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(&epi_bar);
-            const bool ok = mbar_wait(&epi_bar, n_epi & 1, WL);
+            const bool ok = mbar_wait_warp(&epi_bar, n_epi & 1, WL);
             ++n_epi;
             if (!ok) fail(96);
             return ok;
@@ -418,7 +423,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
         // second half once that slot's first-half MMAs have completed
         auto stage_second_halves = [&](int grp) -> bool {
             for (int sl = 0; sl < NS; ++sl) {
-                if (!mbar_wait(&half_done[sl], n_half[sl] & 1, WL)) { fail(97); return false; }
+                if (!mbar_wait_warp(&half_done[sl], n_half[sl] & 1, WL)) { fail(97); return false; }
                 ++n_half[sl];
                 stage(sl, 1, boards(grp));
                 stage_done(sl);
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
                     *reinterpret_cast<float4 *>(bias + 4 * i) =
                         *reinterpret_cast<const float4 *>(s_bias + l * kFW + chq * 16 + 4 * i);
                 for (int sl = 0; sl < NS; ++sl) {
-                    if (!mbar_wait(&acc_full[sl], n_acc[sl] & 1, WL)) { fail(98); goto done_epi; }
+                    if (!mbar_wait_warp(&acc_full[sl], n_acc[sl] & 1, WL)) { fail(98); goto done_epi; }
                     ++n_acc[sl];
                     tc_fence_after();
                     const uint32_t vm = sl < nb ? vmask : 0u;
@@ -668,6 +673,7 @@ struct lg_fast {
     int *g_idx = nullptr, *g_count = nullptr;
     uint8_t *g_fallback = nullptr;
     std::vector<void *> allocs;
+    uint32_t stall_polls = 0;  // test hook: the next launch's wait limits, with one wait that nothing satisfies
     std::mutex mu;
 };
 
@@ -790,7 +796,9 @@ int fast_forward(lg_fast *f, const uint8_t *planes, int B, float T, float *probs
     p.parts_p = f->parts;
     p.parts_v = f->parts + kFParts * p.part_stride;
     p.err = f->err;
-    p.wait_limit = kFWaitLimit;
+    p.wait_limit = f->stall_polls ? f->stall_polls : kFWaitLimit;
+    p.stall = f->stall_polls != 0;
+    f->stall_polls = 0;
     // one board a CTA while every board has an SM of its own
     p.slots = B <= f->sm_count ? 1 : kFSlots;
     const int groups = (B + p.slots - 1) / p.slots;
@@ -954,4 +962,14 @@ extern "C" LG_API int lg_fast_status(lg_fast *f, void *stream) {
     cudaSetDevice(f->device);
     LG_CUDA_TRY(cudaStreamSynchronize((cudaStream_t)stream));
     return fast_check_err(f);
+}
+
+extern "C" LG_API int lg_fast_inject_stall(lg_fast *f, int polls) {
+    if (!f || polls < 0) {
+        lg_set_error("lg_fast_inject_stall: bad arguments");
+        return LG_ERR_ARG;
+    }
+    std::lock_guard<std::mutex> lk(f->mu);
+    f->stall_polls = (uint32_t)(polls ? polls : 1 << 12);
+    return LG_OK;
 }

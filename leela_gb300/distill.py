@@ -47,6 +47,7 @@ def _bind():
     L.lg_fast_destroy.restype = None
     L.lg_fast_device.argtypes = [vp, vp, i32, f32, vp, vp, vp, vp, vp]
     L.lg_fast_status.argtypes = [vp, vp]
+    L.lg_fast_inject_stall.argtypes = [vp, i32]
     L.lg_gated_device.argtypes = [vp, vp, vp, vp, i32, f32, f32, vp, vp, vp, vp, vp]
     L._student_bound = True
     return L
@@ -210,6 +211,10 @@ class FastNet:
 
     def status(self, stream=None):
         _check(library().lg_fast_status(self._h, stream))
+
+    def inject_stall(self, polls: int = 0):
+        """lg_fast_inject_stall: one wait of the next launch runs out."""
+        _check(library().lg_fast_inject_stall(self._h, polls))
 
     def close(self):
         if self._h:

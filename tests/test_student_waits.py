@@ -1,0 +1,41 @@
+"""Waits of the student's kernels that run out: whole warps give up together,
+the launch ends in bounded time with an error status, and what follows is as
+if it had not been."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+# one board a CTA; pairs of boards, a second group on some CTAs
+@pytest.mark.parametrize("n3x3", [1, 5])
+@pytest.mark.parametrize("B", [1, 2 * 152 + 3])
+def test_serving_wait_runs_out(gpu_lib, positions, n3x3, B):
+    import torch
+    from leela_gb300 import distill
+    lg = gpu_lib
+    st = distill.Student(n3x3=n3x3, max_batch=1)
+    st.init_he(2)
+    params = st.get_params()
+    st.close()
+    planes = torch.from_numpy(np.ascontiguousarray(positions["planes_p"][:B, :24])).cuda()
+    with distill.FastNet(params, n3x3=n3x3, max_batch=B) as f:
+        p, v = torch.empty((B, 361), device="cuda"), torch.empty(B, device="cuda")
+
+        def run():
+            f.device(planes.data_ptr(), B, p.data_ptr(), v.data_ptr(), 1.0)
+            f.status()
+            return [t.cpu().numpy() for t in (p, v)]
+
+        good = run()
+        f.inject_stall(1 << 14)
+        t0 = time.perf_counter()
+        with pytest.raises(lg.LeelaGPUError) as e:
+            run()
+        elapsed = time.perf_counter() - t0
+        assert e.value.code == -5, str(e.value)  # LG_ERR_DEVICE
+        assert elapsed < 20.0
+        assert all(np.array_equal(a, b) for a, b in zip(run(), good))
+        print(f"stalled call returned after {elapsed * 1e3:.1f} ms: {e.value}")
