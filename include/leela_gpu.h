@@ -374,7 +374,8 @@ LG_API int lg_inject_fault(lg_ctx *ctx, int nth_call);
 
 /* Test hook (device-side bounded waits): the next launch of kernel `kind`
  * (0: the persistent trunk -- the first item of the second 3x3 layer; for
- * an FP32 net the split trunk, the second layer's first item; 1:
+ * an FP32 net the split trunk, the second layer's first item; for a batch
+ * that runs in clusters, the first CTA's second layer; 1:
  * the small-batch kernel -- row 0 of the second layer) waits for a flag
  * that nothing publishes, with its wait limits cut to `polls` (0: 4096).
  * The wait runs out, the kernel records an error word and unwinds (no trap,

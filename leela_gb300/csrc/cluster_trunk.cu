@@ -32,8 +32,9 @@
 //
 // A neighbour's copy into a row buffer follows, through the layer in between,
 // this CTA's last MMA that read the buffer; a CTA leaves only when the whole
-// cluster has finished.  Every wait is bounded; after one that ran out the CTA
-// stops issuing, lets copies in flight land, and leaves through the same
+// cluster has finished.  Every wait is bounded (the limit is a launch
+// parameter), whole warps decide together; after one that ran out the CTA stops
+// issuing, waits (bounded) for copies in flight, and leaves through the same
 // cluster barrier.
 #include "lg_kernels.h"
 
@@ -59,7 +60,7 @@ constexpr int kClStages = 7;
 constexpr int kClHalo = kClPitch * 128;            // bytes of a board row, one half
 constexpr int kClEpiWarps = 16;
 constexpr int kClThreads = 64 + kClEpiWarps * 32;
-constexpr uint32_t kClWait = 1u << 21;
+constexpr uint32_t kClWait = 1u << 21;             // default limit of a wait, in polls
 // buffer 0: layer inputs of odd index (layer 0's output); buffer 1: the first
 // layer's rows, then layer inputs of even index
 constexpr int kClOff1 = 2 * kClHalf, kClOffW = kClOff1 + 2 * kClHalf5;
@@ -82,6 +83,8 @@ struct ClParams {
     size_t part_stride;
     int nl;
     int *err;
+    uint32_t wait_limit;
+    int stall;                    // test hook: the first CTA's second layer waits for what comes only later
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -140,7 +143,8 @@ __device__ __forceinline__ float cl_transpose_sum(float (&a)[32], int lane) {
 // the buffer's rows at the tap's offset.  Called by a converged warp; false if
 // a stage did not arrive.
 template <bool FIRST, bool F16>
-__device__ __forceinline__ bool cl_layer(ClCtl &ctl, uint32_t tmem, uint64_t w_desc, uint64_t x_desc, uint32_t &g) {
+__device__ __forceinline__ bool cl_layer(ClCtl &ctl, uint32_t tmem, uint64_t w_desc, uint64_t x_desc, uint32_t &g,
+                                         uint32_t limit) {
     constexpr int NT = FIRST ? 5 : 9, HALF = FIRST ? kClHalf5 : kClHalf, PRE = FIRST ? kClPre5 : kClPre;
     constexpr uint32_t idesc = idesc_16(128, kClN, F16);
 #pragma unroll
@@ -148,7 +152,7 @@ __device__ __forceinline__ bool cl_layer(ClCtl &ctl, uint32_t tmem, uint64_t w_d
 #pragma unroll
         for (int t = 0; t < NT; ++t, ++g) {
             const uint32_t s = g % kClStages;
-            if (!mbar_wait(&ctl.w_full[s], (g / kClStages) & 1, kClWait)) return false;
+            if (!mbar_wait_warp(&ctl.w_full[s], (g / kClStages) & 1, limit)) return false;
             tc_fence_after();
             const int shift = FIRST ? (t - 2) * kClPitch : (t / 3 - 1) * kClPitch + t % 3 - 1;
             const uint64_t a = w_desc + (uint64_t)(s * (uint32_t)(kClStage >> 4));
@@ -230,7 +234,7 @@ __global__ void __launch_bounds__(kClThreads, 1) __cluster_dims__(kClSize, 1, 1)
                 for (int j = 0; j < 2 * nt; ++j, ++g) {
                     const int h = j / nt, t = j - h * nt;
                     const uint32_t s = g % kClStages;
-                    if (aborted() || !mbar_wait(&ctl.w_empty[s], ((g / kClStages) & 1) ^ 1, kClWait)) {
+                    if (aborted() || !mbar_wait(&ctl.w_empty[s], ((g / kClStages) & 1) ^ 1, p.wait_limit)) {
                         fail(141);
                         l = p.nl;
                         break;
@@ -245,7 +249,8 @@ __global__ void __launch_bounds__(kClThreads, 1) __cluster_dims__(kClSize, 1, 1)
         const uint64_t w_desc = sdesc_sw128(smem_u32(wst));
         const uint64_t x0 = sdesc_sw128(smem_u32(buf0)), x1 = sdesc_sw128(smem_u32(buf1));
         uint32_t g = 0;
-        bool ok = mbar_wait(&ctl.in_full, 0, kClWait) && cl_layer<true, F16>(ctl, tmem, w_desc, x1, g);
+        bool ok = mbar_wait_warp(&ctl.in_full, 0, p.wait_limit) &&
+                  cl_layer<true, F16>(ctl, tmem, w_desc, x1, g, p.wait_limit);
         if (!ok) fail(142);
         for (int l = 1; l <= p.nl && ok; ++l) {
             // this CTA's rows and both neighbours' (a barrier each: a fast
@@ -256,9 +261,11 @@ __global__ void __launch_bounds__(kClThreads, 1) __cluster_dims__(kClSize, 1, 1)
             }
             __syncwarp();
             const uint32_t ph = (uint32_t)(l - 1) & 1;
-            ok = mbar_wait(&ctl.act_ready, ph, kClWait) && (!up || mbar_wait(&ctl.halo_full[0], ph, kClWait)) &&
-                 (!down || mbar_wait(&ctl.halo_full[1], ph, kClWait));
-            ok = ok && cl_layer<false, F16>(ctl, tmem, w_desc, (l & 1) ? x0 : x1, g);
+            ok = mbar_wait_warp(&ctl.act_ready, ph, p.wait_limit) &&
+                 (!up || mbar_wait_warp(&ctl.halo_full[0], ph, p.wait_limit)) &&
+                 (!down || mbar_wait_warp(&ctl.halo_full[1], ph, p.wait_limit));
+            if (p.stall && l == 1 && blockIdx.x == 0) ok = ok && mbar_wait_warp(&ctl.mma_done, 0, p.wait_limit);
+            ok = ok && cl_layer<false, F16>(ctl, tmem, w_desc, (l & 1) ? x0 : x1, g, p.wait_limit);
             if (!ok) fail(143);
         }
         __syncwarp();
@@ -288,7 +295,7 @@ __global__ void __launch_bounds__(kClThreads, 1) __cluster_dims__(kClSize, 1, 1)
             if (l == p.nl) {
                 // last layer: the 1x1 head's sums, a part per channel quarter
                 const float bias = __ldg(bl + o), scale = sl ? __ldg(sl + o) : 1.0f;
-                if (!mbar_wait(&ctl.acc_full, (uint32_t)l & 1, kClWait)) { fail(144); break; }
+                if (!mbar_wait_warp(&ctl.acc_full, (uint32_t)l & 1, p.wait_limit)) { fail(144); break; }
                 tc_fence_after();
                 uint32_t v[32];
                 tmem_ld32(t_base, v);
@@ -308,7 +315,7 @@ __global__ void __launch_bounds__(kClThreads, 1) __cluster_dims__(kClSize, 1, 1)
                 fb[m] = __ldg(bl + cq + 8 * m);
                 fs[m] = sl ? __ldg(sl + cq + 8 * m) : 1.0f;
             }
-            if (!mbar_wait(&ctl.acc_full, (uint32_t)l & 1, kClWait)) { fail(145); break; }
+            if (!mbar_wait_warp(&ctl.acc_full, (uint32_t)l & 1, p.wait_limit)) { fail(145); break; }
             tc_fence_after();
             uint8_t *const out = (l & 1) ? buf1 : buf0;
             if (l == 0) {
@@ -353,8 +360,8 @@ __global__ void __launch_bounds__(kClThreads, 1) __cluster_dims__(kClSize, 1, 1)
                 if (gives) mbar_arrive(&ctl.row_done[rq == 0 ? 0 : 1]);
                 mbar_arrive(&ctl.act_ready);
                 if (gives && quarter == 0) {
-                    if (l == 0 && !mbar_wait(&ctl.act_ready, 0, kClWait)) fail(146);  // buffer 1 is all zeros
-                    if (!mbar_wait(&ctl.row_done[rq == 0 ? 0 : 1], (uint32_t)l & 1, kClWait)) {
+                    if (l == 0 && !mbar_wait(&ctl.act_ready, 0, p.wait_limit)) fail(146);  // buffer 1 is all zeros
+                    if (!mbar_wait(&ctl.row_done[rq == 0 ? 0 : 1], (uint32_t)l & 1, p.wait_limit)) {
                         fail(147);
                     } else {
                         const uint32_t peer = (uint32_t)(rank + (rq == 0 ? -1 : 1));
@@ -371,14 +378,20 @@ __global__ void __launch_bounds__(kClThreads, 1) __cluster_dims__(kClSize, 1, 1)
     }
 
     __syncthreads();
-    if (aborted()) {
-        if (tid == 0)
-            for (int i = 0; i < kClStages; ++i) {
-                mbar_wait(&ctl.w_full[i], 0, 1u << 16);
-                mbar_wait(&ctl.w_full[i], 1, 1u << 16);
+    if (aborted() && tid == 0) {
+        // copies in flight into this CTA land, or their wait runs out: the
+        // weights, the first layer's rows, the neighbours' rows (whoever sent
+        // one has waited in vain for a row itself since)
+        for (int i = 0; i < kClStages; ++i) {
+            mbar_wait(&ctl.w_full[i], 0, 1u << 16);
+            mbar_wait(&ctl.w_full[i], 1, 1u << 16);
+        }
+        mbar_wait(&ctl.in_full, 0, 1u << 16);
+        for (int i = 0; i < 2; ++i)
+            if (i == 0 ? up : down) {
+                mbar_wait(&ctl.halo_full[i], 0, 1u << 16);
+                mbar_wait(&ctl.halo_full[i], 1, 1u << 16);
             }
-        // rows on their way to a neighbour land before anyone leaves
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
     }
     __syncthreads();
     tc_fence_after();
@@ -435,6 +448,8 @@ int launch_cluster_trunk(const TcTrunk &T, int B, float *parts, size_t part_stri
     p.part_stride = part_stride;
     p.nl = T.nl;
     p.err = err;
+    p.wait_limit = T.wait_limit ? T.wait_limit : kClWait;
+    p.stall = T.stall_item >= 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(B * kClSize);
     cfg.blockDim = dim3(kClThreads);

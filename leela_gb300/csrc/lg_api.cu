@@ -809,10 +809,10 @@ bool trunk_fusable(const Net &n) {
 // side (36 boards: four 227 KB CTAs of a cluster must share a GPC): policy +
 // value pair 148 to 158 us from 1 to 36 positions, against 201 to 250 on the
 // trunk's items; in a second wave the clusters would take 300.  The same
-// results bit for bit.  Nets with another activation than ReLU, device-side
-// batch sizes and the stall hook stay on the trunk.
+// results bit for bit.  Nets with another activation than ReLU and device-side
+// batch sizes stay on the trunk.
 bool use_cluster(const lg_ctx *c, const Net &n, int B, const TcTrunk &t) {
-    return B <= c->cluster_boards && t.buf5 && t.head_w && !t.count && t.stall_item < 0 && n.d.act == LG_ACT_RELU;
+    return B <= c->cluster_boards && t.buf5 && t.head_w && !t.count && n.d.act == LG_ACT_RELU;
 }
 
 // next (optional): the following batch's planes, packed by CTAs of this
