@@ -387,6 +387,9 @@ LG_API int lg_inject_stall(lg_ctx *ctx, int kind, int polls);
  * waits in the second layer for what comes only at its end; lg_fast_status
  * then returns LG_ERR_DEVICE. */
 LG_API int lg_fast_inject_stall(lg_fast *f, int polls);
+/* The same for the training kernels of a 64-wide student: the first CTA of
+ * the next pass's last 3x3 layer's weight gradient. */
+LG_API int lg_student_inject_stall(lg_student *st, int polls);
 
 #ifdef __cplusplus
 }

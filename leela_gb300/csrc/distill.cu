@@ -419,6 +419,7 @@ struct lg_student {
     size_t cap_rows = 0;
     __nv_bfloat16 *xparts = nullptr, *dparts = nullptr, *l5 = nullptr, *dw_parts = nullptr;
     int *flags = nullptr, *err = nullptr;
+    uint32_t stall_polls = 0;  // test hook: limits of the next weight gradient of a 3x3 layer, with one wait that nothing satisfies
     std::mutex mu;
 };
 
@@ -469,7 +470,9 @@ int st_backward_tc(lg_student *s, int B, cudaStream_t st) {
         launch_to_parts(dY, s->Y[l], B, l == 0, s->cap_rows, s->dparts, G(s, c.b), st);
         if (l == 0) return launch_wgrad_first(s->l5, s->dparts, B, s->c_in, s->cap_rows, G(s, c.w), s->err, st);
         launch_to_parts(s->Y[l - 1], nullptr, B, false, s->cap_rows, s->xparts, nullptr, st);
-        if (int rc = launch_wgrad_3x3(s->xparts, s->dparts, B, s->cap_rows, G(s, c.w), s->err, st)) return rc;
+        const uint32_t stall = s->stall_polls;
+        s->stall_polls = 0;
+        if (int rc = launch_wgrad_3x3(s->xparts, s->dparts, B, s->cap_rows, G(s, c.w), s->err, st, stall)) return rc;
         launch_split_weights(P(s, c.w), 3, c.cout, c.cin, s->dw_parts, st, true);
         SplitTrunk T{};
         T.L[0] = SplitLayer{1, 1, c.cin, s->zeros};
@@ -758,5 +761,15 @@ extern "C" int lg_student_forward(lg_student *s, const uint8_t *planes, int B, f
     st_softmax<<<B, 384, 0, st>>>(s->logits, B, probs);
     LG_CUDA_TRY(cudaMemcpyAsync(value, s->vout, B * sizeof(float), cudaMemcpyDeviceToDevice, st));
     LG_CUDA_TRY(cudaGetLastError());
+    return LG_OK;
+}
+
+extern "C" int lg_student_inject_stall(lg_student *s, int polls) {
+    if (!s || polls < 0 || !s->tc) {
+        lg_set_error("lg_student_inject_stall: bad arguments (64-wide students only)");
+        return LG_ERR_ARG;
+    }
+    std::lock_guard<std::mutex> g(s->mu);
+    s->stall_polls = (uint32_t)(polls ? polls : 1 << 12);
     return LG_OK;
 }

@@ -93,16 +93,17 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count);
 // Weight gradients of 64-wide conv layers from such parts (wgrad_tc.cu): dW
 // [taps][channels][64] += X^T dY over all rows.  x, d: [3][cap_rows][64] parts
 // in L3 rows; the 5x5 first layer: l5 the expanded planes [B*399][128] (5 c_in
-// <= 128 real channels), d in L5 rows.
+// <= 128 real channels), d in L5 rows.  stall_polls (test hook): wait limits,
+// with one wait that nothing satisfies; 0: the defaults, no such wait.
 int wgrad_init_device();
 // FP32 [B*361][64] -> parts (L3 rows, or L5 rows with l5); with Y, masked by
 // Y > 0 and summed over rows into db[64].
 void launch_to_parts(const float *src, const float *Y, int B, bool l5, size_t cap_rows, __nv_bfloat16 *parts, float *db,
                      cudaStream_t s);
 int launch_wgrad_3x3(const __nv_bfloat16 *x, const __nv_bfloat16 *d, int B, size_t cap_rows, float *dW, int *err,
-                     cudaStream_t s);
+                     cudaStream_t s, uint32_t stall_polls = 0);
 int launch_wgrad_first(const __nv_bfloat16 *l5, const __nv_bfloat16 *d, int B, int c_in, size_t cap_rows, float *dW,
-                       int *err, cudaStream_t s);
+                       int *err, cudaStream_t s, uint32_t stall_polls = 0);
 
 // Input of the finish kernels: the head output of point (b, p) is
 //   act_head?(sum_k parts[k * part_stride + b * 361 + p] + head_b).

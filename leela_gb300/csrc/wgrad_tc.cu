@@ -41,7 +41,7 @@ constexpr int kWgStages = 3;
 constexpr int kWgFlush = 4;                          // stages per accumulator chain
 constexpr int kWgEpiWarps = 16;
 constexpr int kWgThreads = 128 + kWgEpiWarps * 32;
-constexpr uint32_t kWgWait = 1u << 21;
+constexpr uint32_t kWgWait = 1u << 21;              // default limit of a wait, in polls
 
 template <bool FIRST>
 struct WgCfg {
@@ -73,6 +73,8 @@ struct WgParams {
     int kchan;            // real channels of X (rows of dW per tap)
     float *dW;            // [taps][kchan][64]
     int *err;
+    uint32_t wait_limit;
+    int stall;            // test hook: the first CTA waits for what comes only at its end
 };
 
 // MN-major operand, 128-byte swizzle: 64 channels (128 bytes) a row, 8-row
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const __grid_co
         if (lane == 0) {
             for (int s = s0; s < s1 && !abort_flag; ++s) {
                 const uint32_t n = (uint32_t)(s - s0), st = n % kWgStages;
-                if (!mbar_wait(&ctl.empty[st], ((n / kWgStages) & 1) ^ 1, kWgWait)) { fail(121); break; }
+                if (!mbar_wait(&ctl.empty[st], ((n / kWgStages) & 1) ^ 1, p.wait_limit)) { fail(121); break; }
                 uint8_t *dst = smem + st * C::STAGE;
                 mbar_arrive_expect_tx(&ctl.full[st], C::STAGE);
                 const int r0 = s * kWgRows;
@@ -158,8 +160,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const __grid_co
         for (int s = s0; s < s1; ++s) {
             const uint32_t n = (uint32_t)(s - s0), st = n % kWgStages;
             const bool head = n % kWgFlush == 0;
-            if (head && !mbar_wait(&ctl.acc_empty, ((n / kWgFlush) & 1) ^ 1, kWgWait)) { fail(122); break; }
-            if (!mbar_wait(&ctl.full[st], (n / kWgStages) & 1, kWgWait)) { fail(123); break; }
+            if (head && !mbar_wait_warp(&ctl.acc_empty, ((n / kWgFlush) & 1) ^ 1, p.wait_limit)) { fail(122); break; }
+            if (!mbar_wait_warp(&ctl.full[st], (n / kWgStages) & 1, p.wait_limit)) { fail(123); break; }
+            if (p.stall && blockIdx.x == 0 && !mbar_wait_warp(&ctl.mma_done, 0, p.wait_limit)) { fail(125); break; }
             tc_fence_after();
             const uint32_t xs = base + st * C::STAGE, ds = xs + C::NX * C::XBLK;
             const uint64_t d0 = desc_mn(ds, C::DBLK);
@@ -206,7 +209,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const __grid_co
         const int nflush = (s1 - s0 + kWgFlush - 1) / kWgFlush;
         bool bad = false;
         for (int f = 0; f < nflush; ++f) {
-            if (!mbar_wait(&ctl.acc_full, (uint32_t)f & 1, kWgWait)) { fail(124); bad = true; break; }
+            if (!mbar_wait_warp(&ctl.acc_full, (uint32_t)f & 1, p.wait_limit)) { fail(124); bad = true; break; }
             tc_fence_after();
 #pragma unroll
             for (int i = 0; i < C::TAPS; ++i) {
@@ -335,7 +338,7 @@ void launch_to_parts(const float *src, const float *Y, int B, bool l5, size_t ca
 
 template <bool FIRST>
 static int launch_wgrad(const CUtensorMap &x, const CUtensorMap &d, int rows, int kchan, float *dW, int *err,
-                        cudaStream_t s) {
+                        cudaStream_t s, uint32_t stall_polls) {
     using C = WgCfg<FIRST>;
     WgParams p{};
     p.x = x;
@@ -346,28 +349,30 @@ static int launch_wgrad(const CUtensorMap &x, const CUtensorMap &d, int rows, in
     p.kchan = kchan;
     p.dW = dW;
     p.err = err;
+    p.wait_limit = stall_polls ? stall_polls : kWgWait;
+    p.stall = stall_polls != 0;
     wgrad_tc_kernel<FIRST><<<C::GROUPS * p.ranges, kWgThreads, C::SMEM, s>>>(p);
     return LG_OK;
 }
 
 int launch_wgrad_3x3(const __nv_bfloat16 *x, const __nv_bfloat16 *d, int B, size_t cap_rows, float *dW, int *err,
-                     cudaStream_t s) {
+                     cudaStream_t s, uint32_t stall_polls) {
     using C = WgCfg<false>;
     const int rows = B * kL3Board;
     CUtensorMap mx, md;
     int rc = encode_map_3d_bf16(&mx, x, 64, rows, 3, cap_rows, 64, C::XBLK / 128);
     if (!rc) rc = encode_map_3d_bf16(&md, d, 64, rows, 3, cap_rows, 64, kWgRows);
-    return rc ? rc : launch_wgrad<false>(mx, md, rows, 64, dW, err, s);
+    return rc ? rc : launch_wgrad<false>(mx, md, rows, 64, dW, err, s, stall_polls);
 }
 
 int launch_wgrad_first(const __nv_bfloat16 *l5, const __nv_bfloat16 *d, int B, int c_in, size_t cap_rows, float *dW,
-                       int *err, cudaStream_t s) {
+                       int *err, cudaStream_t s, uint32_t stall_polls) {
     using C = WgCfg<true>;
     const int rows = B * kL5Board;
     CUtensorMap mx, md;
     int rc = encode_map_2d_bf16(&mx, l5, 128, rows, 64, C::XBLK / 128);
     if (!rc) rc = encode_map_3d_bf16(&md, d, 64, rows, 3, cap_rows, 64, kWgRows);
-    return rc ? rc : launch_wgrad<true>(mx, md, rows, 5 * c_in, dW, err, s);
+    return rc ? rc : launch_wgrad<true>(mx, md, rows, 5 * c_in, dW, err, s, stall_polls);
 }
 
 }  // namespace lg

@@ -39,6 +39,7 @@ def _bind():
     L.lg_student_train_step.argtypes = [vp, vp, i32, vp, vp, f32, f32, vp, vp]
     L.lg_student_grads.argtypes = [vp, vp, i32, vp, vp, f32, vp, vp]
     L.lg_student_forward.argtypes = [vp, vp, i32, vp, vp, vp]
+    L.lg_student_inject_stall.argtypes = [vp, i32]
     L.lg_fast_param_count.argtypes = [i32, i32, i32]
     L.lg_fast_param_count.restype = ctypes.c_size_t
     L.lg_fast_create.argtypes = [i32, i32, i32, i32, i32, vp, P(vp)]
@@ -144,6 +145,10 @@ class Student:
 
     def forward(self, planes_ptr, B, probs_ptr, value_ptr, stream=None):
         _check(library().lg_student_forward(self._h, planes_ptr, B, probs_ptr, value_ptr, stream))
+
+    def inject_stall(self, polls: int = 0):
+        """lg_student_inject_stall: one wait of the next backward pass runs out."""
+        _check(library().lg_student_inject_stall(self._h, polls))
 
 
 def train(student: Student, planes, target_probs, target_value, steps: int, batch: int = 256,

@@ -39,3 +39,38 @@ def test_serving_wait_runs_out(gpu_lib, positions, n3x3, B):
         assert elapsed < 20.0
         assert all(np.array_equal(a, b) for a, b in zip(run(), good))
         print(f"stalled call returned after {elapsed * 1e3:.1f} ms: {e.value}")
+
+
+def _batch(positions, B, seed=0):
+    import torch
+    rng = np.random.default_rng(seed)
+    t = rng.random((B, 361)).astype(np.float32) ** 4
+    t /= t.sum(1, keepdims=True)
+    v = rng.uniform(-0.8, 0.8, B).astype(np.float32)
+    return [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (positions["planes_p"][:B, :24], t, v)]
+
+
+# one row range a tap group; every SM busy
+@pytest.mark.parametrize("B", [1, 64])
+def test_weight_gradient_wait_runs_out(gpu_lib, positions, B):
+    from leela_gb300 import distill
+    lg = gpu_lib
+    st = distill.Student(n3x3=2, max_batch=B)
+    st.init_he(3)
+    p, t, v = _batch(positions, B)
+
+    def run():
+        return st.grads(p.data_ptr(), B, t.data_ptr(), v.data_ptr(), 0.5)[1]
+
+    good = run()
+    st.inject_stall(1 << 14)
+    t0 = time.perf_counter()
+    with pytest.raises(lg.LeelaGPUError) as e:
+        run()
+    elapsed = time.perf_counter() - t0
+    assert e.value.code == -5, str(e.value)  # LG_ERR_DEVICE
+    assert elapsed < 20.0
+    # sums over rows are added up in no fixed order
+    assert np.abs(run() - good).max() <= 1e-5 * np.abs(good).max()
+    print(f"stalled call returned after {elapsed * 1e3:.1f} ms: {e.value}")
+    st.close()
