@@ -299,7 +299,10 @@ LG_API size_t lg_student_param_count(const lg_student *st);
 LG_API int lg_student_set_params(lg_student *st, const float *host, size_t n);
 LG_API int lg_student_get_params(lg_student *st, float *host, size_t n);
 /* One Adam step (lr, betas 0.9 / 0.999, eps 1e-8); host_loss (optional)
- * receives {policy KL, value MSE} of the batch. */
+ * receives {policy KL, value MSE} of the batch.  If a kernel of the step gives
+ * up a bounded wait, the update and those after it are left out (the
+ * parameters stay those of the last good step) until a call returns
+ * LG_ERR_DEVICE: this one with host_loss, else a later call of the student. */
 LG_API int lg_student_train_step(lg_student *st, const uint8_t *planes, int B, const float *target_probs,
                                  const float *target_value, float lr, float value_weight, float *host_loss,
                                  void *stream);

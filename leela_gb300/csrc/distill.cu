@@ -373,9 +373,20 @@ __global__ void st_flip_weights(const float *__restrict__ wt, int kk, int Cin, i
     }
 }
 
+// Does nothing where a kernel of the pass (or of one before it that nobody has
+// asked about) gave up a wait: err[0], the error word, is set.  Such updates
+// are counted in err[1], and the word goes to pinned host memory, where the
+// next call sees it without a synchronization.  (err null: no such kernels.)
 __global__ void st_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
                         float *__restrict__ v, size_t n, float lr, float b1, float b2, float eps,
-                        float c1, float c2) {
+                        float c1, float c2, int *__restrict__ err, volatile int *__restrict__ herr) {
+    if (err && err[0]) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            err[1] += 1;
+            *herr = err[0];
+        }
+        return;
+    }
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.0f - b1) * gi;
@@ -418,7 +429,9 @@ struct lg_student {
     int sm_count = 152;
     size_t cap_rows = 0;
     __nv_bfloat16 *xparts = nullptr, *dparts = nullptr, *l5 = nullptr, *dw_parts = nullptr;
-    int *flags = nullptr, *err = nullptr;
+    int *flags = nullptr;
+    int *err = nullptr;    // the error word, updates left out because of it
+    int *h_err = nullptr;  // pinned: the error word as the last update left out saw it
     uint32_t stall_polls = 0;  // test hook: limits of the next weight gradient of a 3x3 layer, with one wait that nothing satisfies
     std::mutex mu;
 };
@@ -528,15 +541,28 @@ int st_backward(lg_student *s, int B, const float *target, const float *vt, floa
     return LG_OK;
 }
 
-// After a synchronization: LG_ERR_DEVICE if a kernel gave up a bounded wait.
+// After a synchronization of the stream that ran the passes: LG_ERR_DEVICE if
+// a kernel gave up a bounded wait.  The parameters and the Adam state are those
+// of the last step whose kernels all ran to their end.
 int st_check_err(lg_student *s) {
     if (!s->tc) return LG_OK;
-    int herr = 0;
-    LG_CUDA_TRY(cudaMemcpy(&herr, s->err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (!herr) return LG_OK;
-    cudaMemset(s->err, 0, sizeof(int));
-    lg_set_error("student: kernel reported error status %d", herr);
+    int e[2] = {0, 0};
+    LG_CUDA_TRY(cudaMemcpy(e, s->err, sizeof e, cudaMemcpyDeviceToHost));
+    if (!e[0]) return LG_OK;
+    LG_CUDA_TRY(cudaMemset(s->err, 0, sizeof e));
+    LG_CUDA_TRY(cudaStreamSynchronize(nullptr));  // before the next pass, on any stream
+    *s->h_err = 0;
+    s->step -= e[1];
+    lg_set_error("student: kernel reported error status %d (%d updates left out)", e[0], e[1]);
     return LG_ERR_DEVICE;
+}
+
+// At the start of a call on stream st: the error of a training step that
+// returned before its kernels had run.
+int st_check_pending(lg_student *s, cudaStream_t st) {
+    if (!s->h_err || !*(volatile int *)s->h_err) return LG_OK;
+    LG_CUDA_TRY(cudaStreamSynchronize(st));
+    return st_check_err(s);
 }
 
 bool valid_batch(lg_student *s, int B) { return s && B >= 1 && B <= s->max_batch; }
@@ -548,6 +574,7 @@ extern "C" void lg_student_destroy(lg_student *s) {
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
     for (void *p : s->allocs) cudaFree(p);
+    if (s->h_err) cudaFreeHost(s->h_err);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
 }
@@ -633,10 +660,15 @@ extern "C" int lg_student_create(int device, int c_in, int width, int n3x3, int 
             (rc = st_alloc(s, &s->xparts, 3 * s->cap_rows * 64)) || (rc = st_alloc(s, &s->dparts, 3 * s->cap_rows * 64)) ||
             (rc = st_alloc(s, &s->l5, (size_t)max_batch * kL5Board * 128)) ||
             (rc = st_alloc(s, &s->dw_parts, split_weight_elems(3, width, width))) ||
-            (rc = st_alloc(s, &s->flags, nf)) || (rc = st_alloc(s, &s->err, 1)))
+            (rc = st_alloc(s, &s->flags, nf)) || (rc = st_alloc(s, &s->err, 2)))
             return fail(rc);
+        if (cudaMallocHost(&s->h_err, sizeof(int)) != cudaSuccess) {
+            lg_set_error("cudaMallocHost failed");
+            return fail(LG_ERR_ALLOC);
+        }
+        *s->h_err = 0;
         cudaMemset(s->flags, 0, nf * sizeof(int));
-        cudaMemset(s->err, 0, sizeof(int));
+        cudaMemset(s->err, 0, 2 * sizeof(int));
     }
     cudaMemset(s->zeros, 0, 256 * sizeof(float));
     cudaMemset(s->params, 0, off * sizeof(float));
@@ -670,6 +702,7 @@ extern "C" int lg_student_set_params(lg_student *s, const float *host, size_t n)
     }
     std::memcpy(&gpu[s->wp], host + hoff, (n - hoff) * sizeof(float));  // heads + FC: same order
     cudaSetDevice(s->device);
+    if (int rc = st_check_err(s)) return rc;
     LG_CUDA_TRY(cudaMemcpy(s->params, gpu.data(), n * sizeof(float), cudaMemcpyHostToDevice));
     LG_CUDA_TRY(cudaMemset(s->m, 0, n * sizeof(float)));
     LG_CUDA_TRY(cudaMemset(s->v, 0, n * sizeof(float)));
@@ -702,6 +735,7 @@ extern "C" int lg_student_get_params(lg_student *s, float *host, size_t n) {
     }
     std::lock_guard<std::mutex> g(s->mu);
     cudaSetDevice(s->device);
+    if (int rc = st_check_err(s)) return rc;
     return to_host_layout(s, s->params, host);
 }
 
@@ -714,6 +748,7 @@ extern "C" int lg_student_grads(lg_student *s, const uint8_t *planes, int B, con
     }
     std::lock_guard<std::mutex> g(s->mu);
     cudaSetDevice(s->device);
+    if (int rc = st_check_pending(s, s->stream)) return rc;
     st_forward(s, planes, B, s->stream, true);
     if (int rc = st_backward(s, B, target_probs, target_value, value_weight, s->stream)) return rc;
     LG_CUDA_TRY(cudaGetLastError());
@@ -733,12 +768,14 @@ extern "C" int lg_student_train_step(lg_student *s, const uint8_t *planes, int B
     std::lock_guard<std::mutex> g(s->mu);
     cudaSetDevice(s->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
+    if (int rc = st_check_pending(s, st)) return rc;
     st_forward(s, planes, B, st, true);
     if (int rc = st_backward(s, B, target_probs, target_value, value_weight, st)) return rc;
     s->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - std::pow(b1, (float)s->step), c2 = 1.0f - std::pow(b2, (float)s->step);
-    st_adam<<<512, 256, 0, st>>>(s->params, s->grads, s->m, s->v, s->nparam, lr, b1, b2, 1e-8f, c1, c2);
+    st_adam<<<512, 256, 0, st>>>(s->params, s->grads, s->m, s->v, s->nparam, lr, b1, b2, 1e-8f, c1, c2, s->err,
+                                 s->h_err);
     LG_CUDA_TRY(cudaGetLastError());
     if (host_loss) {
         LG_CUDA_TRY(cudaMemcpyAsync(host_loss, s->loss, 2 * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -757,6 +794,7 @@ extern "C" int lg_student_forward(lg_student *s, const uint8_t *planes, int B, f
     std::lock_guard<std::mutex> g(s->mu);
     cudaSetDevice(s->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
+    if (int rc = st_check_pending(s, st)) return rc;
     st_forward(s, planes, B, st, false);
     st_softmax<<<B, 384, 0, st>>>(s->logits, B, probs);
     LG_CUDA_TRY(cudaMemcpyAsync(value, s->vout, B * sizeof(float), cudaMemcpyDeviceToDevice, st));

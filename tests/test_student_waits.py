@@ -74,3 +74,48 @@ def test_weight_gradient_wait_runs_out(gpu_lib, positions, B):
     assert np.abs(run() - good).max() <= 1e-5 * np.abs(good).max()
     print(f"stalled call returned after {elapsed * 1e3:.1f} ms: {e.value}")
     st.close()
+
+
+@pytest.mark.parametrize("seen_by", ["loss", "step", "forward", "grads", "params"])
+def test_failed_training_step_leaves_the_parameters(gpu_lib, positions, seen_by):
+    """A step whose weight gradient gave up changes nothing, nor does one after
+    it, until a call reports the error; training then goes on as if neither
+    had been (Adam's step count included)."""
+    import torch
+    from leela_gb300 import distill
+    lg = gpu_lib
+    B = 16
+    st = distill.Student(n3x3=2, max_batch=B)
+    st.init_he(3)
+    p, t, v = _batch(positions, B)
+    probs, value = torch.empty((B, 361), device="cuda"), torch.empty(B, device="cuda")
+
+    def step(want_loss=False):
+        return st.train_step(p.data_ptr(), B, t.data_ptr(), v.data_ptr(), 1e-3, 0.5, want_loss=want_loss)
+
+    start = st.get_params()
+    step(True)
+    one = st.get_params()
+    step(True)
+    two = st.get_params()
+    st.set_params(start)
+    step(True)
+    first = st.get_params()
+    st.inject_stall(1 << 14)
+    report = {"loss": lambda: step(True), "step": step,
+              "forward": lambda: st.forward(p.data_ptr(), B, probs.data_ptr(), value.data_ptr()),
+              "grads": lambda: st.grads(p.data_ptr(), B, t.data_ptr(), v.data_ptr(), 0.5),
+              "params": st.get_params}[seen_by]
+    if seen_by != "loss":
+        step()
+        torch.cuda.synchronize()
+    with pytest.raises(lg.LeelaGPUError) as e:
+        report()
+    assert e.value.code == -5, str(e.value)  # LG_ERR_DEVICE
+    assert np.array_equal(st.get_params(), first)
+    step(True)
+    # one step moves a parameter by about 1e-3; sums are added up in no fixed
+    # order, and a gradient near zero may take either sign of it
+    near = lambda a, b: np.mean(np.abs(a - b) > 1e-5) < 1e-2
+    assert near(first, one) and near(st.get_params(), two) and not near(one, two)
+    st.close()
