@@ -290,7 +290,12 @@ LG_API int lg_set_tuning(lg_ctx *ctx, int B, int variant_3x3, int variant_first)
  * by lg_create at any precision.
  *
  * planes / targets are device pointers: planes [B][c_in][361] bytes, target
- * probabilities [B][361], target values [B] in [-1, 1]. */
+ * probabilities [B][361], target values [B] in [-1, 1].
+ *
+ * stream NULL, and the calls without a stream, use the student's own stream,
+ * which is ordered with the legacy default stream: after work put there
+ * before the call, before work put there later.  Work on other streams is the
+ * caller's to order. */
 typedef struct lg_student lg_student;
 LG_API int lg_student_create(int device, int c_in, int width, int n3x3, int fc_hidden, int max_batch,
                              lg_student **out);

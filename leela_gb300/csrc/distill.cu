@@ -602,7 +602,10 @@ extern "C" int lg_student_create(int device, int c_in, int width, int n3x3, int 
         lg_set_error("no CUDA device %d", device);
         return fail(LG_ERR_CUDA);
     }
-    if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(LG_ERR_CUDA);
+    // A blocking stream: a pass on it comes after what the caller has put on the
+    // legacy default stream (its inputs) and before what follows there (the
+    // parameter copies, the caller's use of the outputs).
+    if (cudaStreamCreate(&s->stream) != cudaSuccess) return fail(LG_ERR_CUDA);
     size_t off = 0;
     for (int l = 0; l <= n3x3; ++l) {
         lg_student::Conv c{};

@@ -161,9 +161,8 @@ def train(student: Student, planes, target_probs, target_value, steps: int, batc
     N = planes.shape[0]
     log = []
     t0 = time.perf_counter()
-    # steps are ordered with the minibatch copies: 1 is the legacy default
-    # stream by its handle (0 would pick the student's own stream, which runs
-    # while the next minibatch is written over this one)
+    # steps go where the minibatch copies go; 1 is the legacy default stream by
+    # its handle (0 would pick the student's own stream, ordered with it)
     stream = torch.cuda.current_stream().cuda_stream or 1
     for it in range(steps):
         idx = torch.randint(0, N, (batch,), generator=g).to(planes.device)
