@@ -257,9 +257,10 @@ LG_API int lg_policy_device_static(lg_ctx *ctx, const uint8_t *planes, int B, fl
  * FP32 kernels, 3 = the trunk in one launch on the tensor cores, each FP32
  * value as the sum of three BF16 parts, 4 = the small-batch kernel), and
  * keeps the fastest.  With a
- * cache path, a table saved for the same device, SM count and net shapes is
- * loaded instead (unless force), and a new table is saved there (written to
- * a temporary file and renamed).  Without tuning (measured defaults): a
+ * cache path, a table saved for the same device, SM count, net shapes and
+ * kernels of the library is loaded instead (unless force), and a new table is
+ * saved there (written to a temporary file and renamed); batches beyond its
+ * last bucket keep what they had, as after measuring.  Without tuning (measured defaults): a
  * context with a 16-bit net uses choice 4 up to 2 positions and choice 3
  * above; an FP32-only context uses choice 4 up to 8 positions and its
  * per-layer kernels above, where nets whose layers have 32 to 256 channels

@@ -2117,25 +2117,42 @@ extern "C" int lg_policy_device_static(lg_ctx *c, const uint8_t *planes, int B, 
 // Autotuner: for every power-of-two batch bucket up to max_batch, time the
 // tensor-core nets' forward with each kernel choice for the 3x3 layers and
 // for the first layer (256-row transposed kernel or 128-row kernel), keep
-// the fastest, and cache the table as JSON keyed by device name, SM count
-// and net widths.  FP32 nets: the per-layer kernels, the split trunk and the
-// small-batch kernel.
+// the fastest, and cache the table as JSON keyed by device name, SM count,
+// the nets' shapes and the kernels that there are.  FP32 nets: the per-layer
+// kernels, the split trunk and the small-batch kernel.
 // ============================================================================
 
 namespace {
+
+// Goes up when a choice comes to mean another kernel, or a kernel's speed
+// changes much: older tables are then measured anew (one from before the split
+// trunk would keep FP32 nets on the FFMA kernels).
+constexpr int kTuneKernels = 2;
 
 std::string tune_key(lg_ctx *c) {
     cudaDeviceProp prop{};
     cudaGetDeviceProperties(&prop, c->device);
     char buf[512];
-    snprintf(buf, sizeof buf, "%s|sm%d|p%d/%d/%d|v%d/%d/%d|mb%d", prop.name, c->sm_count,
-             c->nets[0].present ? c->nets[0].d.precision : -1, c->nets[0].present ? c->nets[0].d.width : 0,
-             c->nets[0].present ? c->nets[0].d.c_in : 0, c->nets[1].present ? c->nets[1].d.precision : -1,
-             c->nets[1].present ? c->nets[1].d.width : 0, c->nets[1].present ? c->nets[1].d.c_in : 0,
-             c->max_batch);
-    return buf;
+    snprintf(buf, sizeof buf, "%s|sm%d", prop.name, c->sm_count);
+    std::string key = buf;
+    for (int i = 0; i < 2; ++i) {
+        const Net &n = c->nets[i];
+        snprintf(buf, sizeof buf, "|%c%d/%d/%d", i ? 'v' : 'p', n.present ? n.d.precision : -1, n.present ? n.d.width : 0,
+                 n.present ? n.d.c_in : 0);
+        key += buf;
+    }
+    snprintf(buf, sizeof buf, "|mb%d|k%d", c->max_batch, kTuneKernels);
+    key += buf;
+    // depth, first width, head and what the small-batch kernel and the split trunk cover
+    for (const Net &n : c->nets) {
+        snprintf(buf, sizeof buf, "|%d/%d/%d/%d%d", n.d.n3x3, n.d.width1, n.d.head_k, n.lat_ok, n.split_ok);
+        key += n.present ? buf : "|";
+    }
+    return key;
 }
 
+// Takes over the buckets that the file holds (powers of two up to max_batch);
+// the others stay as they are, as they do in the context that tuned.
 bool load_tuning(lg_ctx *c, const char *path) {
     FILE *f = fopen(path, "r");
     if (!f) return false;
@@ -2147,6 +2164,7 @@ bool load_tuning(lg_ctx *c, const char *path) {
     std::string key = "\"key\": \"" + tune_key(c) + "\"";
     if (text.find(key) == std::string::npos) return false;
     int table[17][2] = {};
+    bool found[17] = {};
     for (int b = 0; b <= 16; ++b) {
         char pat[64];
         snprintf(pat, sizeof pat, "\"%d\": [", 1 << b);
@@ -2157,9 +2175,13 @@ bool load_tuning(lg_ctx *c, const char *path) {
         if (a < 0 || a > 4 || d < 0 || d > 1) return false;
         table[b][0] = a;
         table[b][1] = d;
+        found[b] = true;
     }
-    std::memcpy(c->tc_variant, table, sizeof table);
-    std::fill(std::begin(c->chosen), std::end(c->chosen), true);
+    for (int b = 0; b <= 16; ++b)
+        if (found[b]) {
+            std::memcpy(c->tc_variant[b], table[b], sizeof table[b]);
+            c->chosen[b] = true;
+        }
     return true;
 }
 
@@ -2170,7 +2192,7 @@ int save_tuning(lg_ctx *c, const char *path, const double (*ms)[8]) {
         lg_set_error("cannot write %s", tmp.c_str());
         return LG_ERR_ARG;
     }
-    fprintf(f, "{\n \"key\": \"%s\",\n \"order\": \"[3x3 layers: 0 = 256-row transposed per layer, 1 = 128-row per layer, 2 = persistent trunk, 3 = persistent trunk with the first layer in it, 4 = the whole net in one small-batch launch (FP32 nets: 0 = per-layer kernels, 4 = small-batch); first layer: 0 = 256-row, 1 = 128-row]; ms_per_forward for (3x3, first) = (0,0) (1,0) (2,0) (0,1) (1,1) (2,1) (3,0) (4,0), 0 = not timed\",\n \"table\": {",
+    fprintf(f, "{\n \"key\": \"%s\",\n \"order\": \"[3x3 layers: 0 = 256-row transposed per layer, 1 = 128-row per layer, 2 = persistent trunk, 3 = persistent trunk with the first layer in it, 4 = the whole net in one small-batch launch (FP32 nets: 0 = per-layer FFMA kernels, 3 = split trunk, 4 = small-batch); first layer: 0 = 256-row, 1 = 128-row]; ms_per_forward for (3x3, first) = (0,0) (1,0) (2,0) (0,1) (1,1) (2,1) (3,0) (4,0), 0 = not timed\",\n \"table\": {",
             tune_key(c).c_str());
     bool first = true;
     for (int b = 0; (1 << b) <= c->max_batch && b <= 16; ++b) {
