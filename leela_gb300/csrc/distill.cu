@@ -659,18 +659,27 @@ extern "C" int lg_student_create(int device, int c_in, int width, int n3x3, int 
         cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, device);
         s->cap_rows = (size_t)max_batch * kL3Board;
         const size_t nf = split_flag_ints(max_batch);
-        if ((rc = split_init_device()) || (rc = wgrad_init_device()) ||
-            (rc = st_alloc(s, &s->xparts, 3 * s->cap_rows * 64)) || (rc = st_alloc(s, &s->dparts, 3 * s->cap_rows * 64)) ||
+        if ((rc = split_init_device()) || (rc = wgrad_init_device())) return fail(rc);
+        // Made last: without room for them the backward stays on the FFMA
+        // kernels, which need none.
+        const size_t before = s->allocs.size();
+        if ((rc = st_alloc(s, &s->xparts, 3 * s->cap_rows * 64)) || (rc = st_alloc(s, &s->dparts, 3 * s->cap_rows * 64)) ||
             (rc = st_alloc(s, &s->l5, (size_t)max_batch * kL5Board * 128)) ||
             (rc = st_alloc(s, &s->dw_parts, split_weight_elems(3, width, width))) ||
-            (rc = st_alloc(s, &s->flags, nf)) || (rc = st_alloc(s, &s->err, 2)))
-            return fail(rc);
+            (rc = st_alloc(s, &s->flags, nf)) || (rc = st_alloc(s, &s->err, 2))) {
+            for (; s->allocs.size() > before; s->allocs.pop_back()) cudaFree(s->allocs.back());
+            cudaGetLastError();  // the allocation's
+            s->tc = false;
+            s->err = nullptr;
+        }
+    }
+    if (s->tc) {
         if (cudaMallocHost(&s->h_err, sizeof(int)) != cudaSuccess) {
             lg_set_error("cudaMallocHost failed");
             return fail(LG_ERR_ALLOC);
         }
         *s->h_err = 0;
-        cudaMemset(s->flags, 0, nf * sizeof(int));
+        cudaMemset(s->flags, 0, split_flag_ints(max_batch) * sizeof(int));
         cudaMemset(s->err, 0, 2 * sizeof(int));
     }
     cudaMemset(s->zeros, 0, 256 * sizeof(float));

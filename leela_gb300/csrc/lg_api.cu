@@ -334,15 +334,20 @@ int build_lat(lg_ctx *c, Net &n, const std::vector<std::vector<float>> &Wraw) {
 // and 3x3 layers of 32 to 256 channels, padded to groups of 64, with finite
 // weights (an infinite weight has no parts).  Narrower nets keep the FFMA
 // kernels: less than half of a padded group would be theirs.
-int build_split(lg_ctx *c, Net &n, const std::vector<std::vector<float>> &Wraw,
-                const std::vector<std::vector<float>> &Braw) {
+bool split_covers(const Net &n, const std::vector<std::vector<float>> &Wraw) {
     const int ntrunk = (int)n.shapes.size() - 1;
     bool ok = ntrunk >= 2 && ntrunk <= kSpMaxLayers;
     for (int l = 0; l < ntrunk && ok; ++l) {
         ok = n.shapes[l].cout >= 32 && n.shapes[l].cout <= 256;
         for (float v : Wraw[l]) ok = ok && std::isfinite(v);
     }
-    if (!ok) return LG_OK;
+    return ok;
+}
+
+// A covered net's weights as parts and its biases padded to whole groups, from
+// the FP32 path's copies on the device.
+int build_split(lg_ctx *c, Net &n) {
+    const int ntrunk = (int)n.shapes.size() - 1;
     size_t elems = 0;
     for (int l = 0; l < ntrunk; ++l) elems += split_weight_elems(n.shapes[l].k, n.shapes[l].cin, n.shapes[l].cout);
     if (int rc = dev_alloc(c, &n.split_w, elems)) return rc;
@@ -356,15 +361,61 @@ int build_split(lg_ctx *c, Net &n, const std::vector<std::vector<float>> &Wraw,
         n.split_pitch = std::max(n.split_pitch, S.groups * 64);
         launch_split_weights(n.wt[l], sh.k, sh.cin, sh.cout, n.split_w + at, c->stream);
         at += split_weight_elems(sh.k, sh.cin, sh.cout);
-        std::vector<float> b(Braw[l]);
-        b.resize((size_t)S.groups * 64, 0.0f);
         float *db;
-        if (int rc = upload(c, &db, b)) return rc;
+        if (int rc = dev_alloc(c, &db, (size_t)S.groups * 64)) return rc;
+        LG_CUDA_TRY(cudaMemset(db, 0, (size_t)S.groups * 64 * sizeof(float)));
+        LG_CUDA_TRY(cudaMemcpy(db, n.bias[l], sh.cout * sizeof(float), cudaMemcpyDeviceToDevice));
         S.bias = db;
         n.split.push_back(S);
     }
     LG_CUDA_TRY(cudaGetLastError());
-    n.split_ok = true;
+    return LG_OK;
+}
+
+// The split trunk's weights and buffers, made after everything that a context
+// cannot do without.  Where memory is short, its launches take fewer positions
+// (the same bits); where not even one has room, the nets keep their other
+// kernels.
+int make_split(lg_ctx *c) {
+    bool any = false;
+    for (const Net &n : c->nets) any = any || n.split_ok;
+    if (!any) return LG_OK;
+    if (int rc = split_init_device()) return rc;
+    auto give_back = [&](size_t keep) {
+        cudaStreamSynchronize(c->stream);
+        for (; c->allocs.size() > keep; c->allocs.pop_back()) cudaFree(c->allocs.back());
+        cudaGetLastError();  // the allocation's
+    };
+    const size_t before = c->allocs.size();
+    int rc = LG_OK, pitch = 0, halves = 0;
+    for (Net &n : c->nets)
+        if (n.split_ok && rc == LG_OK && (rc = build_split(c, n)) == LG_OK) {
+            pitch = std::max(pitch, n.split_pitch);
+            halves = std::max(halves, n.split[0].halves);
+        }
+    const size_t weights = c->allocs.size();
+    for (int b = std::min(c->max_batch, kSplitMaxBatch); rc == LG_OK && b >= 1; b /= 2) {
+        const size_t nf = split_flag_ints(b);
+        for (auto &a : c->sp_act)
+            if (rc == LG_OK) rc = dev_alloc(c, &a, 3 * (size_t)b * kL3Board * pitch);
+        if (rc == LG_OK) rc = dev_alloc(c, &c->sp_l5, (size_t)b * kL5Board * halves * 64);
+        if (rc == LG_OK) rc = dev_alloc(c, &c->sp_flags, nf);
+        if (rc == LG_OK) {
+            LG_CUDA_TRY(cudaMemset(c->sp_flags, 0, nf * sizeof(int)));
+            c->split_batch = b;
+            return LG_OK;
+        }
+        if (rc == LG_ERR_ALLOC) {
+            give_back(weights);
+            rc = b > 1 ? LG_OK : rc;
+        }
+    }
+    if (rc != LG_ERR_ALLOC) return rc;
+    give_back(before);
+    for (Net &n : c->nets) {
+        n.split_ok = false;
+        n.split.clear();
+    }
     return LG_OK;
 }
 
@@ -483,7 +534,8 @@ int build_net(lg_ctx *c, Net &n, const lg_net_desc *d) {
             for (int t = 0; t < kk; ++t) wh[(size_t)t * hs.cin + ci] = Wraw.back()[(size_t)ci * kk + t];
         if ((rc = upload(c, &n.head_w, wh))) return rc;
         n.head_b = Braw.back()[0];
-        if ((rc = build_lat(c, n, Wraw)) || (rc = build_split(c, n, Wraw, Braw))) return rc;
+        if ((rc = build_lat(c, n, Wraw))) return rc;
+        n.split_ok = split_covers(n, Wraw);
     } else {
         // ---- tensor-core layouts: [tap][half][N][64] 16-bit operands (BF16,
         // or FP16 for LG_FP16), K-major rows.
@@ -1626,7 +1678,7 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
         return fail(LG_ERR_CUDA);
     const lg_net_desc *descs[2] = {policy, value};
     size_t max_act = 0, max_partial = 0, max_tc_l3 = 0, max_tc_l5 = 0;
-    int max_c_in = 0, max_fc = 0, sp_pitch = 0, sp_halves = 0;
+    int max_c_in = 0, max_fc = 0;
     for (int i = 0; i < 2; ++i) {
         if (!descs[i]) continue;
         if ((rc = build_net(c, c->nets[i], descs[i]))) return fail(rc);
@@ -1634,11 +1686,6 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
         max_c_in = std::max(max_c_in, n.d.c_in);
         if (n.d.value_head) max_fc = std::max(max_fc, n.d.fc_hidden);
         if (n.d.precision == LG_FP32) {
-            if (n.split_ok) {
-                if ((rc = split_init_device())) return fail(rc);
-                sp_pitch = std::max(sp_pitch, n.split_pitch);
-                sp_halves = std::max(sp_halves, n.split[0].halves);
-            }
             for (auto &s : n.shapes) {
                 max_act = std::max(max_act, (size_t)std::max(s.cin, s.cout));
                 for (int b = 1; b <= max_batch; b = (b < 64 ? b + 1 : b * 2))
@@ -1659,15 +1706,6 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
             (rc = dev_alloc(c, &c->act[1], mb * kPoints * max_act)) ||
             (rc = dev_alloc(c, &c->partial, max_partial)))
             return fail(rc);
-    }
-    if (sp_pitch) {
-        c->split_batch = std::min(max_batch, kSplitMaxBatch);
-        const size_t sb = (size_t)c->split_batch, nf = split_flag_ints(c->split_batch);
-        if ((rc = dev_alloc(c, &c->sp_act[0], 3 * sb * kL3Board * sp_pitch)) ||
-            (rc = dev_alloc(c, &c->sp_act[1], 3 * sb * kL3Board * sp_pitch)) ||
-            (rc = dev_alloc(c, &c->sp_l5, sb * kL5Board * sp_halves * 64)) || (rc = dev_alloc(c, &c->sp_flags, nf)))
-            return fail(rc);
-        if (cudaMemset(c->sp_flags, 0, nf * sizeof(int)) != cudaSuccess) return fail(LG_ERR_CUDA);
     }
     if (max_tc_l3) {
         if ((rc = dev_alloc(c, &c->l3[0], mb * kL3Board * max_tc_l3)) ||
@@ -1735,6 +1773,7 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
             return fail(LG_ERR_ALLOC);
         }
     }
+    if ((rc = make_split(c))) return fail(rc);
     if (cudaDeviceSynchronize() != cudaSuccess) {
         lg_set_error("device error after upload");
         return fail(LG_ERR_CUDA);
