@@ -442,6 +442,7 @@ template <class T>
 int st_alloc(lg_student *s, T **p, size_t count) {
     if (cudaMalloc((void **)p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) {
         lg_set_error("cudaMalloc failed (%zu bytes)", count * sizeof(T));
+        cudaGetLastError();  // reported here: a later call's check must not find it
         return LG_ERR_ALLOC;
     }
     s->allocs.push_back(*p);
@@ -596,6 +597,7 @@ extern "C" int lg_student_create(int device, int c_in, int width, int n3x3, int 
     s->max_batch = max_batch;
     auto fail = [&](int rc) {
         lg_student_destroy(s);
+        cudaGetLastError();  // as in st_alloc
         return rc;
     };
     if (cudaSetDevice(device) != cudaSuccess) {
@@ -668,7 +670,6 @@ extern "C" int lg_student_create(int device, int c_in, int width, int n3x3, int 
             (rc = st_alloc(s, &s->dw_parts, split_weight_elems(3, width, width))) ||
             (rc = st_alloc(s, &s->flags, nf)) || (rc = st_alloc(s, &s->err, 2))) {
             for (; s->allocs.size() > before; s->allocs.pop_back()) cudaFree(s->allocs.back());
-            cudaGetLastError();  // the allocation's
             s->tc = false;
             s->err = nullptr;
         }

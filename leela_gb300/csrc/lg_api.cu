@@ -232,6 +232,7 @@ int dev_alloc(lg_ctx *c, T **p, size_t count) {
     cudaError_t e = cudaMalloc((void **)p, count * sizeof(T));
     if (e != cudaSuccess) {
         lg_set_error("cudaMalloc(%zu bytes): %s", count * sizeof(T), cudaGetErrorString(e));
+        cudaGetLastError();  // reported here: a later call's check must not find it
         *p = nullptr;
         return LG_ERR_ALLOC;
     }
@@ -384,7 +385,6 @@ int make_split(lg_ctx *c) {
     auto give_back = [&](size_t keep) {
         cudaStreamSynchronize(c->stream);
         for (; c->allocs.size() > keep; c->allocs.pop_back()) cudaFree(c->allocs.back());
-        cudaGetLastError();  // the allocation's
     };
     const size_t before = c->allocs.size();
     int rc = LG_OK, pitch = 0, halves = 0;
@@ -1058,6 +1058,7 @@ int pipe_alloc(lg_ctx *c) {
     if ((!c->pl_h_in && cudaMallocHost(&c->pl_h_in, R * c->pl_in_bytes) != cudaSuccess) ||
         (!c->pl_h_out && cudaMallocHost(&c->pl_h_out, R * c->pl_out_floats * sizeof(float)) != cudaSuccess)) {
         lg_set_error("board pipeline: cudaMallocHost failed");
+        cudaGetLastError();  // as in dev_alloc
         return LG_ERR_ALLOC;
     }
     if (!c->pl_d_out)
@@ -1670,6 +1671,7 @@ extern "C" int lg_create(const lg_net_desc *policy, const lg_net_desc *value, in
     int rc = LG_OK;
     auto fail = [&](int r) {
         lg_destroy(c);
+        cudaGetLastError();  // as in dev_alloc
         return r;
     };
     if (cudaSetDevice(device) != cudaSuccess) return fail(LG_ERR_CUDA);

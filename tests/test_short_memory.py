@@ -76,3 +76,23 @@ def test_student_with_little_memory(gpu_lib, positions):
     with _leaving(need - 150 * MIB):  # of 200 for the backward's buffers
         _, got = grads()
     assert np.linalg.norm(got - good) <= 1e-5 * np.linalg.norm(good)
+
+
+def test_a_failed_creation_leaves_no_error_behind(gpu_lib, weights, positions):
+    import torch
+    from leela_gb300 import distill
+    lg = gpu_lib
+    x = positions["planes_p"][:8]
+    kw = dict(policy=lg.NetDesc.reference_policy(weights["ref_p"][1]))
+    with lg.Context(max_batch=8, **kw) as c:
+        good = c.policy(x)
+    for make in (lambda: lg.Context(max_batch=4096, **kw), lambda: distill.Student(max_batch=2048)):
+        with _leaving(512 * MIB):
+            with pytest.raises(lg.LeelaGPUError) as e:
+                make()
+        assert e.value.code == -2, str(e.value)  # LG_ERR_ALLOC
+        with lg.Context(max_batch=8, **kw) as c:
+            planes, probs = torch.from_numpy(x).cuda(), torch.empty((8, 361), device="cuda")
+            c.policy_device(planes.data_ptr(), 8, probs.data_ptr(), 1.0)
+            torch.cuda.synchronize()
+            assert np.array_equal(probs.cpu().numpy(), good)
