@@ -382,6 +382,9 @@ int make_split(lg_ctx *c) {
     for (const Net &n : c->nets) any = any || n.split_ok;
     if (!any) return LG_OK;
     if (int rc = split_init_device()) return rc;
+    // the weights' copies to the device go by the default stream, which c->stream
+    // does not wait for, and may still be on their way when cudaMemcpy returns
+    LG_CUDA_TRY(cudaDeviceSynchronize());
     auto give_back = [&](size_t keep) {
         cudaStreamSynchronize(c->stream);
         for (; c->allocs.size() > keep; c->allocs.pop_back()) cudaFree(c->allocs.back());
