@@ -266,10 +266,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const bool active = HEAD ? (chalf == 0) : true;
         const int cbase = HEAD ? 0 : chalf * (N / 2);
         int local = 0;
-        for (int tile = blockIdx.x; tile < p.ntiles && !abort_flag; tile += gridDim.x, ++local) {
+        for (int tile = blockIdx.x; tile < p.ntiles && !__any_sync(0xffffffffu, abort_flag); tile += gridDim.x, ++local) {
             const int acc = local & 1;
             const uint32_t ak = (uint32_t)(local >> 1);
-            if (!mbar_wait(&acc_full[acc], ak & 1, kWaitLimit)) { fail(31); break; }
+            if (!mbar_wait_warp(&acc_full[acc], ak & 1, kWaitLimit)) { fail(31); break; }
             tc_fence_after();
             if (active) {
                 int orow, point;
@@ -549,12 +549,12 @@ __global__ void __launch_bounds__(kTcThreadsT, 1)
         uint32_t uses = 0;  // staging buffer uses of this row group (same for its 4 warps)
         int r0, r1;
         cta_row_range(p.rows, r0, r1);
-        for (int cs = r0; cs < r1 && !abort_flag; cs += C::TP, ++local) {
+        for (int cs = r0; cs < r1 && !__any_sync(0xffffffffu, abort_flag); cs += C::TP, ++local) {
             const int nrows = min(C::TP, r1 - cs);
             const int nhalf = max(0, min(2, (nrows - rq * 64) / 32));  // 32-row halves of this group
             const int acc = local & 1;
             const uint32_t ak = (uint32_t)(local >> 1);
-            if (!mbar_wait(&acc_full[acc], ak & 1, kWaitLimit)) { fail(61); break; }
+            if (!mbar_wait_warp(&acc_full[acc], ak & 1, kWaitLimit)) { fail(61); break; }
             tc_fence_after();
             const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) +
                                     (uint32_t)(acc * C::TP + rq * 64);
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(kTcThreadsT, 1)
                     // one TMA store by the group's quarter-0 warp.
                     const uint32_t use = uses++;
                     uint8_t *buf = stg + rq * C::STG_BYTES;
-                    if (!mbar_wait(&stg_empty[rq], (use & 1) ^ 1, kWaitLimit)) { fail(62); break; }
+                    if (!mbar_wait_warp(&stg_empty[rq], (use & 1) ^ 1, kWaitLimit)) { fail(62); break; }
                     const int row_lane = q_base + c * 32 + lane;
                     const int rl = row_lane % kL3Board;
                     const bool valid_lane = (rl % kL3Pitch) < kBoard && (rl / kL3Pitch) < kBoard;
@@ -1066,7 +1066,7 @@ __global__ void __maxnreg__(96)
         uint32_t uses = 0, done_n = 0;
         for (int q = 0;; ++q) {
             const int slot = q % kItemRing;
-            if (!mbar_wait(&item_full[slot], (uint32_t)(q / kItemRing) & 1, WAIT_LIM)) { fail(79); break; }
+            if (!mbar_wait_warp(&item_full[slot], (uint32_t)(q / kItemRing) & 1, WAIT_LIM)) { fail(79); break; }
             const int it = item_id[slot];
             __syncwarp();
             if (lane == 0) mbar_arrive(&item_empty[slot]);
@@ -1086,7 +1086,7 @@ __global__ void __maxnreg__(96)
             const int nhalf = max(0, min(C::NH, (nrows - rq * C::RG + 31) / 32));
             const int acc = q & 1;
             const uint32_t ak = (uint32_t)(q >> 1);
-            if (!mbar_wait(&acc_full[acc], ak & 1, WAIT_LIM)) { fail(80); break; }
+            if (!mbar_wait_warp(&acc_full[acc], ak & 1, WAIT_LIM)) { fail(80); break; }
             tc_fence_after();
             const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256 + rq * C::RG);
             const int q_base = cs + rq * C::RG;
@@ -1124,7 +1124,7 @@ __global__ void __maxnreg__(96)
                     }
                     if (c >= nhalf || bad) continue;
                     const uint32_t use = uses++;
-                    if (!mbar_wait(&stg_empty[rq], (use & 1) ^ 1, WAIT_LIM)) {
+                    if (!mbar_wait_warp(&stg_empty[rq], (use & 1) ^ 1, WAIT_LIM)) {
                         fail(81);
                         bad = true;
                         continue;
@@ -1198,7 +1198,7 @@ __global__ void __maxnreg__(96)
                 } else {
                     const uint32_t use = uses++;
                     uint8_t *buf = stg + rq * C::STG_BYTES;
-                    if (!mbar_wait(&stg_empty[rq], (use & 1) ^ 1, WAIT_LIM)) {
+                    if (!mbar_wait_warp(&stg_empty[rq], (use & 1) ^ 1, WAIT_LIM)) {
                         fail(81);
                         bad = true;
                         continue;

@@ -50,3 +50,14 @@ def test_cluster_trunk_wait_runs_out(gpu_lib, oracle_mod, positions, n3x3, B):
                     max_batch=64) as c:
         c.set_tuning(B, 3, 0)
         _stalled_call_and_after(lg, c, lambda: c.policy(pp), cluster=True)
+
+
+# 128- and 256-row items, the first layer inside the launch and before it; 64-row
+# items (batches of this size run in clusters with choice 3)
+@pytest.mark.parametrize("B,choice", [(24, 2), (40, 3), (97, 2), (256, 3)])
+def test_persistent_trunk_wait_runs_out(gpu_lib, weights, positions, B, choice):
+    lg = gpu_lib
+    pv = positions["planes_v"][:B, :24]
+    with lg.Context(value=lg.NetDesc.config1_value(weights["cfg_v"][1], "fp16"), max_batch=256) as c:
+        c.set_tuning(B, choice, 0)
+        _stalled_call_and_after(lg, c, lambda: c.value(pv))
