@@ -35,7 +35,13 @@ extern "C" {
 #define LG_ERR_TIMEOUT -4  /* a bounded wait ran out */
 #define LG_ERR_DEVICE -5   /* a kernel reported an error status */
 
-#define LG_FP32 0 /* plain FP32: the drop-in path */
+#define LG_FP32 0 /* FP32 weights, activations and sums: the drop-in path.  Products
+                   are FP32 multiply-adds up to 2 positions (nets that the small-
+                   batch kernel covers) and in kernel choice 0 (lg_set_tuning);
+                   else, for nets whose layers have 32 to 256 channels, six tensor-
+                   core products of the values' three BF16 parts (all 24 bits),
+                   added in FP32, with an error against 64 bits no larger than the
+                   multiply-adds' */
 #define LG_BF16 1 /* BF16 activations and weights, FP32 accumulate (tcgen05) */
 #define LG_FP8W 2 /* E4M3 weights with per-output-channel FP32 scales, BF16 activations */
 #define LG_FP16 3 /* FP16 activations and weights, FP32 accumulate (tcgen05, same rate as BF16) */
@@ -101,7 +107,10 @@ LG_API int lg_weights_load(const char *path, int index, lg_net_desc *desc, char 
 LG_API size_t lg_weight_count(const lg_net_desc *desc);
 
 /* Uploads the nets (either may be NULL) to `device` and sizes every buffer
- * for up to max_batch positions per call.
+ * for up to max_batch positions per call.  The split trunk of FP32 nets has
+ * buffers of its own for up to 1,024 positions (0.6 GB for layers of up to 128
+ * channels, twice that up to 256), made last: fewer where memory is short, none
+ * (and the other kernels) where not even one position has room.
  * Replaces: Network::initialize (Network.cpp:201-235), i.e.
  * OpenCL_Network::push_convolve / push_innerproduct (OpenCL.h:66-87,
  * OpenCL.cpp:579-744) and the device pick in OpenCL::initialize
@@ -262,12 +271,14 @@ LG_API int lg_policy_device_static(lg_ctx *ctx, const uint8_t *planes, int B, fl
  * saved there (written to a temporary file and renamed); batches beyond its
  * last bucket keep what they had, as after measuring.  Without tuning (measured defaults): a
  * context with a 16-bit net uses choice 4 up to 2 positions and choice 3
- * above; an FP32-only context uses choice 4 up to 8 positions and its
- * per-layer kernels above, where nets whose layers have 32 to 256 channels
- * run the split trunk from 3 positions on.  No reference
+ * above; in an FP32-only context the table starts with choice 4 up to 8
+ * positions and choice 0 above, and while nobody has chosen for a bucket (by
+ * hand, by measuring or from a cache), FP32 nets whose layers have 32 to 256
+ * channels run the split trunk (as in choice 3) from 3 positions on.  Choosing
+ * 0 for a bucket keeps its FP32 nets on the FFMA kernels.  No reference
  * counterpart (the OpenCL backend reads a fixed cfg_rowtiles,
- * OpenCL.cpp:634-646).  lg_tuning reports the choice for batch B; it returns
- * 1 once tuned, 0 if not, < 0 on error. */
+ * OpenCL.cpp:634-646).  lg_tuning reports the table's choice for batch B; it
+ * returns 1 once tuned, 0 if not, < 0 on error. */
 LG_API int lg_autotune(lg_ctx *ctx, const char *cache_path, int force);
 LG_API int lg_tuning(lg_ctx *ctx, int B, int *variant_3x3, int *variant_first);
 /* Sets the kernel choice of B's bucket by hand (3x3: 0-4, first: 0-1); a

@@ -24,7 +24,7 @@
 //
 // What bounds it: shared memory in the MMAs (8 KB of operands for 64 cycles and
 // a weight stage written every four: ~6.7k cycles a layer), then the hand-over
-// (~2k).  24 positions, policy + value: 154 us against 223 on the trunk's
+// (~2k).  24 positions, policy + value: 150 us against 223 on the trunk's
 // 64-row items.
 //
 // Warps: 0 weights (and the first layer's rows), 1 MMA issuer and TMEM owner,

@@ -476,7 +476,7 @@ int st_forward(lg_student *s, const uint8_t *planes, int B, cudaStream_t st, boo
 // weight gradient from X's and dY's parts, the input gradient as a conv of
 // dY's parts with the flipped weights.  dY of the last layer in s->dA.  512
 // boards: 1.25 ms against 8.1 on the FFMA kernels (2.2 input gradients, 5.3
-// weight gradients, 0.27 masks), a whole pass 3.4 ms against 11.1.
+// weight gradients, 0.27 masks), a whole pass 3.24 ms against 11.1.
 int st_backward_tc(lg_student *s, int B, cudaStream_t st) {
     float *dY = s->dA, *dX = s->dB;
     for (int l = (int)s->convs.size() - 1; l >= 0; --l) {

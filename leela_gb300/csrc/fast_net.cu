@@ -39,12 +39,13 @@
 //     memory; the softmax and the value FC run as the library's finish
 //     kernels, which add the parts in a fixed order.
 //
-// A batch with an SM for every board runs one board a CTA (152 boards: 55 us
-// against 89 in pairs).  8,192 boards, with softmax and value head: 1.54 ms
-// with four epilogue warps per TMEM lane quarter, a warp-uniform MMA issuer and
-// each slice's and job's waits before the last MMAs ahead of it; 1.62 with the
-// waits between the slices; 1.85 also with two epilogue warps and a
-// one-lane issuer.  Of ~105k cycles a pair of boards 84k are the MMAs' own (N
+// A batch with an SM for every board runs one board a CTA (152 boards: 49 us
+// against 89 in pairs).  8,192 boards, with softmax and value head: 1.47 ms
+// with four epilogue warps per TMEM lane quarter, a warp-uniform MMA issuer,
+// one vote per poll of a wait and each slice's and job's waits before the last
+// MMAs ahead of it; 1.54 with each lane deciding on its own; 1.62 also with the
+// waits between the slices; 1.85 also with two epilogue warps and a one-lane
+// issuer.  Of ~105k cycles a pair of boards 84k are the MMAs' own (N
 // = 64: 48 cycles each, shared-memory reads), 6k the epilogue's stores in the
 // same shared memory (a deeper ring of slices gains nothing).
 //
@@ -131,8 +132,9 @@ __device__ __forceinline__ uint32_t relu_bf16x2(float lo, float hi) {
 // issuing thread spends an add per operand and MMA.  FIRST: the slice
 // starts every accumulator.  Tiles T0 .. T1 - 1: the issuer waits for the
 // next slice before the last tile of the one ahead of it, so that the tensor
-// pipe does not run dry meanwhile (8,192 positions: waits between the slices
-// 1,620 us, before the last tile 1,568, before the last two 1,575).
+// pipe does not run dry meanwhile (8,192 positions, polls without a vote: waits
+// between the slices 1,620 us, before the last tile 1,568, before the last two
+// 1,575).
 template <int T0, int T1, bool FIRST>
 __device__ __forceinline__ void fast_slice(uint32_t tmem, uint64_t a0, uint64_t b0, uint32_t idesc) {
 #pragma unroll
@@ -300,8 +302,9 @@ __global__ void __launch_bounds__(kFThreads, 1)
                     if (!waited && !slice_ready(g)) { fail(95); goto done_mma; }
                     // with two slots the next job is the other one's, whose
                     // layer before does not wait for this job: its waits come
-                    // before this job's last MMAs too (8,192 positions 1,567
-                    // -> 1,537 us; the first layer's jobs as well: 1,556)
+                    // before this job's last MMAs too (8,192 positions, polls
+                    // without a vote, 1,567 -> 1,537 us; the first layer's jobs
+                    // as well: 1,556)
                     waited = NS == 2 && (l + 1 < nl || sl == 0);
 #pragma unroll
                     for (int tap = 0; tap < 9; ++tap, ++g) {

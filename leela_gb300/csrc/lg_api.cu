@@ -696,8 +696,12 @@ int bucket_of(int B) {
 // small-batch kernel for it from 3 positions on: that kernel's time grows
 // with the batch (benchmark nets, policy + value pair: 162, 276, 398, 643,
 // 1010 us at 1, 2, 3, 5, 8 positions), the split trunk's items run side by
-// side (307 to 316 us over the same sizes).  A hand-set choice 0 stays the
-// FFMA kernels per layer (at 256 positions 14.3 ms a pair against 2.6).
+// side (275 to 293 us over the same sizes).  Its error against 64 bits is no
+// larger: means of 24 seeds at 3 to 8 positions, small-batch kernel / split
+// trunk, relative 2-norm, logits 8.9e-7 / 7.8e-7, probabilities 2.0e-7 / 1.6e-7
+// (reference-shaped nets 9.3e-7 / 7.2e-7, 1.4e-6 / 1.1e-6).  A hand-set choice
+// 0 stays the FFMA kernels per layer (at 256 positions 14.3 ms a pair against
+// 2.6).
 constexpr int kLatSplitB = 2;
 bool use_lat(lg_ctx *c, const Net &n, int B) {
     const int bl = bucket_of(B);
@@ -713,9 +717,9 @@ bool use_split(lg_ctx *c, const Net &n, int B) {
 // device-resident inputs): FP32 nets run the small-batch kernel up to 8
 // positions (but see use_lat) and the split trunk above; 16-bit
 // nets run it up to 2 and the trunk with the first layer inside from 3
-// positions on (B = 3: 273 against 150 us; B = 256: 0.43 against 0.76 ms a
+// positions on (B = 3: 273 against 148 us; B = 256: 0.43 against 0.76 ms a
 // pair on the per-layer kernels).  The cluster trunk would be faster at 2 as
-// well (191 against 150 us), but it rounds differently: the line stays, and
+// well (193 against 146 us), but it rounds differently: the line stays, and
 // the tuner moves it.  A context with a 16-bit net takes the 16-bit rule.
 void default_tuning(lg_ctx *c) {
     bool lowp = false;
@@ -862,7 +866,7 @@ bool trunk_fusable(const Net &n) {
 
 // Choice 3 with a cluster of four CTAs a board while all of them run side by
 // side (36 boards: four 227 KB CTAs of a cluster must share a GPC): policy +
-// value pair 148 to 158 us from 1 to 36 positions, against 201 to 250 on the
+// value pair 144 to 154 us from 1 to 36 positions, against 201 to 250 on the
 // trunk's items; in a second wave the clusters would take 300.  The same
 // results bit for bit.  Nets with another activation than ReLU and device-side
 // batch sizes stay on the trunk.

@@ -20,9 +20,11 @@
 // (the parts have the weight's sign, so an infinite activation gives the
 // same infinity as one product would).
 //
-// Against 64 bits the benchmark nets' logits are 7.9e-7 off at every batch
-// (FFMA kernels 6.9e-7 to 1.64e-6, growing with the batch as their K splits
-// go; 64-deep chains gain nothing over a whole net and cost 10%).
+// Against 64 bits the benchmark nets' logits are 7.8e-7 off at every batch
+// (relative 2-norm, mean of 24 seeds; the small-batch FFMA kernel 8.9e-7, the
+// FFMA kernels per layer 7.0e-7 at one position to 2.3e-6 at 256, growing as
+// their K splits go; 64-deep chains gain nothing over a whole net and cost
+// 10%).
 //
 // GEMM shape (NO = 64 output channels an item; 32 for small batches, with
 // half the N): M = 128 flat rows (the L3 / L5 layouts of lg_common.cuh: a tap
@@ -47,15 +49,16 @@
 //              channels): two groups of 8 taking items in turn, so that one's
 //              stores overlap the other's sums
 //
-// What bounds it: the tensor pipe (832 cycles a weight stage, of ~1,130
-// spent; 69% active under ncu, shared memory 68%, L2 31%), then the issuer's
+// What bounds it: the tensor pipe (832 cycles a weight stage, of ~1,090
+// spent; 72% active under ncu, shared memory 71%, L2 34%), then the issuer's
 // commits and waits: a barrier for each part of a stage, so that a part is
-// refilled as soon as its MMAs are done, took 13.1 ms where one a stage takes
-// 10.2 (two commits and two waits more a stage).  With one epilogue group
+// refilled as soon as its MMAs are done, took 13.1 ms where one a stage took
+// 10.2 (two commits and two waits more a stage); polls that each lane decided
+// on its own, in a divergent loop, 2 to 8%.  With one epilogue group
 // the MMAs waited 4.8k of 26k cycles an item for the stores.  Policy + value
-// nets of 1,024 positions: 10.2 to 10.6 ms = 240 TFLOP/s of FP32 multiply-adds
+// nets of 1,024 positions: 9.8 to 10.3 ms = 250 TFLOP/s of FP32 multiply-adds
 // against 53.2 ms on the FFMA kernels; 77 positions of the reference's shapes
-// through the host call 0.83 against 3.62 ms.  Pairs of CTAs (M = 256 MMAs,
+// through the host call 0.80 against 3.62 ms.  Pairs of CTAs (M = 256 MMAs,
 // half of B's rows read and, with shared units, 20 KB of weights a stage) were
 // correct but slower (12.3 ms against 11.8, 14.2 against 10.4 with the waits
 // moved).
@@ -216,7 +219,7 @@ __device__ __forceinline__ void store_zero_parts(__nv_bfloat16 *dst, size_t part
 // ring.  Called by a converged warp.  A stage's waits come between the MMAs of
 // the stage ahead of it: the tensor pipe has few MMAs queued, and ran dry while
 // the issuer polled between two stages.  Policy + value nets of 1,024
-// positions: waits between the stages 11.8 ms, before the last four of the 12
+// positions (polls without a vote): waits between the stages 11.8 ms, before the last four of the 12
 // MMAs 10.3, before the last eight 10.2, before the last ten 11.1 (stages that
 // arrive late then hold up more); the next half's first stage and window
 // waited for as well: no gain.  False if a wait ran out.
@@ -696,8 +699,9 @@ int launch_split_trunk(const SplitTrunk &T, cudaStream_t s, int sm_count) {
     // 32-channel items while 64-channel ones would leave a third of the SMs
     // without any: their MMAs (N = 96, 64, 32) run at two thirds of the rate,
     // but twice as many SMs work on a layer.  Policy + value pair of the
-    // benchmark nets, us, 32 / 64 channels: 5 positions 311 / 364, 16 positions
-    // (100 wide items) 344 / 371, 20 positions (126) 391 / 375.
+    // benchmark nets, us, 32 / 64 channels: 5 positions 286 / 341, 16 positions
+    // (100 wide items) 316 / 351, 20 positions (126) 355 / 359, 24 positions 405 /
+    // 360.
     const int no = 3 * n3 * wide <= 2 * sm_count ? 32 : 64;
     int wrows = 0, items = 0, done3 = 0;
     for (int l = 0; l < T.nl; ++l) {

@@ -1382,10 +1382,14 @@ int tc_head_parts(int n, int variant) { return (n == 128 && variant != 1) ? 4 : 
 // items while every SM has at most one (24 positions), 128-row items while
 // 256-row ones would leave SMs without any (97); then the largest, whose MMAs
 // run at the full rate and read each weight stage for the most rows.  (ReLU nets
-// of up to 36 positions run in clusters instead, cluster_trunk.cu.)  Policy +
-// value pair, us, with 64 / 128 / 256 rows: 8 positions 217 / 220 / 253, 24
-// positions 233 / 235 / 269, 48 positions 277 / 252 / 283, 96 positions
-// 486 / 294 / 300, 128 positions 633 / 356 / 316.  Every output is the same
+// of up to 36 positions run in clusters instead, cluster_trunk.cu, where the
+// first layer is in the launch and the batch's size known.)  Policy + value
+// pair, us, with 64 / 128 rows, ReLU nets with the first layer ahead of the
+// launch (ELU nets with it inside): 1 position 203 / 209 (232 / 241), 8 positions
+// 219 / 224 (253 / 258), 20 positions 228 / 237 (259 / 269), 24 positions 233 /
+// 237 (267 / 269); five blocks of one differ by 0.1%.  With 64 / 128 / 256 rows:
+// 48 positions 277 / 252 / 283, 96 positions 486 / 294 / 300, 128 positions
+// 633 / 356 / 316.  Every output is the same
 // accumulation whatever the item's size: the results are bit for bit equal.
 static int trunk_tp(int rows) { return rows <= 64 * 152 ? 64 : (rows <= 256 * 152 ? 128 : 256); }
 static int trunk_tp5(int tp) { return tp == 256 ? TrunkCfg<256>::TP5 : tp; }
