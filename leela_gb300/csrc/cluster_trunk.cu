@@ -234,7 +234,9 @@ __global__ void __launch_bounds__(kClThreads, 1) __cluster_dims__(kClSize, 1, 1)
                 for (int j = 0; j < 2 * nt; ++j, ++g) {
                     const int h = j / nt, t = j - h * nt;
                     const uint32_t s = g % kClStages;
-                    if (aborted() || !mbar_wait(&ctl.w_empty[s], ((g / kClStages) & 1) ^ 1, p.wait_limit)) {
+                    // (a constant limit: with the parameter in this loop 24
+                    // positions take 156 us, not 150)
+                    if (aborted() || !mbar_wait(&ctl.w_empty[s], ((g / kClStages) & 1) ^ 1, kClWait)) {
                         fail(141);
                         l = p.nl;
                         break;

@@ -112,21 +112,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t phase) {
 
 // Bounded wait: gives up after `limit` polls and returns false.  Every
 // spin in this library is bounded so that a wrong count can never hang the
-// GPU; the caller records the failure in an error word and unwinds.  (Polls
-// first, then counts: the other way round, with a limit known only at run
-// time, the cluster trunk takes 156 us for 24 positions, not 150.)
+// GPU; the caller records the failure in an error word and unwinds.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t phase, uint32_t limit) {
-    uint32_t i = 0;
-    do
+    for (uint32_t i = 0; i < limit; ++i)
         if (mbar_try_wait(bar, phase)) return true;
-    while (++i < limit);
     return false;
 }
 
 // The same for a converged warp, one answer for all of its lanes: what
 // follows (elect.sync, tcgen05.ld, __syncwarp) needs every lane, also where a
-// barrier completes around the last poll.  (Here the count comes first: the
-// other way round 5 FP32 positions take 311 us, not 289.)
+// barrier completes around the last poll.  (The count comes before the poll:
+// the other way round 5 FP32 positions take 311 us, not 289.)
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t phase, uint32_t limit) {
     for (uint32_t i = 0; i < limit; ++i)
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, phase))) return true;

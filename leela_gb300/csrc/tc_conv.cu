@@ -46,6 +46,17 @@ constexpr int kTrunkThreads = 608;
 constexpr int kEpiWarpsT = 16;
 constexpr uint32_t kWaitLimit = 1u << 26;
 
+// mbar_wait_warp for the epilogue warps of this file, the lanes' answers joined
+// by a reduction: with votes 37 to 128 positions take 1 to 3% longer on the
+// trunk (64: 254 us a pair against 247), with reductions as long as with each
+// lane deciding alone.  (The issuers of the other files are the other way
+// round: 5 FP32 positions 307 us, not 287.)
+__device__ __forceinline__ bool mbar_wait_epi(uint64_t *bar, uint32_t phase, uint32_t limit) {
+    for (uint32_t i = 0; i < limit; ++i)
+        if (__reduce_and_sync(0xffffffffu, mbar_try_wait(bar, phase) ? 1u : 0u)) return true;
+    return false;
+}
+
 struct TcParams {
     int f16;  // operands are FP16 (else BF16)
     const float *bias;
@@ -269,7 +280,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         for (int tile = blockIdx.x; tile < p.ntiles && !__any_sync(0xffffffffu, abort_flag); tile += gridDim.x, ++local) {
             const int acc = local & 1;
             const uint32_t ak = (uint32_t)(local >> 1);
-            if (!mbar_wait_warp(&acc_full[acc], ak & 1, kWaitLimit)) { fail(31); break; }
+            if (!mbar_wait_epi(&acc_full[acc], ak & 1, kWaitLimit)) { fail(31); break; }
             tc_fence_after();
             if (active) {
                 int orow, point;
@@ -554,7 +565,7 @@ __global__ void __launch_bounds__(kTcThreadsT, 1)
             const int nhalf = max(0, min(2, (nrows - rq * 64) / 32));  // 32-row halves of this group
             const int acc = local & 1;
             const uint32_t ak = (uint32_t)(local >> 1);
-            if (!mbar_wait_warp(&acc_full[acc], ak & 1, kWaitLimit)) { fail(61); break; }
+            if (!mbar_wait_epi(&acc_full[acc], ak & 1, kWaitLimit)) { fail(61); break; }
             tc_fence_after();
             const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) +
                                     (uint32_t)(acc * C::TP + rq * 64);
@@ -586,7 +597,7 @@ __global__ void __launch_bounds__(kTcThreadsT, 1)
                     // one TMA store by the group's quarter-0 warp.
                     const uint32_t use = uses++;
                     uint8_t *buf = stg + rq * C::STG_BYTES;
-                    if (!mbar_wait_warp(&stg_empty[rq], (use & 1) ^ 1, kWaitLimit)) { fail(62); break; }
+                    if (!mbar_wait_epi(&stg_empty[rq], (use & 1) ^ 1, kWaitLimit)) { fail(62); break; }
                     const int row_lane = q_base + c * 32 + lane;
                     const int rl = row_lane % kL3Board;
                     const bool valid_lane = (rl % kL3Pitch) < kBoard && (rl / kL3Pitch) < kBoard;
@@ -1066,7 +1077,7 @@ __global__ void __maxnreg__(96)
         uint32_t uses = 0, done_n = 0;
         for (int q = 0;; ++q) {
             const int slot = q % kItemRing;
-            if (!mbar_wait_warp(&item_full[slot], (uint32_t)(q / kItemRing) & 1, WAIT_LIM)) { fail(79); break; }
+            if (!mbar_wait_epi(&item_full[slot], (uint32_t)(q / kItemRing) & 1, WAIT_LIM)) { fail(79); break; }
             const int it = item_id[slot];
             __syncwarp();
             if (lane == 0) mbar_arrive(&item_empty[slot]);
@@ -1086,7 +1097,7 @@ __global__ void __maxnreg__(96)
             const int nhalf = max(0, min(C::NH, (nrows - rq * C::RG + 31) / 32));
             const int acc = q & 1;
             const uint32_t ak = (uint32_t)(q >> 1);
-            if (!mbar_wait_warp(&acc_full[acc], ak & 1, WAIT_LIM)) { fail(80); break; }
+            if (!mbar_wait_epi(&acc_full[acc], ak & 1, WAIT_LIM)) { fail(80); break; }
             tc_fence_after();
             const uint32_t t_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256 + rq * C::RG);
             const int q_base = cs + rq * C::RG;
@@ -1124,7 +1135,7 @@ __global__ void __maxnreg__(96)
                     }
                     if (c >= nhalf || bad) continue;
                     const uint32_t use = uses++;
-                    if (!mbar_wait_warp(&stg_empty[rq], (use & 1) ^ 1, WAIT_LIM)) {
+                    if (!mbar_wait_epi(&stg_empty[rq], (use & 1) ^ 1, WAIT_LIM)) {
                         fail(81);
                         bad = true;
                         continue;
@@ -1198,7 +1209,7 @@ __global__ void __maxnreg__(96)
                 } else {
                     const uint32_t use = uses++;
                     uint8_t *buf = stg + rq * C::STG_BYTES;
-                    if (!mbar_wait_warp(&stg_empty[rq], (use & 1) ^ 1, WAIT_LIM)) {
+                    if (!mbar_wait_epi(&stg_empty[rq], (use & 1) ^ 1, WAIT_LIM)) {
                         fail(81);
                         bad = true;
                         continue;
