@@ -595,16 +595,18 @@ __global__ void __launch_bounds__(kSoftmaxThreads, 5)
 }
 
 // Results of a small host call straight into pinned host memory: up to two
-// arrays of n floats and the error word.
+// arrays of n floats; and the error word, taken out, so that it is reported with
+// the results that it belongs to and not with those of the next call in the
+// stream.
 __global__ void __launch_bounds__(256) export_kernel(const float *__restrict__ a, float *__restrict__ ha,
                                                      const float *__restrict__ b, float *__restrict__ hb, int n,
-                                                     const int *__restrict__ err, int *__restrict__ herr) {
+                                                     int *__restrict__ err, int *__restrict__ herr) {
     ptx::grid_dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         ha[i] = a[i];
         if (b) hb[i] = b[i];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *herr = *err;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *herr = atomicExch(err, 0);
 }
 
 // ------------------------------------------------------------ host launchers
@@ -707,7 +709,7 @@ size_t value_fc_counter_ints(int B, int H) {
 
 int value_fc_slice_units() { return kFcUnits; }
 
-void launch_export(const float *a, float *ha, const float *b, float *hb, int n, const int *err, int *herr,
+void launch_export(const float *a, float *ha, const float *b, float *hb, int n, int *err, int *herr,
                    cudaStream_t s) {
     launch_ex(export_kernel, std::max(1, std::min(64, (n + 255) / 256)), 256, s, true, a, ha, b, hb, n, err, herr);
 }

@@ -1206,7 +1206,9 @@ int run_host_boards_pipe(lg_ctx *c, int net, int B, float T, float *probs, float
 // graph).  Up to 32 KB an array by one kernel: a copy per array and a
 // synchronous one for the error word after the chunk were 16 us of a
 // one-position call (109 -> 93 us; the copy in, by a kernel as well, gave
-// less than 1 us).
+// less than 1 us).  The kernel takes the error word out: clearing it from the
+// host, on another stream, came too late for the next chunk where that stream
+// was busy.
 void results_out(lg_ctx *c, const float *a, float *ha, const float *b, float *hb, int n, int *herr) {
     if (n <= 8192) {
         launch_export(a, ha, b, hb, n, c->d_err, herr, c->stream);
@@ -1214,7 +1216,7 @@ void results_out(lg_ctx *c, const float *a, float *ha, const float *b, float *hb
     }
     cudaMemcpyAsync(ha, a, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
     if (b) cudaMemcpyAsync(hb, b, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    launch_export(nullptr, nullptr, nullptr, nullptr, 0, c->d_err, herr, c->stream);
 }
 
 // Host call: chunks of up to max_batch positions go through a cached CUDA
@@ -1274,7 +1276,6 @@ int run_host(lg_ctx *c, int net, const uint8_t *planes, int B, float T, float *p
         LG_CUDA_TRY(cudaEventSynchronize(c->host_done[slot]));
         const int herr = c->h_err[slot];
         if (herr) {
-            cudaMemset(c->d_err, 0, sizeof(int));
             lg_set_error("kernel reported error status %d", herr);
             return LG_ERR_DEVICE;
         }
@@ -1490,7 +1491,6 @@ int server_finish(lg_ctx *c, int slot) {
     LG_CUDA_TRY(cudaEventSynchronize(c->srv_done[slot]));
     const int herr = c->h_err[2 + slot];
     if (herr) {
-        cudaMemset(c->d_err, 0, sizeof(int));
         lg_set_error("kernel reported error status %d", herr);
         return LG_ERR_DEVICE;
     }

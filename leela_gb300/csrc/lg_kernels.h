@@ -143,10 +143,11 @@ int finish_init_device();
 size_t value_fc_counter_ints(int B, int H);
 int value_fc_slice_units();
 
-// a (and b, unless null) of n floats and the error word into pinned host
-// memory, by a kernel (a programmatic dependent of the previous one).  Like
-// the copies it stands for, it is not counted among a net's launches.
-void launch_export(const float *a, float *ha, const float *b, float *hb, int n, const int *err, int *herr,
+// a (and b, unless null) of n floats into pinned host memory, and the error
+// word, which it leaves zero, by a kernel (a programmatic dependent of the
+// previous one).  Like the copies it stands for, it is not counted among a
+// net's launches.
+void launch_export(const float *a, float *ha, const float *b, float *hb, int n, int *err, int *herr,
                    cudaStream_t s);
 
 // The finish of one batch (softmax, or the value head as launch_value_fc)
